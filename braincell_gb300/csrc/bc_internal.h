@@ -53,36 +53,46 @@ constexpr int kParamStride = BC_NPARAM + 1;
 constexpr int kParamStrideExtra = BC_P_EXT_MASK + 1;
 constexpr int kParamStrideCore = BC_P_CA_CI0 + 2;
 
-// A chain: nodes [start, start+count) of the tile, bottom (deepest) first; node
-// start+k+1 is the parent of node start+k and top_parent is the parent of the top
-// node (-1 at a root).  The record owns the consecutive contribution slots
-// aux .. aux + n_child, one per child chain, and writes its own contribution to
-// the parent's slot `slot` (-1 at a root).  32 bytes, read as two 16-byte vectors.
-struct ChainRec {
-  int32_t start;
-  int32_t count;
-  int32_t top_parent;   // tile node that is the parent of the top node, -1 at a root
-  int32_t aux;
-  int32_t n_child;
-  int32_t kind;
-  int32_t slot;
-  int32_t first;
+// The solver's view of a tile.  Each cell's tree is rooted at a branch point and
+// cut at its separators: branch points, the root, and cuts of long unbranched
+// runs.  A segment is an unbranched run of nodes between an upper separator and
+// either a lower separator or a leaf; its nodes are counted from the bottom.
+//
+// Segments are packed 32 to a warp slot, in decreasing length, and a slot's nodes
+// are stored jagged: node k of its lanes is the contiguous range of the lanes with
+// more than k nodes, so the lanes of a warp walking their segments touch
+// consecutive addresses and nothing is padded.  Separators come after all segment
+// nodes, grouped by the warp that sweeps them and, inside a group, by level
+// (children before parents).
+// The root, whose row needs no elimination, has a segment of no nodes to itself.
+struct alignas(16) SegRec {
+  uint16_t t, s;   // upper / lower separator (tile separator index); s = kLinkNone at a leaf
+  uint16_t len;    // nodes
+  uint16_t pad;
+  int32_t inbox;   // leaf segments: their entry in the upper separator's inbox
+  int32_t pad2;
 };
-constexpr int32_t kChainRegular = 0;
-
-// A warp slot of one phase: nodes [n_begin, n_begin + n_count) in lane order.
-// Lane l owns the chunk [n_begin + off[l], n_begin + off[l+1]) (the last used
-// lane ends at n_count; idle lanes have off[l] = n_count).  steps = 0: every
-// lane's chunk holds whole chains, walked serially; steps > 0: chains spread
-// over up to 2^steps lanes each, joined by shuffle scans; unit = 1: one node
-// per lane (lane l owns node n_begin + l).
-struct SlotRec {
-  int32_t n_begin;
-  int16_t n_count;
-  uint8_t steps;
-  uint8_t unit;
-  uint16_t off[32];
+struct alignas(16) SlotRec {
+  int32_t n_begin;   // first node
+  int32_t seg0;      // first segment (lane 0)
+  int16_t n_lanes;
+  uint16_t max_len;
+  int32_t lower;     // 1: the slot's segments have a lower separator
 };
+// A separator's inbox holds an entry per segment below it, padded to pairs.
+struct alignas(16) SepRec {
+  int32_t in0;     // first pair of inbox entries
+  int32_t inbox;   // this separator's entry in its upper separator's inbox (one nobody reads at a root)
+  uint16_t n_in;   // pairs
+  uint16_t t;      // upper separator (itself at a root)
+  int32_t pad;
+};
+// Separator levels [lv0, lv0 + n_lv) swept by one warp.
+struct alignas(8) GroupRec {
+  int32_t lv0, n_lv;
+};
+constexpr uint32_t kLinkNone = 0xFFFF;
+constexpr uint32_t kLinkSelf = 0xFFFE;  // lower half of a separator node's own link
 
 // Per-tile descriptor (global memory, read-only).
 struct TileDesc {
@@ -91,8 +101,8 @@ struct TileDesc {
   int32_t dyn_bytes;        // leading bytes written back (V, states)
   int32_t n_nodes;          // N (padded node count used for array strides)
   int32_t n_real_nodes;     // nodes actually used
-  int32_t n_chains;
-  int32_t n_phases;
+  int32_t n_segs;
+  int32_t n_phases;         // 1 + separator levels
   int32_t n_params;         // param records in this tile
   int32_t n_pulses;
   int64_t pulse_offset;     // into plan pulse array
@@ -104,12 +114,17 @@ struct TileDesc {
   int32_t off_plist;        // the tile's mechanism-probe list (ProbeRef)
   int64_t state_offset;     // elements into the plan's global mechanism-state array ([slot][n_nodes])
   int32_t off_ab;           // (alpha, beta) pairs
-  int32_t off_diag0, off_pidx, off_spec, off_specs;
-  int32_t off_chains, off_slots, off_phase, off_crec, off_params, off_mech;
-  int32_t scratch_bytes;    // diag/rhs/cD/cR scratch (shared memory after the blob)
-  int32_t off_dr;           // (diagonal, rhs) pairs, inside the scratch area
-  int32_t off_scd, off_scr;  // contribution slots, inside the scratch area
-  int32_t n_slots;          // contribution slots (scd / scr / sh entries)
+  int32_t off_pidx, off_spec, off_specs;
+  int32_t off_segs, off_slots, off_seps, off_levels, off_groups, off_link;
+  int32_t off_crec, off_params, off_mech;
+  int32_t scratch_bytes;    // solver scratch (shared memory after the blob)
+  int32_t off_dr;           // rows, inside the scratch area
+  int32_t off_q, off_inbox, off_srow, off_own, off_xsep;  // inside the scratch area
+  int32_t n_slots;          // warp slots of the segment elimination
+  int32_t n_groups;
+  int32_t sep0;             // first separator node
+  int32_t n_seps;
+  int32_t n_inbox;          // inbox entries
   int32_t n_cells;          // cells in the tile
   // network: tile synapse list (global ids), per-node tile-local cell index and
   // per-cell global id of spike sources (-1: not a source); off_ncell = -1 when

@@ -9,10 +9,12 @@
 // too large for shared memory run the same code on their global-memory blob.
 //
 // Per time step (reference: quad/_staggered.py:54-154):
-//   forward elimination   -- barrier-separated phases; in each, every thread walks
-//                            its chains leaf -> root (comp_triang_raw, :641-657);
-//   back-substitution     -- phases in reverse, chains root -> leaf (the O(n) sweep
-//                            whose result equals comp_backsub_raw, :742-760);
+//   segment elimination   -- every unbranched run of nodes between two separators
+//                            (branch points, the root, cuts of long runs) is
+//                            eliminated by one lane, all runs of the tile at once;
+//   separator sweep       -- the small tree of separators, leaf -> root and back
+//                            (comp_triang_raw, :641-657; comp_backsub_raw, :742-760),
+//                            a warp per group of cells;
 //   per-node update       -- V += delta (float-float), CalciumDetailed Ci from the
 //                            step-start current (cell.py:2261-2280, ion/calcium.py:
 //                            499-505), gates by exp-Euler at the new V (cell.py:
@@ -92,6 +94,19 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 
 constexpr uint32_t kBulkChunk = 32768;  // bytes per bulk copy instruction (multiple of 16)
 
+// A separator's row after the elimination of the segment above it: excess e, rhs r,
+// the coupling a to the upper separator and the coupling b of this separator in the
+// upper separator's row (a = b = 0 at a root).
+template <typename Real>
+struct alignas(16) SepRow {
+  Real e, r, a, b;
+};
+// Two inbox entries, read together.
+template <typename Real>
+struct alignas(16) InPair {
+  Real e0, r0, e1, r1;
+};
+
 // ------------------------------------------------------------------ tile view
 // Per-node pairs, loaded and stored as one vector access.
 template <typename Real>
@@ -119,21 +134,28 @@ template <typename Real>
 struct TileView {
   Pair<Real>* v;   // (V_hi, V_lo)
   Pair<Real>* ab;  // (alpha, beta); (alpha dt, beta dt) once pre-scaled
-  Pair<Real>* dr;  // (diagonal, rhs) of the row; (1 / pivot, rhs or x) during the sweeps
+  Pair<Real>* dr;  // (row excess, rhs); segment nodes: (p, u) after the elimination
   Real* state;
-  const Real *diag0, *params;
-  const SlotRec* slots;   // warp slots, phase by phase
-  const int32_t* phase;    // [n_phases + 1] slot ranges
-  const uint16_t *pidx, *spec, *crec;
-  const ChainRec* chains;
+  const Real* params;
+  const SlotRec* slots;        // warp slots of the segment elimination
+  const SegRec* segs;
+  const SepRec* seps;
+  const int32_t* levels;       // separator levels: [level] first separator, one past the last level at the end
+  const GroupRec* groups;
+  const uint32_t* link;        // per node: upper separator | lower separator << 16 (kLinkNone, kLinkSelf)
+  const uint16_t *pidx, *spec, *crec;  // crec: lane tiles only
   const SpecRec* specs;
   const uint32_t* mech;
-  Real *scd, *scr;
+  Real* q;                     // nodes of segments with a lower separator
+  Pair<Real>* inbox;           // per segment: (excess, rhs) it adds to its upper separator
+  SepRow<Real>* srow;          // per separator
+  Pair<Real>* own;             // per separator: what the segment above it adds to its upper separator by itself
+  Real* xsep;                  // per separator: its solved increment
   const int32_t* syn;       // tile synapse list (global synapse ids)
   const uint16_t* ncell;    // per node: tile-local cell (spike-source tiles only)
   const int32_t* srccell;   // per tile cell: global id of a spike source, -1 otherwise
   int32_t* stamp;           // per tile cell: last step with a crossing
-  int N, n_real, n_phases, n_cells;
+  int N, n_real, n_cells, n_slots, n_groups, sep0, n_seps, n_inbox;
   int pstride;  // reals per parameter record
   bool has_src;
 
@@ -142,18 +164,23 @@ struct TileView {
     ab = reinterpret_cast<Pair<Real>*>(base + td.off_ab);
     dr = reinterpret_cast<Pair<Real>*>(scratch + td.off_dr);
     state = reinterpret_cast<Real*>(gstate) + td.state_offset;
-    diag0 = reinterpret_cast<const Real*>(base + td.off_diag0);
     params = reinterpret_cast<const Real*>(base + td.off_params);
     slots = reinterpret_cast<const SlotRec*>(base + td.off_slots);
-    phase = reinterpret_cast<const int32_t*>(base + td.off_phase);
+    segs = reinterpret_cast<const SegRec*>(base + td.off_segs);
+    seps = reinterpret_cast<const SepRec*>(base + td.off_seps);
+    levels = reinterpret_cast<const int32_t*>(base + td.off_levels);
+    groups = reinterpret_cast<const GroupRec*>(base + td.off_groups);
+    link = reinterpret_cast<const uint32_t*>(base + td.off_link);
     crec = reinterpret_cast<const uint16_t*>(base + td.off_crec);
     pidx = reinterpret_cast<const uint16_t*>(base + td.off_pidx);
     spec = reinterpret_cast<const uint16_t*>(base + td.off_spec);
-    chains = reinterpret_cast<const ChainRec*>(base + td.off_chains);
     specs = reinterpret_cast<const SpecRec*>(base + td.off_specs);
     mech = reinterpret_cast<const uint32_t*>(base + td.off_mech);
-    scd = reinterpret_cast<Real*>(scratch + td.off_scd);
-    scr = reinterpret_cast<Real*>(scratch + td.off_scr);
+    q = reinterpret_cast<Real*>(scratch + td.off_q);
+    inbox = reinterpret_cast<Pair<Real>*>(scratch + td.off_inbox);
+    srow = reinterpret_cast<SepRow<Real>*>(scratch + td.off_srow);
+    own = reinterpret_cast<Pair<Real>*>(scratch + td.off_own);
+    xsep = reinterpret_cast<Real*>(scratch + td.off_xsep);
     syn = reinterpret_cast<const int32_t*>(base + td.off_syn);
     has_src = td.off_ncell >= 0;
     ncell = has_src ? reinterpret_cast<const uint16_t*>(base + td.off_ncell) : nullptr;
@@ -163,7 +190,11 @@ struct TileView {
     pstride = td.param_stride;
     N = td.n_nodes;
     n_real = td.n_real_nodes;
-    n_phases = td.n_phases;
+    n_slots = td.n_slots;
+    n_groups = td.n_groups;
+    sep0 = td.sep0;
+    n_seps = td.n_seps;
+    n_inbox = td.n_inbox;
   }
 };
 
@@ -908,15 +939,16 @@ __device__ __forceinline__ void steady_states(const Real* P, uint32_t m, Real* s
   }
 }
 
-// Row i of the next linear system: diag = 1 + dt (D + G / cm), rhs = dt I / cm
-// on membrane rows; diag = dt D, rhs = 0 on boundary rows.
+// Row i of the next linear system without its axial part: excess = diagonal minus
+// the row's axial coefficients = 1 + dt G / cm, rhs = dt I / cm on membrane rows;
+// 0, 0 on boundary rows.
 template <typename Real>
 __device__ __forceinline__ void write_row(const TileView<Real>& tv, int i, uint16_t pr, Real dt, Real G, Real I) {
   if (pr == kBoundary) {
-    tv.dr[i] = make_pair(dt * tv.diag0[i], Real(0));
+    tv.dr[i] = make_pair(Real(0), Real(0));
   } else {
     const Real invcm = tv.params[size_t(pr) * tv.pstride + BC_P_INVCM];
-    tv.dr[i] = make_pair(Real(1) + dt * (tv.diag0[i] + invcm * G), dt * invcm * I);
+    tv.dr[i] = make_pair(Real(1) + dt * (invcm * G), dt * invcm * I);
   }
 }
 
@@ -967,41 +999,34 @@ __device__ __forceinline__ void add_node_pulses(const TileView<Real>& tv, const 
   }
 }
 
-// ---------------------------------------------------------------- Hines sweeps
-// Row i of the increment system (V_{n+1} = V_n + x):
-//   d_i x_i - alpha_i x_parent - sum_c beta_c x_c = rhs_i - alpha_i Delta_i + sum_c beta_c Delta_c
-// with Delta_i = V_i - V_parent (float-float).  Along a chain (node k+1 is the
-// parent of node k; a = alpha dt, b = beta dt) elimination is the recurrence
-//   D_0 = d_0 - sum cD(children),  R_0 = r_0 + sum cR(children),
-//   R'_k = R_k - a_k Delta_k,  w_k = b_k / D_k,
-//   D_{k+1} = d_{k+1} - a_k b_k / D_k,  R_{k+1} = r_{k+1} + w_k R'_k + b_k Delta_k,
-// the chain top hands (cD, cR) = (a w, w R' + b Delta) to its parent, and back-
-// substitution is x_k = (R'_k + a_k x_{k+1}) / D_k.  All three are associative
-// scans along the chain: D through the projective (Moebius) form
-//   [p; q]_{k+1} = [[d_{k+1}, -a_k b_k], [1, 0]] [p; q]_k,  D = p / q,
-// R' and x through affine maps.  Each phase's chains are packed into 32-lane warp
-// slots.  In a "serial" slot every lane owns whole chains (at most lane_nodes
-// nodes) and walks them one after another.  In a "scan" slot a chain spans
-// several lanes: each lane composes the maps of its chunk, the lanes scan them
-// with shuffles (segmented at chain bottoms going up, at chain tops going down),
-// and each lane re-walks its chunk from the carry of its neighbours.
+// ---------------------------------------------------------------- tree solve
+// Row k of the increment system (V_{n+1} = V_n + x), with a = alpha dt of the node,
+// b = beta dt of a child (its coefficient in this row) and Delta = V - V_parent in
+// float-float:
+//   (e + a + sum b) x - a x_parent - sum b x_child = r - a Delta + sum b Delta_child
+// where e is the excess of the diagonal over the axial coefficients.
+//
+// 1. Segments (eliminate_segments): one lane eliminates the nodes of a segment
+//    between its lower separator s and upper separator t,
+//      E_k = e_k + wE,  F_k = wF,  R_k = r_k + wR - a_k Delta_k,  inv_k = 1 / (E_k + a_k),
+//      (wE, wF) = b_k inv_k (E_k, F_k),  wR = b_k (inv_k R_k + Delta_k),
+//    starting from wE = wF = b_s, wR = b_s Delta_s (0 at a leaf), then walks back down
+//    to leave x_k = p_k + q_k x_s + u_k x_t in every node and to hand both separators
+//    their rows' share.  The excess form has no subtraction in the pivots.
+// 2. Separators (sweep_separators): the same elimination on the tree of separators,
+//    one warp per group of cells, level by level, then back down to x.
+// 3. Every other node's x is one or two multiply-adds on its separators' x, taken by
+//    the update pass (node_increment).
+//
+// Why this split.  The time of a tile's step is latency: the walks down the tree
+// levels with a block barrier at each (18 per step for the 10,000-cell uneven
+// population, whose runs have 6.4 nodes on average) took 37 of 54 thousand cycles per
+// step of a 2,500-node tile, most of them waiting.  Runs do not depend on one another,
+// so one pass covers 94 % of the nodes, and what stays serial is the separator tree
+// (one row per branch point), which a warp sweeps without block barriers: three
+// barriers per step.
 
 constexpr unsigned kFullMask = 0xffffffffu;
-
-__device__ __forceinline__ ChainRec load_rec(const ChainRec* recs, int c) {
-  const int4* p = reinterpret_cast<const int4*>(recs + c);
-  const int4 x = p[0], y = p[1];
-  ChainRec r;
-  r.start = x.x;
-  r.count = x.y;
-  r.top_parent = x.z;
-  r.aux = x.w;
-  r.n_child = y.x;
-  r.kind = y.y;
-  r.slot = y.z;
-  r.first = y.w;
-  return r;
-}
 
 // (alpha dt, beta dt) of node i: pre-scaled in shared-memory tiles, scaled here otherwise.
 template <typename Real, bool kPre>
@@ -1014,487 +1039,215 @@ __device__ __forceinline__ Pair<Real> coef(const TileView<Real>& tv, int i, Real
   return c;
 }
 
-__device__ __forceinline__ float rabs(float x) { return fabsf(x); }
-__device__ __forceinline__ double rabs(double x) { return fabs(x); }
-__device__ __forceinline__ float rmax(float x, float y) { return fmaxf(x, y); }
-__device__ __forceinline__ double rmax(double x, double y) { return fmax(x, y); }
-
-// 2^-floor(log2 m) for m > 0 (exact scaling by a power of two; the exponent is
-// clamped so that the result stays a normal number).
-__device__ __forceinline__ float pow2_inv(float m) {
-  int e = (__float_as_int(m) >> 23) & 0xff;
-  e = min(max(e, 1), 253);
-  return __int_as_float((254 - e) << 23);
-}
-__device__ __forceinline__ double pow2_inv(double m) {
-  long long e = (__double_as_longlong(m) >> 52) & 0x7ff;
-  e = min(max(e, 1LL), 2045LL);
-  return __longlong_as_double((2046LL - e) << 52);
-}
-
-template <typename Real>
-struct Mob {
-  Real m00, m01, m10, m11;  // [[m00, m01], [m10, m11]]
-};
-
-// Rescale by a power of two: the projective ratio a map defines does not change,
-// and the entries stay in range.
-template <typename Real>
-__device__ __forceinline__ void mob_norm(Mob<Real>& r) {
-  const Real s = pow2_inv(rmax(rmax(rabs(r.m00), rabs(r.m01)), rmax(rabs(r.m10), rabs(r.m11))));
-  r.m00 *= s;
-  r.m01 *= s;
-  r.m10 *= s;
-  r.m11 *= s;
-}
-
-// hi * lo (hi is the later map).
-template <typename Real>
-__device__ __forceinline__ Mob<Real> mob_mul(const Mob<Real>& hi, const Mob<Real>& lo) {
-  Mob<Real> r;
-  r.m00 = hi.m00 * lo.m00 + hi.m01 * lo.m10;
-  r.m01 = hi.m00 * lo.m01 + hi.m01 * lo.m11;
-  r.m10 = hi.m10 * lo.m00 + hi.m11 * lo.m10;
-  r.m11 = hi.m10 * lo.m01 + hi.m11 * lo.m11;
-  return r;
-}
-
-template <typename Real>
-__device__ __forceinline__ Mob<Real> mob_shfl_up(const Mob<Real>& m, int off) {
-  Mob<Real> o;
-  o.m00 = __shfl_up_sync(kFullMask, m.m00, off);
-  o.m01 = __shfl_up_sync(kFullMask, m.m01, off);
-  o.m10 = __shfl_up_sync(kFullMask, m.m10, off);
-  o.m11 = __shfl_up_sync(kFullMask, m.m11, off);
-  return o;
-}
-
-// Lane of the segment start at or below `lane` (bit l of `heads` marks a start).
-__device__ __forceinline__ int seg_first(unsigned heads, int lane) {
-  return 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
-}
-// Lane of the segment end at or above `lane` (bit l of `tops` marks an end).
-__device__ __forceinline__ int seg_last(unsigned tops, int lane) {
-  return lane + __ffs(tops >> lane) - 1;
-}
-
-// Inclusive segmented scan of Moebius maps over the lanes (lane order = chain
-// order); `reach` = lane - first lane of the segment; 2^steps >= segment lanes.
-// Inputs are normalised maps; a product of four of them stays far inside the
-// FP32 range (each factor changes the scale by at most ~1e6 either way), so the
-// partial products are renormalised after every second step only.
-template <typename Real>
-__device__ __forceinline__ Mob<Real> scan_mob(Mob<Real> m, int reach, int steps) {
-  for (int s = 0, off = 1; s < steps; ++s, off <<= 1) {
-    const Mob<Real> o = mob_shfl_up(m, off);
-    if (off <= reach) m = mob_mul(m, o);
-    if (s & 1) mob_norm(m);
-  }
-  return m;
-}
-
-// Inclusive segmented scan of affine maps x -> a x + b, later lanes applied last.
-template <typename Real>
-__device__ __forceinline__ void scan_aff_up(Real& a, Real& b, int reach, int steps) {
-  for (int s = 0, off = 1; s < steps; ++s, off <<= 1) {
-    const Real oa = __shfl_up_sync(kFullMask, a, off);
-    const Real ob = __shfl_up_sync(kFullMask, b, off);
-    if (off <= reach) {
-      b = a * ob + b;
-      a = a * oa;
-    }
-  }
-}
-
-// The same towards lower lanes (back-substitution runs from chain tops down);
-// `reach` = last lane of the segment - lane.
-template <typename Real>
-__device__ __forceinline__ void scan_aff_down(Real& a, Real& b, int reach, int steps) {
-  for (int s = 0, off = 1; s < steps; ++s, off <<= 1) {
-    const Real oa = __shfl_down_sync(kFullMask, a, off);
-    const Real ob = __shfl_down_sync(kFullMask, b, off);
-    if (off <= reach) {
-      b = a * ob + b;
-      a = a * oa;
-    }
-  }
-}
-
-template <typename Real>
-__device__ __forceinline__ Pair<Real> shfl_up_pair(const Pair<Real>& p, int off) {
-  return make_pair<Real>(__shfl_up_sync(kFullMask, p.x, off), __shfl_up_sync(kFullMask, p.y, off));
-}
-template <typename Real>
-__device__ __forceinline__ Pair<Real> shfl_down_pair(const Pair<Real>& p, int off) {
-  return make_pair<Real>(__shfl_down_sync(kFullMask, p.x, off), __shfl_down_sync(kFullMask, p.y, off));
-}
-
 template <typename Real>
 __device__ __forceinline__ Real vdelta(const Pair<Real>& v, const Pair<Real>& up) {
   return (v.x - up.x) + (v.y - up.y);
 }
 
-// Children's contributions pulled by a chain bottom: the first four slots are
-// loaded together (predicated), further ones in a loop.
-template <typename Real>
-__device__ __forceinline__ void pull_children(const TileView<Real>& tv, const ChainRec& ch, Real& D, Real& R) {
-  const int n = ch.n_child, a0 = ch.aux;
-  Real cd[4], cr[4];
+// One warp slot: lane l eliminates segment seg0 + l.  kLower: the slot's segments
+// have a lower separator.  Nodes are taken kBatch at a time, all loads of a batch
+// issued together: taken one by one, each node cost about 250 cycles of exposed
+// shared-memory latency on each of the two walks.  A lane past its segment's end
+// reads its upper separator's node and drops the result.
+template <typename Real, bool kPre, bool kLower>
+__device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
+  constexpr int kBatch = 4;
+  const bool valid = lane < sr.n_lanes;
+  const SegRec sg = tv.segs[sr.seg0 + (valid ? lane : 0)];
+  const int len = valid ? int(sg.len) : 0;
+  const int max_len = sr.max_len;
+  const int nt = tv.sep0 + sg.t;
+  int off = sr.n_begin;  // first node of row k of the slot
+  auto next_id = [&](int k) {
+    const int id = len > k ? off + lane : nt;
+    off += __popc(__ballot_sync(kFullMask, len > k));
+    return id;
+  };
+  int id0 = next_id(0);
+  Pair<Real> v0 = tv.v[id0];
+  Real wE = Real(0), wF = Real(0), wR = Real(0), as = Real(0), ds = Real(0);
+  Pair<Real> row_s = make_pair(Real(0), Real(0));
+  if (kLower) {
+    const int ns = tv.sep0 + sg.s;
+    const Pair<Real> cs = coef<Real, kPre>(tv, ns, dt);
+    row_s = tv.dr[ns];
+    ds = vdelta<Real>(tv.v[ns], v0);
+    as = cs.x;
+    wE = wF = cs.y;
+    wR = cs.y * ds;
+  }
+  for (int k = 0; k < max_len; k += kBatch) {
+    int id[kBatch + 1];
+    Pair<Real> row[kBatch], c[kBatch], v[kBatch + 1];
+    id[0] = id0;
+    v[0] = v0;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    cd[j] = j < n ? tv.scd[a0 + j] : Real(0);
-    cr[j] = j < n ? tv.scr[a0 + j] : Real(0);
-  }
+    for (int j = 1; j <= kBatch; ++j) id[j] = next_id(k + j);
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    D -= cd[j];
-    R += cr[j];
-  }
-  for (int j = 4; j < n; ++j) {
-    D -= tv.scd[a0 + j];
-    R += tv.scr[a0 + j];
-  }
-}
-
-// Lane chunk of a warp slot: nodes [k0, k0 + len) (len = 0 for an idle lane).
-__device__ __forceinline__ void lane_chunk(const SlotRec& sr, int lane, int& k0, int& len) {
-  const int o0 = sr.off[lane];
-  const int o1 = lane < 31 ? int(sr.off[lane + 1]) : int(sr.n_count);
-  k0 = sr.n_begin + o0;
-  len = o1 - o0;
-}
-
-// Elimination of one warp slot holding one node per lane.
-template <typename Real, bool kPre>
-__device__ __forceinline__ void eliminate_lanes(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  const bool valid = lane < sr.n_count;
-  const int k = sr.n_begin + (valid ? lane : 0);
-  const ChainRec ch = load_rec(tv.chains, tv.crec[k]);
-  const bool head = !valid || k == ch.start;
-  const bool tail = valid && k == ch.start + ch.count - 1;
-  const Pair<Real> q = tv.dr[k];
-  const Pair<Real> c = coef<Real, kPre>(tv, k, dt);
-  const Pair<Real> v = tv.v[k];
-  Pair<Real> vup = shfl_down_pair<Real>(v, 1);  // node k+1 sits in the next lane
-  if (tail) vup = ch.top_parent >= 0 ? tv.v[ch.top_parent] : v;
-  const Real delta = vdelta<Real>(v, vup);
-  const Pair<Real> cp = shfl_up_pair<Real>(c, 1);  // node k-1 sits in the previous lane
-  const Real deltap = __shfl_up_sync(kFullMask, delta, 1);
-  Real D0 = q.x, R0 = q.y;
-  if (head && valid) pull_children(tv, ch, D0, R0);
-  Mob<Real> m;
-  m.m10 = Real(1);
-  m.m11 = Real(0);
-  if (head) {
-    m.m00 = D0;
-    m.m01 = Real(0);
-  } else {
-    m.m00 = q.x;
-    m.m01 = -cp.x * cp.y;
-  }
-  mob_norm(m);
-  const int reach = lane - seg_first(__ballot_sync(kFullMask, head), lane);
-  m = scan_mob(m, reach, sr.steps);
-  const Real inv = m.m10 * pivot_rcp(m.m00);
-  const Real w = c.y * inv;
-  const Real wp = __shfl_up_sync(kFullMask, w, 1);
-  Real a, b;
-  if (head) {
-    a = Real(0);
-    b = R0 - c.x * delta;
-  } else {
-    a = wp;
-    b = q.y + cp.y * deltap - c.x * delta;
-  }
-  scan_aff_up(a, b, reach, sr.steps);
-  if (valid) {
-    tv.dr[k] = make_pair(inv, b);
-    if (tail && ch.slot >= 0) {
-      tv.scd[ch.slot] = c.x * w;
-      tv.scr[ch.slot] = w * b + c.y * delta;
+    for (int j = 0; j < kBatch; ++j) {
+      row[j] = tv.dr[id[j]];
+      c[j] = coef<Real, kPre>(tv, id[j], dt);
+      v[j + 1] = tv.v[id[j + 1]];
     }
-  }
-}
-
-// Back-substitution of one warp slot holding one node per lane.
-template <typename Real, bool kPre>
-__device__ __forceinline__ void backsub_lanes(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  const bool valid = lane < sr.n_count;
-  const int k = sr.n_begin + (valid ? lane : 0);
-  const ChainRec ch = load_rec(tv.chains, tv.crec[k]);
-  const bool tail = valid && k == ch.start + ch.count - 1;
-  const Pair<Real> q = tv.dr[k];  // (1 / D, R')
-  Real A = coef<Real, kPre>(tv, k, dt).x * q.x, B = q.y * q.x;
-  if (tail) {
-    const Real xp = ch.top_parent >= 0 ? tv.dr[ch.top_parent].y : Real(0);
-    B = A * xp + B;
-    A = Real(0);
-  }
-  const bool top = !valid || tail;
-  scan_aff_down(A, B, seg_last(__ballot_sync(kFullMask, top), lane) - lane, sr.steps);
-  if (valid) tv.dr[k].y = B;
-}
-
-// Serial elimination of one whole chain by one lane.
-template <typename Real, bool kPre>
-__device__ __forceinline__ void eliminate_chain(const TileView<Real>& tv, const ChainRec& ch, Real dt) {
-  const int s0 = ch.start, end = ch.start + ch.count;
-  const Pair<Real> q = tv.dr[s0];
-  Real D = q.x, R = q.y;
-  pull_children(tv, ch, D, R);
-  Pair<Real> c = coef<Real, kPre>(tv, s0, dt), v = tv.v[s0];
-  // node s0 + 1 (or the chain's parent, or -- at the root -- the top node itself)
-  const Pair<Real> v_top = ch.top_parent >= 0 ? tv.v[ch.top_parent] : tv.v[end - 1];
-  Pair<Real> q1 = q, c1 = c, v1 = v_top;
-  if (s0 + 1 < end) {
-    q1 = tv.dr[s0 + 1];
-    c1 = coef<Real, kPre>(tv, s0 + 1, dt);
-    v1 = tv.v[s0 + 1];
-  }
-  for (int i = s0;; ++i) {
-    Pair<Real> q2 = q1, c2 = c1, v2 = v_top;
-    if (i + 2 < end) {
-      q2 = tv.dr[i + 2];
-      c2 = coef<Real, kPre>(tv, i + 2, dt);
-      v2 = tv.v[i + 2];
-    }
-    const Real inv = pivot_rcp(D);
-    const Real delta = vdelta<Real>(v, v1);
-    R -= c.x * delta;
-    tv.dr[i] = make_pair(inv, R);
-    const Real w = c.y * inv;
-    if (i + 1 == end) {
-      if (ch.slot >= 0) {
-        tv.scd[ch.slot] = c.x * w;
-        tv.scr[ch.slot] = w * R + c.y * delta;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const Real delta = vdelta<Real>(v[j], v[j + 1]);
+      const Real E = row[j].x + wE;
+      const Real R = (row[j].y + wR) - c[j].x * delta;
+      const Real inv = pivot_rcp(E + c[j].x);
+      if (len > k + j) {
+        tv.dr[id[j]] = make_pair(inv * R, c[j].x * inv);
+        const Real g = c[j].y * inv;
+        if (kLower) {
+          tv.q[id[j]] = inv * wF;
+          wF *= g;
+        }
+        wE = (c[j].y * E) * inv;
+        wR = g * R + c[j].y * delta;
       }
-      break;
     }
-    D = q1.x - c.x * w;
-    R = q1.y + w * R + c.y * delta;
-    c = c1;
-    v = v1;
-    q1 = q2;
-    c1 = c2;
-    v1 = v2;
+    id0 = id[kBatch];
+    v0 = v[kBatch];
   }
-}
-
-// Serial back-substitution of one whole chain by one lane (top down).
-template <typename Real, bool kPre>
-__device__ __forceinline__ void backsub_chain(const TileView<Real>& tv, const ChainRec& ch, Real dt) {
-  const int top = ch.start + ch.count - 1;
-  Real dp = ch.top_parent >= 0 ? tv.dr[ch.top_parent].y : Real(0);
-  Pair<Real> q = tv.dr[top];
-  Real al = coef<Real, kPre>(tv, top, dt).x;
-  Pair<Real> q1 = q;
-  Real al1 = al;
-  if (top - 1 >= ch.start) {
-    q1 = tv.dr[top - 1];
-    al1 = coef<Real, kPre>(tv, top - 1, dt).x;
-  }
-  for (int i = top;; --i) {
-    Pair<Real> q2 = q1;
-    Real al2 = al1;
-    if (i - 2 >= ch.start) {
-      q2 = tv.dr[i - 2];
-      al2 = coef<Real, kPre>(tv, i - 2, dt).x;
+  if (!kLower && valid) tv.inbox[sg.inbox] = make_pair(wE, wR);
+  // back down (off is one past the slot's last node): x_k = p + q x_s + u x_t
+  Real p = Real(0), q = Real(0), u = Real(1);
+  for (int k = max_len - 1; k >= 0; k -= kBatch) {
+    int id[kBatch];
+    Pair<Real> d[kBatch];
+    Real f[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      off -= k >= j ? __popc(__ballot_sync(kFullMask, len > k - j)) : 0;
+      id[j] = k >= j && len > k - j ? off + lane : -1;
     }
-    const Real x = (q.y + al * dp) * q.x;
-    tv.dr[i].y = x;
-    dp = x;
-    if (i == ch.start) break;
-    q = q1;
-    al = al1;
-    q1 = q2;
-    al1 = al2;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      d[j] = id[j] >= 0 ? tv.dr[id[j]] : make_pair(Real(0), Real(1));
+      f[j] = kLower && id[j] >= 0 ? tv.q[id[j]] : Real(0);
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      p = d[j].x + d[j].y * p;
+      u = d[j].y * u;
+      q = f[j] + d[j].y * q;
+      if (id[j] >= 0) {
+        tv.dr[id[j]] = make_pair(p, u);
+        if (kLower) tv.q[id[j]] = q;
+      }
+    }
   }
-}
-
-// A slot of whole chains: every lane walks the chains of its chunk one after another.
-template <typename Real, bool kPre>
-__device__ __forceinline__ void eliminate_serial(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  int k, len;
-  lane_chunk(sr, lane, k, len);
-  const int end = k + len;
-  while (k < end) {
-    const ChainRec ch = load_rec(tv.chains, tv.crec[k]);
-    eliminate_chain<Real, kPre>(tv, ch, dt);
-    k += ch.count;
+  if (kLower && valid) {
+    SepRow<Real> o;
+    o.e = row_s.x + as * (Real(1) - q - u);
+    o.r = row_s.y + as * (p - ds);
+    o.a = as * u;
+    o.b = wF;
+    tv.srow[sg.s] = o;
+    tv.own[sg.s] = make_pair(wE - wF, wR);
   }
 }
 
 template <typename Real, bool kPre>
-__device__ __forceinline__ void backsub_serial(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  int k0, len;
-  lane_chunk(sr, lane, k0, len);
-  int k = k0 + len - 1;
-  while (k >= k0) {
-    const ChainRec ch = load_rec(tv.chains, tv.crec[k]);
-    backsub_chain<Real, kPre>(tv, ch, dt);
-    k = ch.start - 1;
-  }
-}
-
-// A slot of chains spread over several lanes each: every lane composes the maps
-// of its chunk, the lanes scan them (segmented per chain), and every lane
-// re-walks its chunk from the carry of the lanes below.
-template <typename Real, bool kPre>
-__device__ __forceinline__ void eliminate_scan(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  int k0, len;
-  lane_chunk(sr, lane, k0, len);
-  ChainRec ch{};
-  if (len > 0) ch = load_rec(tv.chains, tv.crec[k0]);
-  const int top = ch.start + ch.count - 1;
-  const bool head = len > 0 && k0 == ch.start;
-  const bool seg = head || len == 0;
-  const int reach = lane - seg_first(__ballot_sync(kFullMask, seg), lane);
-  Real D0 = Real(0), R0 = Real(0);
-  if (head) {
-    const Pair<Real> q = tv.dr[k0];
-    D0 = q.x;
-    R0 = q.y;
-    pull_children(tv, ch, D0, R0);
-  }
-  // chunk map of the pivot recurrence
-  Mob<Real> m{Real(1), Real(0), Real(0), Real(1)};
-  for (int j = 0; j < len; ++j) {
-    const int k = k0 + j;
-    Mob<Real> e;
-    e.m10 = Real(1);
-    e.m11 = Real(0);
-    if (k == ch.start) {
-      e.m00 = D0;
-      e.m01 = Real(0);
-    } else {
-      const Pair<Real> cp = coef<Real, kPre>(tv, k - 1, dt);
-      e.m00 = tv.dr[k].x;
-      e.m01 = -cp.x * cp.y;
-    }
-    m = mob_mul(e, m);
-    mob_norm(m);
-  }
-  m = scan_mob(m, reach, sr.steps);
-  const Mob<Real> mx = mob_shfl_up(m, 1);
-  // re-walk: pivots of the chunk from the state after the lane below
-  Real p = mx.m00, pq = mx.m10;
-  for (int j = 0; j < len; ++j) {
-    const int k = k0 + j;
-    if (k == ch.start) {
-      p = D0;
-      pq = Real(1);
-    } else {
-      const Pair<Real> cp = coef<Real, kPre>(tv, k - 1, dt);
-      const Real np = tv.dr[k].x * p - cp.x * cp.y * pq;
-      pq = p;
-      p = np;
-      const Real s = pow2_inv(rmax(rabs(p), rabs(pq)));
-      p *= s;
-      pq *= s;
-    }
-    tv.dr[k].x = pq * pivot_rcp(p);  // 1 / D_k
-  }
-  __syncwarp();
-  // chunk map of the right-hand-side recurrence R'_k = a_k R'_{k-1} + b_k
-  Real fa = Real(1), fb = Real(0);
-  for (int j = 0; j < len; ++j) {
-    const int k = k0 + j;
-    const Pair<Real> c = coef<Real, kPre>(tv, k, dt);
-    const Pair<Real> v = tv.v[k];
-    const Pair<Real> vup = k == top ? (ch.top_parent >= 0 ? tv.v[ch.top_parent] : v) : tv.v[k + 1];
-    const Real delta = vdelta<Real>(v, vup);
-    Real a, b;
-    if (k == ch.start) {
-      a = Real(0);
-      b = R0 - c.x * delta;
-    } else {
-      const Pair<Real> cp = coef<Real, kPre>(tv, k - 1, dt);
-      a = cp.y * tv.dr[k - 1].x;
-      b = tv.dr[k].y + cp.y * vdelta<Real>(tv.v[k - 1], v) - c.x * delta;
-    }
-    tv.dr[k].y = b;
-    fb = a * fb + b;
-    fa = a * fa;
-  }
-  scan_aff_up(fa, fb, reach, sr.steps);
-  Real r = __shfl_up_sync(kFullMask, fb, 1);
-  for (int j = 0; j < len; ++j) {
-    const int k = k0 + j;
-    Real a = Real(0);
-    if (k != ch.start) a = coef<Real, kPre>(tv, k - 1, dt).y * tv.dr[k - 1].x;
-    r = a * r + tv.dr[k].y;
-    tv.dr[k].y = r;
-    if (k == top && ch.slot >= 0) {
-      const Pair<Real> c = coef<Real, kPre>(tv, k, dt);
-      const Pair<Real> v = tv.v[k];
-      const Pair<Real> vup = ch.top_parent >= 0 ? tv.v[ch.top_parent] : v;
-      const Real w = c.y * tv.dr[k].x;
-      tv.scd[ch.slot] = c.x * w;
-      tv.scr[ch.slot] = w * r + c.y * vdelta<Real>(v, vup);
-    }
-  }
-}
-
-template <typename Real, bool kPre>
-__device__ __forceinline__ void backsub_scan(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  int k0, len;
-  lane_chunk(sr, lane, k0, len);
-  ChainRec ch{};
-  if (len > 0) ch = load_rec(tv.chains, tv.crec[k0]);
-  const int top = ch.start + ch.count - 1;
-  const bool has_top = len > 0 && k0 + len - 1 == top;
-  const bool seg_top = len == 0 || has_top;
-  const int reach = seg_last(__ballot_sync(kFullMask, seg_top), lane) - lane;
-  const Real xp = has_top && ch.top_parent >= 0 ? tv.dr[ch.top_parent].y : Real(0);
-  Real fa = Real(1), fb = Real(0);
-  for (int j = len - 1; j >= 0; --j) {
-    const int k = k0 + j;
-    const Pair<Real> q = tv.dr[k];
-    Real A = coef<Real, kPre>(tv, k, dt).x * q.x, B = q.y * q.x;
-    if (k == top) {
-      B = A * xp + B;
-      A = Real(0);
-    }
-    fb = A * fb + B;
-    fa = A * fa;
-  }
-  scan_aff_down(fa, fb, reach, sr.steps);
-  Real x = __shfl_down_sync(kFullMask, fb, 1);  // x of the node after this chunk
-  for (int j = len - 1; j >= 0; --j) {
-    const int k = k0 + j;
-    const Pair<Real> q = tv.dr[k];
-    const Real A = coef<Real, kPre>(tv, k, dt).x * q.x;
-    x = k == top ? A * xp + q.y * q.x : A * x + q.y * q.x;
-    tv.dr[k].y = x;
-  }
-}
-
-template <typename Real, bool kPre>
-__device__ __forceinline__ void eliminate_phase(const TileView<Real>& tv, int p, int warp, int n_warps, int lane,
-                                                Real dt) {
-  for (int s = tv.phase[p] + warp; s < tv.phase[p + 1]; s += n_warps) {
-    const SlotRec& sr = tv.slots[s];
-    if (sr.steps == 0)
-      eliminate_serial<Real, kPre>(tv, sr, lane, dt);
-    else if (sr.unit)
-      eliminate_lanes<Real, kPre>(tv, sr, lane, dt);
+__device__ __forceinline__ void eliminate_segments(const TileView<Real>& tv, int warp, int n_warps, int lane, Real dt) {
+  for (int s = warp; s < tv.n_slots; s += n_warps) {
+    const SlotRec sr = tv.slots[s];
+    if (sr.lower)
+      eliminate_slot<Real, kPre, true>(tv, sr, lane, dt);
     else
-      eliminate_scan<Real, kPre>(tv, sr, lane, dt);
+      eliminate_slot<Real, kPre, false>(tv, sr, lane, dt);
   }
 }
 
-template <typename Real, bool kPre>
-__device__ __forceinline__ void backsub_phase(const TileView<Real>& tv, int p, int warp, int n_warps, int lane,
-                                              Real dt) {
-  for (int s = tv.phase[p] + warp; s < tv.phase[p + 1]; s += n_warps) {
-    const SlotRec& sr = tv.slots[s];
-    if (sr.steps == 0)
-      backsub_serial<Real, kPre>(tv, sr, lane, dt);
-    else if (sr.unit)
-      backsub_lanes<Real, kPre>(tv, sr, lane, dt);
-    else
-      backsub_scan<Real, kPre>(tv, sr, lane, dt);
+// What the level below does not change about a separator: loaded one level ahead.
+template <typename Real>
+struct SepItem {
+  SepRec rec;
+  SepRow<Real> row;
+  Pair<Real> own;
+};
+
+template <typename Real>
+__device__ __forceinline__ SepItem<Real> load_sep(const TileView<Real>& tv, int j) {
+  SepItem<Real> it;
+  it.rec = tv.seps[j];
+  it.row = tv.srow[j];
+  it.own = tv.own[j];
+  return it;
+}
+
+template <typename Real>
+__device__ __forceinline__ void eliminate_sep(const TileView<Real>& tv, int j, const SepItem<Real>& it) {
+  const InPair<Real>* in = reinterpret_cast<const InPair<Real>*>(tv.inbox) + it.rec.in0;
+  InPair<Real> c = in[0];
+  Real E = it.row.e + (c.e0 + c.e1), R = it.row.r + (c.r0 + c.r1);
+  for (int k = 1; k < it.rec.n_in; ++k) {
+    c = in[k];
+    E += c.e0 + c.e1;
+    R += c.r0 + c.r1;
   }
+  const Real inv = pivot_rcp(E + it.row.a);
+  const Real w = it.row.b * inv;
+  tv.inbox[it.rec.inbox] = make_pair(it.own.x + w * E, it.own.y + w * R);
+  tv.dr[tv.sep0 + j] = make_pair(it.row.a * inv, R * inv);
+}
+
+// The separator tree: a warp per group of cells, lanes over the separators of a
+// level.  A level's own data are loaded while the level before is eliminated, so
+// what is left per level is the inbox, one reciprocal and two stores: the sweep is
+// one warp's chain of dependent instructions, and every one of them counts.
+template <typename Real>
+__device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int warp, int n_warps, int lane) {
+  for (int g = warp; g < tv.n_groups; g += n_warps) {
+    const GroupRec gr = tv.groups[g];
+    const int32_t* lv = tv.levels + gr.lv0;
+    int b = lv[0], e = lv[1];
+    SepItem<Real> it = load_sep(tv, min(b + lane, e - 1));
+    for (int l = 0; l < gr.n_lv; ++l) {
+      const int e1 = lv[min(l + 2, gr.n_lv)];
+      const SepItem<Real> nx = load_sep(tv, min(e + lane, tv.n_seps - 1));
+      if (b + lane < e) eliminate_sep(tv, b + lane, it);
+      for (int j = b + lane + 32; j < e; j += 32) eliminate_sep(tv, j, load_sep(tv, j));
+      __syncwarp();
+      b = e;
+      e = e1;
+      it = nx;
+    }
+    // back down: x = R / D + A / D x_t (A = 0 and t = itself at a root), the next
+    // level's pairs loaded ahead
+    e = lv[gr.n_lv];
+    b = lv[gr.n_lv - 1];
+    int j = min(b + lane, e - 1);
+    uint32_t t = tv.seps[j].t;
+    Pair<Real> d = tv.dr[tv.sep0 + j];
+    for (int l = gr.n_lv - 1; l >= 0; --l) {
+      const int b1 = lv[max(l - 1, 0)];
+      const int j1 = min(b1 + lane, e - 1);
+      const uint32_t t1 = tv.seps[j1].t;
+      const Pair<Real> d1 = tv.dr[tv.sep0 + j1];
+      if (b + lane < e) tv.xsep[b + lane] = d.y + d.x * tv.xsep[t];
+      for (int i = b + lane + 32; i < e; i += 32) {
+        const Pair<Real> di = tv.dr[tv.sep0 + i];
+        tv.xsep[i] = di.y + di.x * tv.xsep[tv.seps[i].t];
+      }
+      __syncwarp();
+      e = b;
+      b = b1;
+      t = t1;
+      d = d1;
+    }
+  }
+}
+
+// The solved increment of node i.
+template <typename Real>
+__device__ __forceinline__ Real node_increment(const TileView<Real>& tv, int i) {
+  const uint32_t lk = tv.link[i], s = lk >> 16;
+  const Real xt = tv.xsep[lk & 0xFFFF];
+  if (s == kLinkSelf) return xt;
+  const Pair<Real> d = tv.dr[i];
+  const Real x = d.x + d.y * xt;
+  return s == kLinkNone ? x : x + tv.q[i] * tv.xsep[s];
 }
 
 // ------------------------------------------------------------ surrogate ports
@@ -1762,6 +1515,9 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
     write_row(tv, i, pr, dt, G, I);
     if (sp != kNoSpecial) add_node_pulses(tv, pulses, tv.specs[sp], i, pr, a.step0, dt);
   }
+  // inbox entries that no segment fills stay 0; a root reads its own xsep times 0
+  for (int i = tid; i < tv.n_inbox; i += T) tv.inbox[i] = make_pair(Real(0), Real(0));
+  for (int i = tid; i < tv.n_seps; i += T) tv.xsep[i] = Real(0);
   if (tv.has_src)
     for (int c = tid; c < tv.n_cells; c += T) tv.stamp[c] = -1;
   __syncthreads();
@@ -1803,17 +1559,11 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
 #endif
   for (int s = 0; s < a.n_steps; ++s) {
     const int64_t step = a.step0 + s;
-    // forward elimination, leaves first
-    for (int p = 0; p < tv.n_phases; ++p) {
-      eliminate_phase<Real, kSmem>(tv, p, warp, n_warps, lane, dt);
-      __syncthreads();
-    }
+    eliminate_segments<Real, kSmem>(tv, warp, n_warps, lane, dt);
+    __syncthreads();
     BC_TICK(0);
-    // back-substitution, root first
-    for (int p = tv.n_phases - 1; p >= 0; --p) {
-      backsub_phase<Real, kSmem>(tv, p, warp, n_warps, lane, dt);
-      __syncthreads();
-    }
+    sweep_separators<Real>(tv, warp, n_warps, lane);
+    __syncthreads();
     BC_TICK(1);
     // V update, mechanism states, next row, probes and next pulses
     const bool last = s + 1 == a.n_steps;
@@ -1837,7 +1587,7 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
       const Pair<Real> vv = tv.v[i];
       Real hi = vv.x, lo = vv.y;
       const Real v_old = hi, lo_old = lo;
-      ff_add(hi, lo, tv.dr[i].y);
+      ff_add(hi, lo, node_increment(tv, i));
       tv.v[i] = make_pair(hi, lo);
       if (last) {  // last_V of the per-CV spike indicator (cell.py:2384-2386)
         tv.state[size_t(kSlotVLastHi) * tv.N + i] = v_old;
@@ -1991,12 +1741,12 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
   for (int s = 0; s < a.n_steps; ++s) {
     const int64_t step = a.step0 + s;
     // Elimination, deepest node first.  Node k's contribution to its parent stays
-    // in registers (cD, cR) when the parent is node k - 1, the next one visited
+    // in registers (cE, cR) when the parent is node k - 1, the next one visited
     // (the common case along a branch); otherwise it is added to the parent's
     // row in memory, which only a later iteration reads.  Node k - 1's inputs are
     // loaded one iteration ahead: iteration k writes no row but its own and one of
     // a node below k - 1.
-    Real cD = Real(0), cR = Real(0);
+    Real cE = Real(0), cR = Real(0);
     if (n > 1) {
       int i = (n - 1) * L + lane;
       int pv = par[i];
@@ -2013,21 +1763,22 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
           vp1 = tv.v[pv1 * L + lane];
         }
         const Real delta = vdelta<Real>(vi, vp);
-        const Real inv = pivot_rcp(q.x - cD);
+        const Real E = q.x + cE;  // excess form, as in the segment elimination: no subtraction in the pivots
+        const Real inv = pivot_rcp(E + c.x);
         const Real Rp = (q.y + cR) - c.x * delta;
         tv.dr[i] = make_pair(inv, Rp);
         const Real w = c.y * inv;
-        const Real oD = c.x * w, oR = w * Rp + c.y * delta;
+        const Real oE = w * E, oR = w * Rp + c.y * delta;
         if (pv == k - 1) {
-          cD = oD;
+          cE = oE;
           cR = oR;
         } else {
           const int ip = pv * L + lane;
           Pair<Real> pp = tv.dr[ip];
-          pp.x -= oD;
+          pp.x += oE;
           pp.y += oR;
           tv.dr[ip] = pp;
-          cD = Real(0);
+          cE = Real(0);
           cR = Real(0);
         }
         i = i1;
@@ -2043,7 +1794,7 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
     Real x_prev = Real(0);
     if (n > 0) {
       const Pair<Real> q = tv.dr[lane];
-      const Real inv = pivot_rcp(q.x - cD);
+      const Real inv = pivot_rcp(q.x + cE);
       x_prev = (q.y + cR) * inv;
       tv.dr[lane] = make_pair(inv, x_prev);
     }

@@ -56,12 +56,8 @@ struct CellSched;
 // launch classes: 0 packed shared-memory tiles, 1 one big cell per shared-memory
 // tile, 2 global-memory tiles, 3 lane tiles (one small cell per thread)
 constexpr int kMaxClasses = 4;
-// Serial-walk lengths of the warp slots (lane_nodes / narrow_lane_nodes).  Swept on
-// GB300 over the 10,000-cell uneven population (FP32, 1,000 steps per launch):
-// lane_nodes 1 / 4 / 8 / 10 / 12 with narrow phases at 1 ran 2.18 / 2.24 / 2.35 /
-// 2.38 / 2.33e10 compartment-steps/s; narrow phases at 2 instead of 1 cost 23%.
+// Longest unbranched run that one lane eliminates in one piece (lane_nodes).
 constexpr int kDefaultLaneNodes = 10;
-constexpr int kDefaultNarrowLaneNodes = 1;
 
 constexpr uint32_t kMarkovBits = BC_M_NAV16 | BC_M_KCA22 | BC_M_KCA11;
 constexpr uint32_t kCerebellarBits = BC_M_KV34 | BC_M_KV43 | BC_M_KV11 | BC_M_KIR23 | BC_M_HCN1F | BC_M_HCN1H |
@@ -136,7 +132,6 @@ struct bc_plan {
   int threads_global = 512;
   int tile_nodes = 0;
   int lane_nodes = 1;
-  int narrow_lane_nodes = 1;
   int steps_per_launch = 1000;
   int record_every = 1;
   int max_spikes = 64;
@@ -278,15 +273,23 @@ static void free_plan(bc_plan* p) {
 }
 
 // ------------------------------------------------------------------ chain schedule
-struct Chain {
-  std::vector<int32_t> nodes;  // bottom -> top (cell-local node ids)
-  std::vector<int32_t> kids;   // chain ids (cell-local) whose top's parent is nodes[0]
-  int32_t level = 0;
+// A cell's tree cut into segments at its separators (see SegRec).
+struct Seg {
+  std::vector<int32_t> nodes;  // bottom -> top (cell-local node ids), may be empty between two separators
+  int32_t s = -1, t = -1;      // lower (-1: leaf) / upper separator of the cell
 };
-
+struct Sep {
+  int32_t node = -1;
+  int32_t t = -1;              // upper separator, -1 at the root
+  int32_t level = 0;           // 1 + the highest level of the separators below
+  std::vector<int32_t> in;     // segments whose upper separator this is
+};
 struct CellSched {
-  std::vector<Chain> chains;   // ordered by level ascending
-  int32_t max_level = 0;
+  std::vector<Seg> segs;
+  std::vector<Sep> seps;
+  // lowered root .. tree root of the solve; the edges along it are turned around
+  std::vector<int32_t> path;
+  int32_t n_levels = 0;
 };
 
 // fn(i) for i in [0, n) on up to BC_PLAN_THREADS host threads (default: the
@@ -322,71 +325,97 @@ static void parallel_for(int64_t n, F&& fn) {
   for (auto& th : pool) th.join();
 }
 
-static void decompose(const LoweredCell& lc, CellSched& cs) {
+// Segments and separators of one cell.  Runs of more than lane_nodes nodes are cut:
+// a lane's walk costs about 60 cycles a node and a further separator level about
+// 190, so a run of L nodes is cut into about sqrt(L / 3.2) pieces (measured on the
+// 2,500-node tiles of the uneven population).  The cuts depend on the cell alone, so
+// its results do not depend on its tile mates or on the launch shape.
+static void decompose(const LoweredCell& lc, int lane_nodes, CellSched& cs) {
   const int32_t n = lc.n_node;
-  std::vector<int32_t> nchild(n, 0);
-  for (int32_t i = 0; i < n; ++i)
-    if (lc.parent[i] >= 0) nchild[lc.parent[i]]++;
-  std::vector<int32_t> chain_of(n, -1);
-  std::vector<Chain> chains;
+  std::vector<std::array<int32_t, 2>> kid(n, {-1, -1});
+  std::vector<int32_t> nchild(n, 0), parent(lc.parent);
+  int32_t root = 0;
   for (int32_t i = 0; i < n; ++i) {
-    if (nchild[i] == 1) continue;  // interior of some chain
-    Chain ch;
-    int32_t cur = i;
-    ch.nodes.push_back(cur);
-    while (true) {
-      const int32_t p = lc.parent[cur];
-      if (p < 0 || nchild[p] != 1) break;
-      cur = p;
-      ch.nodes.push_back(cur);
+    const int32_t p = lc.parent[i];
+    if (p < 0)
+      root = i;
+    else if (nchild[p]++ == 0)
+      kid[p][0] = i;
+  }
+  // the root of the solve: the first branch point below the lowered root, or the
+  // middle of a tree without one
+  cs.path.assign(1, root);
+  for (int32_t v = root; nchild[v] == 1;) {
+    v = kid[v][0];
+    cs.path.push_back(v);
+  }
+  if (nchild[cs.path.back()] == 0) cs.path.resize(cs.path.size() / 2 + 1);
+  for (size_t k = 0; k + 1 < cs.path.size(); ++k) {  // turn the edges of the path around
+    parent[cs.path[k]] = cs.path[k + 1];
+    --nchild[cs.path[k]];
+    ++nchild[cs.path[k + 1]];
+  }
+  root = cs.path.back();
+  parent[root] = -1;
+  std::vector<int32_t> sep_of(n, -1), start;
+  auto add_sep = [&](int32_t v) {
+    sep_of[v] = int32_t(cs.seps.size());
+    cs.seps.emplace_back();
+    cs.seps.back().node = v;
+  };
+  for (int32_t v = 0; v < n; ++v) {
+    if (v == root || nchild[v] >= 2) add_sep(v);
+    if (v != root && nchild[v] != 1) start.push_back(v);
+  }
+  // separators are indexed by 16 bits in a tile: cut less where a cell has very many
+  const int64_t room = std::max<int64_t>(0, 60000 - int64_t(cs.seps.size()));
+  const int64_t most_per_run = std::max<int64_t>(1, 1 + room / std::max<int64_t>(1, int64_t(start.size())));
+  const int64_t whole = std::min(std::max(lane_nodes, 1), 4096);
+  std::vector<int32_t> run;
+  for (const int32_t v0 : start) {
+    // the run from a leaf (itself the bottom node) or above a separator, up to the next separator
+    run.clear();
+    int32_t lower = sep_of[v0], v = lower >= 0 ? parent[v0] : v0;
+    for (; sep_of[v] < 0; v = parent[v]) run.push_back(v);
+    const int32_t upper = sep_of[v];
+    const int64_t L = int64_t(run.size());
+    int64_t pieces = 1;
+    if (L > whole) pieces = std::max<int64_t>(1, std::llround(std::sqrt(double(L) / 3.2)));
+    pieces = std::min({pieces, most_per_run, (L + 1) / 2});
+    pieces = std::max<int64_t>(pieces, 1);
+    int64_t k0 = 0;
+    for (int64_t q = 0; q < pieces; ++q) {
+      // pieces - 1 of the L nodes become separators; the others are shared out evenly
+      const int64_t k1 = k0 + (L - (pieces - 1)) * (q + 1) / pieces - (L - (pieces - 1)) * q / pieces;
+      Seg sg;
+      sg.nodes.assign(run.begin() + k0, run.begin() + k1);
+      sg.s = lower;
+      if (q + 1 < pieces) {
+        add_sep(run[k1]);
+        sg.t = sep_of[run[k1]];
+      } else {
+        sg.t = upper;
+      }
+      if (sg.s >= 0) cs.seps[sg.s].t = sg.t;
+      lower = sg.t;
+      cs.segs.push_back(std::move(sg));
+      k0 = k1 + 1;
     }
-    for (int32_t v : ch.nodes) chain_of[v] = int32_t(chains.size());
-    chains.push_back(std::move(ch));
   }
-  // child chains: top's parent is a bottom of another chain
-  for (size_t c = 0; c < chains.size(); ++c) {
-    const int32_t top = chains[c].nodes.back();
-    const int32_t p = lc.parent[top];
-    if (p >= 0) chains[chain_of[p]].kids.push_back(int32_t(c));
-  }
-  // levels (iterative: process chains in order of decreasing depth)
-  std::vector<int32_t> order(chains.size());
-  std::iota(order.begin(), order.end(), 0);
-  // depth of the bottom node from the root
-  std::vector<int32_t> depth(n, -1);
-  for (int32_t i = 0; i < n; ++i) {
-    if (depth[i] >= 0) continue;
-    std::vector<int32_t> path;
-    int32_t cur = i;
-    while (cur >= 0 && depth[cur] < 0) {
-      path.push_back(cur);
-      cur = lc.parent[cur];
-    }
-    int32_t d = cur >= 0 ? depth[cur] : -1;
-    for (auto it = path.rbegin(); it != path.rend(); ++it) depth[*it] = ++d;
-  }
-  std::sort(order.begin(), order.end(),
-            [&](int32_t a, int32_t b) { return depth[chains[a].nodes[0]] > depth[chains[b].nodes[0]]; });
-  for (int32_t c : order) {
-    int32_t lv = 0;
-    for (int32_t k : chains[c].kids) lv = std::max(lv, chains[k].level + 1);
-    chains[c].level = lv;
-  }
-  // reorder by level ascending, remap kid ids
-  std::vector<int32_t> by_level(chains.size());
-  std::iota(by_level.begin(), by_level.end(), 0);
-  std::stable_sort(by_level.begin(), by_level.end(),
-                   [&](int32_t a, int32_t b) { return chains[a].level < chains[b].level; });
-  std::vector<int32_t> newid(chains.size());
-  for (size_t k = 0; k < by_level.size(); ++k) newid[by_level[k]] = int32_t(k);
-  cs.chains.clear();
-  cs.chains.reserve(chains.size());
-  cs.max_level = 0;
-  for (int32_t old : by_level) {
-    Chain ch = std::move(chains[old]);
-    for (auto& k : ch.kids) k = newid[k];
-    cs.max_level = std::max(cs.max_level, ch.level);
-    cs.chains.push_back(std::move(ch));
+  for (size_t k = 0; k < cs.segs.size(); ++k) cs.seps[cs.segs[k].t].in.push_back(int32_t(k));
+  // levels, children before parents
+  const int32_t ns = int32_t(cs.seps.size());
+  std::vector<int32_t> waits(ns, 0), ready;
+  for (const Sep& sp : cs.seps)
+    if (sp.t >= 0) waits[sp.t]++;
+  for (int32_t j = 0; j < ns; ++j)
+    if (waits[j] == 0) ready.push_back(j);
+  for (size_t k = 0; k < ready.size(); ++k) {
+    const Sep& sp = cs.seps[ready[k]];
+    cs.n_levels = std::max(cs.n_levels, sp.level + 1);
+    if (sp.t < 0) continue;
+    cs.seps[sp.t].level = std::max(cs.seps[sp.t].level, sp.level + 1);
+    if (--waits[sp.t] == 0) ready.push_back(sp.t);
   }
 }
 
@@ -426,8 +455,6 @@ struct BuildCtx {
   const std::vector<std::vector<int64_t>>* port_pulse_ids;
   int precision;
   int state_slots;
-  int lane_nodes;  // nodes a lane walks serially in a warp slot
-  int narrow_lane_nodes;  // the same in phases with fewer nodes than 32 x warps
   int param_stride;       // reals per parameter record in the tile blobs
 };
 
@@ -440,180 +467,146 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   const bc_batch_spec& s = *cx.spec;
   const int R = s.n_regions;
   const size_t rs = cx.precision == BC_PREC_F64 ? 8 : 4;
-  std::vector<int64_t> cell_list = tb.cells;
-  std::vector<std::pair<int64_t, size_t>> cmap;
-  for (size_t i = 0; i < cell_list.size(); ++i) cmap.push_back({cell_list[i], i});
-  std::sort(cmap.begin(), cmap.end());
-  // -------- chains -> phases -> warp slots
-  // One record per chain.  The phase of a chain is its chain level (children first).
-  // Inside a phase, chains of at most 32 nodes are packed first-fit-decreasing into
-  // 32-lane warp slots, one node per lane; a longer chain gets a slot of its own in
-  // which every lane takes a contiguous chunk of ceil(L / 32) nodes.
-  struct CRef {
-    int32_t li, chain, L;
-  };
-  struct RecSpec {
-    int32_t li, chain, kind, seg, K, lo, hi;
-  };
+  const std::vector<int64_t>& cell_list = tb.cells;
   int64_t n_real = 0;
   std::vector<std::vector<int32_t>> node_tile(cell_list.size());
-  std::vector<std::vector<int32_t>> handle(cell_list.size());  // chain -> record
   for (size_t li = 0; li < cell_list.size(); ++li) {
     const LoweredCell& lc = (*cx.cells)[cell_list[li]];
-    const CellSched& cs = (*cx.sched)[cell_list[li]];
     node_tile[li].assign(lc.n_node, -1);
-    handle[li].assign(cs.chains.size(), -1);
     n_real += lc.n_node;
   }
   const int W = std::max(1, T / 32);
-  const int C_wide = std::max(1, cx.lane_nodes);
-  const int C_narrow = cx.narrow_lane_nodes > 0 ? cx.narrow_lane_nodes : C_wide;
-  std::vector<ChainRec> chains;
-  std::vector<RecSpec> rec_src;
+  const bool lane = tb.cls == 3;  // a lane tile has no segments, separators or warp slots
+  auto sched_of = [&](size_t li) -> const CellSched& { return (*cx.sched)[cell_list[li]]; };
+  std::vector<SegRec> segs;
   std::vector<SlotRec> slots;
-  int32_t next_node = 0;
-  int64_t crit = 0;
-  std::vector<std::vector<CRef>> levels;
-  for (size_t li = 0; li < cell_list.size(); ++li) {
-    const CellSched& cs = (*cx.sched)[cell_list[li]];
-    for (size_t k = 0; k < cs.chains.size(); ++k) {
-      const int32_t lv = cs.chains[k].level;
-      if (int(levels.size()) <= lv) levels.resize(lv + 1);
-      levels[lv].push_back({int32_t(li), int32_t(k), int32_t(cs.chains[k].nodes.size())});
+  std::vector<SepRec> seps;
+  std::vector<GroupRec> groups;
+  std::vector<int32_t> levels;
+  std::vector<uint32_t> link;
+  int32_t next_node = 0, sep0 = 0, n_inbox = 0;
+  int n_levels = 0;
+  int64_t crit = 0, n_lower = 0;  // nodes of segments with a lower separator (they come first)
+  if (!lane) {
+    // -------- separators: cells dealt to the warps (longest sweep first, to the warp with the least), then
+    // a tile index per separator by warp, level and cell
+    struct Cost {
+      int64_t cost;
+      size_t li;
+    };
+    std::vector<Cost> by_cost;
+    size_t n_sep = 0;
+    for (size_t li = 0; li < cell_list.size(); ++li) {
+      by_cost.push_back({int64_t(sched_of(li).n_levels) + int64_t(sched_of(li).seps.size()) / 32, li});
+      n_sep += sched_of(li).seps.size();
     }
-  }
-  const bool lane = tb.cls == 3;  // a lane tile has no chains, phases or warp slots
-  std::vector<std::vector<CRef>> phases;
-  for (auto& v : levels)
-    if (!v.empty() && !lane) phases.push_back(std::move(v));
-  const int n_phases = int(phases.size());
-  std::vector<int32_t> phase_ptr(size_t(n_phases) + 1, 0);
-  // A lane plan: the chains (whole, or one chain's part) of one lane.
-  struct Lane {
-    std::vector<CRef> whole;  // serial slots: whole chains
-    int32_t nodes = 0;
-  };
-  struct Slot {
-    bool scan = false;
-    std::vector<Lane> lanes;              // serial slots
-    std::vector<CRef> spread;             // scan slots: chains, each over `parts` lanes
-    std::vector<std::vector<int32_t>> parts;  // per spread chain: part sizes
-    int32_t used = 0, steps = 0, cost = 0;
-  };
-  for (int p = 0; p < n_phases; ++p) {
-    std::vector<CRef>& v = phases[p];
-    std::stable_sort(v.begin(), v.end(), [](const CRef& a, const CRef& b) { return a.L > b.L; });
-    // a phase with fewer nodes than one unit slot per warp is latency-bound: short
-    // chains there are walked serially (C_narrow) rather than scanned
-    int64_t phase_nodes = 0;
-    for (const CRef& c : v) phase_nodes += c.L;
-    const int C = phase_nodes < int64_t(32) * W ? C_narrow : C_wide;
-    std::vector<Slot> ps;
-    // chains longer than a lane's share: split into near-equal parts over lanes
-    std::vector<Lane> lanes;
-    for (const CRef& c : v) {
-      if (c.L > C) {
-        int32_t m = (c.L + C - 1) / C;
-        int32_t chunk = C;
-        if (m > 32) {
-          chunk = (c.L + 31) / 32;
-          m = (c.L + chunk - 1) / chunk;
-        }
-        std::vector<int32_t> sizes(m);
-        for (int32_t q = 0; q < m; ++q) sizes[q] = int32_t(int64_t(c.L) * (q + 1) / m - int64_t(c.L) * q / m);
-        int32_t st = 0;
-        while ((1 << st) < m) ++st;
-        Slot* tgt = nullptr;
-        for (Slot& s : ps)
-          if (s.scan && s.used + m <= 32) {
-            tgt = &s;
-            break;
-          }
-        if (!tgt) {
-          ps.emplace_back();
-          tgt = &ps.back();
-          tgt->scan = true;
-        }
-        tgt->spread.push_back(c);
-        tgt->parts.push_back(sizes);
-        tgt->used += m;
-        tgt->steps = std::max(tgt->steps, st);
-        tgt->cost = std::max<int32_t>(tgt->cost, 4 * sizes[0] + 8 * st);
-        continue;
-      }
-      // whole chain: first lane with room (lanes fill to C nodes)
-      bool placed = false;
-      for (Lane& ln : lanes)
-        if (ln.nodes + c.L <= C) {
-          ln.whole.push_back(c);
-          ln.nodes += c.L;
-          placed = true;
-          break;
-        }
-      if (!placed) {
-        Lane ln;
-        ln.whole.push_back(c);
-        ln.nodes = c.L;
-        lanes.push_back(std::move(ln));
-      }
+    if (n_sep >= kLinkSelf) return fail(BC_ERR_CAPACITY, "too many branch points in one tile");
+    std::stable_sort(by_cost.begin(), by_cost.end(), [](const Cost& a, const Cost& b) { return a.cost > b.cost; });
+    const size_t n_groups = std::min(cell_list.size(), size_t(W));
+    std::vector<std::vector<size_t>> members(n_groups);
+    std::vector<int64_t> group_seps(n_groups, 0);
+    for (size_t k = 0; k < by_cost.size(); ++k) {
+      const size_t g = k < n_groups ? k
+                                    : size_t(std::min_element(group_seps.begin(), group_seps.end()) - group_seps.begin());
+      members[g].push_back(by_cost[k].li);
+      group_seps[g] += int64_t(sched_of(by_cost[k].li).seps.size());
     }
-    for (size_t q = 0; q < lanes.size(); q += 32) {
-      Slot s;
-      for (size_t r = q; r < std::min(lanes.size(), q + 32); ++r) {
-        s.cost = std::max<int32_t>(s.cost, 2 * lanes[r].nodes);
-        s.lanes.push_back(std::move(lanes[r]));
+    std::vector<std::vector<int32_t>> sep_tile(cell_list.size());
+    for (size_t li = 0; li < cell_list.size(); ++li) sep_tile[li].resize(sched_of(li).seps.size());
+    std::vector<std::pair<size_t, int32_t>> sep_src;  // (cell of the tile, separator of the cell) by tile index
+    for (auto& m : members) {
+      std::vector<std::vector<std::pair<size_t, int32_t>>> lv;
+      for (const size_t li : m) {
+        const CellSched& cs = sched_of(li);
+        if (lv.size() < size_t(cs.n_levels)) lv.resize(cs.n_levels);
+        for (size_t j = 0; j < cs.seps.size(); ++j) lv[cs.seps[j].level].push_back({li, int32_t(j)});
       }
-      s.used = int32_t(s.lanes.size());
-      ps.push_back(std::move(s));
+      groups.push_back({int32_t(levels.size()), int32_t(lv.size())});
+      n_levels = std::max(n_levels, int(lv.size()));
+      for (auto& v : lv) {
+        levels.push_back(int32_t(sep_src.size()));
+        for (auto& x : v) {
+          sep_tile[x.first][x.second] = int32_t(sep_src.size());
+          sep_src.push_back(x);
+        }
+      }
+      levels.push_back(int32_t(sep_src.size()));
     }
-    // dearest slots first: warp w takes slots w, w + W, ...
-    std::stable_sort(ps.begin(), ps.end(), [](const Slot& a, const Slot& b) { return a.cost > b.cost; });
-    std::vector<int64_t> warp_cost(W, 0);
-    phase_ptr[p] = int32_t(slots.size());
-    for (size_t si = 0; si < ps.size(); ++si) {
-      const Slot& s = ps[si];
-      SlotRec sr{};
-      sr.n_begin = next_node;
-      sr.steps = uint8_t(s.scan ? std::max(1, s.steps) : 0);
-      int lane = 0;
-      auto emit_chain = [&](const CRef& c) {
-        const Chain& ch = (*cx.sched)[cell_list[c.li]].chains[c.chain];
-        ChainRec rec{};
-        rec.start = next_node;
-        rec.count = c.L;
-        rec.kind = kChainRegular;
-        rec.slot = -1;
-        for (int32_t q = 0; q < c.L; ++q) node_tile[c.li][ch.nodes[q]] = next_node++;
-        handle[c.li][c.chain] = int32_t(chains.size());
-        chains.push_back(rec);
-        rec_src.push_back({c.li, c.chain, kChainRegular, 0, 1, 0, c.L});
+    // -------- inboxes: one entry per segment, consecutive per upper separator, padded to pairs
+    std::vector<std::vector<int32_t>> seg_inbox(cell_list.size());
+    for (size_t li = 0; li < cell_list.size(); ++li) seg_inbox[li].resize(sched_of(li).segs.size());
+    seps.resize(sep_src.size());
+    for (size_t j = 0; j < sep_src.size(); ++j) {
+      const auto [li, q] = sep_src[j];
+      const Sep& sp = sched_of(li).seps[q];
+      const size_t pairs = std::max<size_t>(1, (sp.in.size() + 1) / 2);
+      if (pairs > 0xFFFF) return fail(BC_ERR_CAPACITY, "too many branches at one point");
+      seps[j] = SepRec{n_inbox / 2, -1, uint16_t(pairs), uint16_t(sp.t >= 0 ? size_t(sep_tile[li][sp.t]) : j), 0};
+      for (size_t k = 0; k < sp.in.size(); ++k) seg_inbox[li][sp.in[k]] = n_inbox + int32_t(k);
+      n_inbox += int32_t(2 * pairs);
+    }
+    for (size_t li = 0; li < cell_list.size(); ++li)
+      for (size_t k = 0; k < sched_of(li).segs.size(); ++k) {
+        const Seg& sg = sched_of(li).segs[k];
+        if (sg.s >= 0) seps[sep_tile[li][sg.s]].inbox = seg_inbox[li][k];
+      }
+    for (SepRec& sp : seps)
+      if (sp.inbox < 0) sp.inbox = n_inbox++;
+    // -------- warp slots: segments with a lower separator first, then the leaves', longest first
+    std::vector<std::pair<size_t, int32_t>> seg_src;
+    for (int lower = 1; lower >= 0; --lower) {
+      std::vector<std::pair<size_t, int32_t>> v;
+      for (size_t li = 0; li < cell_list.size(); ++li)
+        for (size_t k = 0; k < sched_of(li).segs.size(); ++k)
+          if ((sched_of(li).segs[k].s >= 0) == (lower == 1)) v.push_back({li, int32_t(k)});
+      // the roots' segments to themselves (k = -1)
+      for (size_t li = 0; lower == 1 && li < cell_list.size(); ++li) v.push_back({li, -1});
+      auto len = [&](const std::pair<size_t, int32_t>& x) {
+        return x.second < 0 ? size_t(0) : sched_of(x.first).segs[x.second].nodes.size();
       };
-      if (s.scan) {
-        for (size_t ci = 0; ci < s.spread.size(); ++ci) {
-          const int32_t base = next_node - sr.n_begin;
-          int32_t o = base;
-          for (int32_t sz : s.parts[ci]) {
-            sr.off[lane++] = uint16_t(o);
-            o += sz;
+      std::stable_sort(v.begin(), v.end(), [&](const auto& x, const auto& y) { return len(x) > len(y); });
+      for (size_t q = 0; q < v.size(); q += 32) {
+        const size_t n_lanes = std::min<size_t>(32, v.size() - q);
+        SlotRec sr{next_node, int32_t(segs.size()), int16_t(n_lanes), uint16_t(len(v[q])), lower};
+        for (size_t l = 0; l < n_lanes; ++l) {
+          const auto& st = sep_tile[v[q + l].first];
+          if (v[q + l].second < 0) {
+            const CellSched& cs = sched_of(v[q + l].first);
+            const size_t r = size_t(std::find_if(cs.seps.begin(), cs.seps.end(), [](const Sep& x) { return x.t < 0; }) -
+                                    cs.seps.begin());
+            segs.push_back(SegRec{uint16_t(st[r]), uint16_t(st[r]), 0, 0, 0, 0});
+            continue;
           }
-          emit_chain(s.spread[ci]);
+          const Seg& sg = sched_of(v[q + l].first).segs[v[q + l].second];
+          if (sg.nodes.size() > 0xFFFF) return fail(BC_ERR_CAPACITY, "an unbranched run holds too many nodes");
+          segs.push_back(SegRec{uint16_t(st[sg.t]), uint16_t(sg.s >= 0 ? uint32_t(st[sg.s]) : kLinkNone),
+                                uint16_t(sg.nodes.size()), 0, seg_inbox[v[q + l].first][v[q + l].second], 0});
         }
-      } else {
-        for (const Lane& ln : s.lanes) {
-          sr.off[lane++] = uint16_t(next_node - sr.n_begin);
-          for (const CRef& c : ln.whole) emit_chain(c);
-        }
+        for (size_t k = 0; k < sr.max_len; ++k)
+          for (size_t l = 0; l < n_lanes && len(v[q + l]) > k; ++l) {
+            const Seg& sg = sched_of(v[q + l].first).segs[v[q + l].second];
+            node_tile[v[q + l].first][sg.nodes[k]] = next_node++;
+            const SegRec& rec = segs[sr.seg0 + l];
+            link.push_back(uint32_t(rec.t) | (uint32_t(rec.s) << 16));
+          }
+        slots.push_back(sr);
       }
-      if (next_node - sr.n_begin > 0x7fff) return fail(BC_ERR_CAPACITY, "a warp slot holds more than 32767 nodes");
-      sr.n_count = int16_t(next_node - sr.n_begin);
-      sr.unit = uint8_t(s.scan && sr.n_count == lane ? 1 : 0);
-      for (; lane < 32; ++lane) sr.off[lane] = uint16_t(sr.n_count);
-      slots.push_back(sr);
-      warp_cost[si % W] += s.cost;
+      if (lower == 1) n_lower = next_node;
     }
-    crit += *std::max_element(warp_cost.begin(), warp_cost.end());
+    // warp w takes slots w, w + W, ...: the dearest first
+    std::stable_sort(slots.begin(), slots.end(), [](const SlotRec& a, const SlotRec& b) {
+      return int(a.max_len) + 2 * a.lower > int(b.max_len) + 2 * b.lower;
+    });
+    sep0 = next_node;
+    for (size_t j = 0; j < sep_src.size(); ++j) {
+      node_tile[sep_src[j].first][sched_of(sep_src[j].first).seps[sep_src[j].second].node] = next_node++;
+      link.push_back(uint32_t(j) | (kLinkSelf << 16));
+    }
+    // relative length of a step (it orders tiles): the walks of the dearest warp, the sweep, the update
+    std::vector<int64_t> warp_cost(W, 0);
+    for (size_t k = 0; k < slots.size(); ++k) warp_cost[k % W] += 2 * slots[k].max_len;
+    crit = *std::max_element(warp_cost.begin(), warp_cost.end()) + 2 * n_levels + n_real / 32;
   }
-  phase_ptr[n_phases] = int32_t(slots.size());
   out.crit = crit;
   // lane tile: node v of the cell in lane l is tile node v * T + l
   std::vector<int32_t> lane_n;
@@ -631,37 +624,9 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     n_real = int64_t(lane_kmax) * T;
     out.crit = lane_kmax;
   }
-  if (chains.size() >= 0xFFFF) return fail(BC_ERR_CAPACITY, "too many chains in one tile");
-  // -------- links: parents and contribution slots
-  // A record owns the consecutive contribution slots aux .. aux + n_child, one per
-  // child chain; each child writes its (cD, cR) into its own slot.
-  int32_t n_slots = 0;
-  for (size_t k = 0; k < chains.size(); ++k) {
-    const RecSpec& rsp = rec_src[k];
-    const LoweredCell& lc = (*cx.cells)[cell_list[rsp.li]];
-    const Chain& ch = (*cx.sched)[cell_list[rsp.li]].chains[rsp.chain];
-    const int32_t chain_top_parent = lc.parent[ch.nodes.back()];
-    ChainRec& rec = chains[k];
-    rec.top_parent = chain_top_parent >= 0 ? node_tile[rsp.li][chain_top_parent] : -1;
-    rec.first = 1;
-    rec.aux = n_slots;
-    rec.n_child = int32_t(ch.kids.size());
-    n_slots += rec.n_child;
-  }
-  for (size_t k = 0; k < chains.size(); ++k) {
-    const RecSpec& rsp = rec_src[k];
-    const Chain& ch = (*cx.sched)[cell_list[rsp.li]].chains[rsp.chain];
-    for (size_t j = 0; j < ch.kids.size(); ++j) {
-      const int32_t kid_rec = handle[rsp.li][ch.kids[j]];
-      if (kid_rec < 0) return fail(BC_ERR_INVALID, "internal: unresolved chain link");
-      chains[kid_rec].slot = chains[k].aux + int32_t(j);
-    }
-  }
-  // per-node record index
-  std::vector<uint16_t> crec(size_t(n_real), 0);
-  for (size_t k = 0; k < chains.size(); ++k)
-    for (int32_t q = 0; q < chains[k].count; ++q) crec[size_t(chains[k].start + q)] = uint16_t(k);
+  std::vector<uint16_t> crec;
   if (lane) {  // lane tiles: the parent's node index v within the cell (0xFFFF at the root)
+    crec.assign(size_t(n_real), 0);
     for (size_t li = 0; li < cell_list.size(); ++li) {
       const LoweredCell& lc = (*cx.cells)[cell_list[li]];
       for (int32_t v = 0; v < lc.n_node; ++v)
@@ -701,7 +666,6 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   if (cell_list.size() >= 0xFFFF) return fail(BC_ERR_CAPACITY, "too many cells in one tile");
   // -------- layout
   const int64_t N = (n_real + 3) & ~int64_t(3);
-  const int S = cx.state_slots;
   const int64_t n_params = int64_t(cell_list.size()) * R;
   if (n_params >= 0xFFFF) return fail(BC_ERR_CAPACITY, "too many parameter records in one tile");
   TileDesc d{};
@@ -712,22 +676,26 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   d.dyn_bytes = int32_t(off);
   d.off_ab = int32_t(off);
   off = align16(off + 2 * N * rs);
-  d.off_diag0 = int32_t(off);
-  off = align16(off + N * rs);
   d.off_pidx = int32_t(off);
   off = align16(off + N * 2);
   d.off_spec = int32_t(off);
   off = align16(off + N * 2);
   d.off_specs = int32_t(off);
   off = align16(off + spec_nodes.size() * sizeof(SpecRec));
-  d.off_chains = int32_t(off);
-  off = align16(off + chains.size() * sizeof(ChainRec));
+  d.off_link = int32_t(off);
+  off = align16(off + link.size() * 4);
+  d.off_segs = int32_t(off);
+  off = align16(off + segs.size() * sizeof(SegRec));
   d.off_slots = int32_t(off);
   off = align16(off + slots.size() * sizeof(SlotRec));
-  d.off_phase = int32_t(off);
-  off = align16(off + phase_ptr.size() * 4);
+  d.off_seps = int32_t(off);
+  off = align16(off + seps.size() * sizeof(SepRec));
+  d.off_levels = int32_t(off);
+  off = align16(off + levels.size() * 4);
+  d.off_groups = int32_t(off);
+  off = align16(off + groups.size() * sizeof(GroupRec));
   d.off_crec = int32_t(off);
-  off = align16(off + N * 2);
+  off = align16(off + crec.size() * 2);
   d.off_params = int32_t(off);
   off = align16(off + size_t(n_params) * cx.param_stride * rs);
   d.off_mech = int32_t(off);
@@ -756,11 +724,16 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   size_t so = 0;
   d.off_dr = int32_t(so);
   so = align16(so + 2 * N * rs);
-  d.off_scd = int32_t(so);
-  so = align16(so + size_t(std::max(n_slots, 1)) * rs);
-  d.off_scr = int32_t(so);
-  so = align16(so + size_t(std::max(n_slots, 1)) * rs);
-  d.n_slots = n_slots;
+  d.off_inbox = int32_t(so);
+  so = align16(so + 2 * size_t(n_inbox) * rs);
+  d.off_srow = int32_t(so);
+  so = align16(so + 4 * seps.size() * rs);
+  d.off_own = int32_t(so);
+  so = align16(so + 2 * seps.size() * rs);
+  d.off_q = int32_t(so);
+  so = align16(so + size_t(n_lower) * rs);
+  d.off_xsep = int32_t(so);
+  so = align16(so + seps.size() * rs);
   d.off_stamp = -1;
   if (has_src) {
     d.off_stamp = int32_t(so);
@@ -776,8 +749,13 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   d.scratch_bytes = int32_t(so);
   d.n_nodes = int32_t(N);
   d.n_real_nodes = int32_t(n_real);
-  d.n_chains = int32_t(chains.size());
-  d.n_phases = n_phases;
+  d.n_segs = int32_t(segs.size());
+  d.n_phases = lane ? 0 : 1 + n_levels;
+  d.n_slots = int32_t(slots.size());
+  d.n_seps = int32_t(seps.size());
+  d.n_inbox = n_inbox;
+  d.n_groups = int32_t(groups.size());
+  d.sep0 = sep0;
   d.n_params = int32_t(n_params);
   // -------- fill
   std::vector<unsigned char>& b = out.blob;
@@ -802,10 +780,19 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
       putr(d.off_v, 2 * size_t(j), lc.node_vrest[v]);
       putr(d.off_ab, 2 * size_t(j), lc.alpha[v]);
       putr(d.off_ab, 2 * size_t(j) + 1, lc.beta[v]);
-      putr(d.off_diag0, j, lc.diag[v]);
       const uint16_t pi = lc.region[v] >= 0 ? uint16_t(li * R + lc.region[v]) : uint16_t(0xFFFF);
       std::memcpy(b.data() + d.off_pidx + size_t(j) * 2, &pi, 2);
       out.vinit[j] = lc.node_vrest[v];
+    }
+    if (!lane) {
+      // the solve's root is path.back(): along the path the old parent is the child
+      const std::vector<int32_t>& path = sched_of(li).path;
+      for (size_t k = 0; k < path.size(); ++k) {
+        const size_t j = size_t(node_tile[li][path[k]]);
+        const bool top = k + 1 == path.size();
+        putr(d.off_ab, 2 * j, top ? 0.0 : lc.beta[path[k + 1]]);
+        putr(d.off_ab, 2 * j + 1, top ? 0.0 : lc.alpha[path[k + 1]]);
+      }
     }
     for (int r = 0; r < R; ++r) {
       const int64_t rc = c * R + r;
@@ -935,10 +922,16 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     }
   }
   d.n_ports = int32_t(out.ports.size());
-  std::memcpy(b.data() + d.off_chains, chains.data(), chains.size() * sizeof(ChainRec));
-  if (!slots.empty()) std::memcpy(b.data() + d.off_slots, slots.data(), slots.size() * sizeof(SlotRec));
-  std::memcpy(b.data() + d.off_phase, phase_ptr.data(), phase_ptr.size() * 4);
-  std::memcpy(b.data() + d.off_crec, crec.data(), crec.size() * 2);
+  auto put_all = [&](int32_t at, const void* src, size_t bytes) {
+    if (bytes) std::memcpy(b.data() + at, src, bytes);
+  };
+  put_all(d.off_link, link.data(), link.size() * 4);
+  put_all(d.off_segs, segs.data(), segs.size() * sizeof(SegRec));
+  put_all(d.off_slots, slots.data(), slots.size() * sizeof(SlotRec));
+  put_all(d.off_seps, seps.data(), seps.size() * sizeof(SepRec));
+  put_all(d.off_levels, levels.data(), levels.size() * 4);
+  put_all(d.off_groups, groups.data(), groups.size() * sizeof(GroupRec));
+  put_all(d.off_crec, crec.data(), crec.size() * 2);
   out.desc = d;
   return BC_OK;
 }
@@ -1245,7 +1238,6 @@ void bc_default_options(bc_plan_options* o) {
   o->threads_per_tile = 0;
   o->tile_nodes = 0;
   o->lane_nodes = kDefaultLaneNodes;
-  o->narrow_lane_nodes = kDefaultNarrowLaneNodes;
   o->steps_per_launch = 0;
   o->record_every = 1;
   o->max_spikes = 64;
@@ -1284,7 +1276,6 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   p->use_graph = opts.use_graph;
   p->steps_per_launch = opts.steps_per_launch > 0 ? opts.steps_per_launch : 1000;
   p->lane_nodes = opts.lane_nodes > 0 ? opts.lane_nodes : kDefaultLaneNodes;
-  p->narrow_lane_nodes = opts.narrow_lane_nodes > 0 ? opts.narrow_lane_nodes : kDefaultNarrowLaneNodes;
   p->n_cells = s.n_cells;
   // ---------------------------------------------------- lower
   std::vector<LoweredCell> cells(s.n_cells);
@@ -1558,7 +1549,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     std::vector<char> dbad(s.n_cells, 0);
     parallel_for(s.n_cells, [&](int64_t c) {
       try {
-        decompose(cells[c], sched[c]);
+        decompose(cells[c], p->lane_nodes, sched[c]);
       } catch (const std::exception& ex) {
         dbad[c] = 1;
         dmsg[c] = std::string("scheduling cell ") + std::to_string(c) + ": " + ex.what();
@@ -1579,10 +1570,10 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   }
   const size_t static_smem = 1024;  // static shared memory of the kernel (mbarrier, status) + slack
   const size_t smem_budget = smem_cap - static_smem;
-  // bytes per node (approx.) for packing: V hi/lo, states, alpha/beta/diag0, parent, pidx, scratch diag/rhs
-  // shared bytes per node: V hi/lo, alpha/beta/diag0, scratch diag/rhs/fill (Real),
-  // region index (2 B), plus ~1 chain record per 5 nodes (record, child slot, cD/cR/H)
-  const double bpn = double(8 * rs + 2) + (28.0 + 4.0 + 3.0 * double(rs)) / 5.0;
+  // shared bytes per node, for packing: V, (alpha, beta) and row pairs, link and region / special indices, and
+  // per 6.4 nodes a segment (record, inbox), per 16 a separator, a third of the nodes with a q entry
+  const double bpn = 6.0 * double(rs) + 8.0 + (16.0 + 2.0 * double(rs)) / 6.4 + (20.0 + 9.0 * double(rs)) / 16.0 +
+                     double(rs) / 3.0;
   int tile_nodes = opts.tile_nodes;
   if (tile_nodes <= 0) tile_nodes = 900;
   tile_nodes = std::max(tile_nodes, 16);
@@ -1662,7 +1653,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     if (tile_nodes - nn > 0) room.emplace(tile_nodes - nn, builds.size() - 1);
   }
   BuildCtx cx{&s, &cells, &sched, &cv_base, &cell_pulses, &cell_probes, &pulse_node, &probe_node, &cell_syns, &is_src,
-              &cell_ports, &port_pulse_ids, p->precision, S, p->lane_nodes, p->narrow_lane_nodes,
+              &cell_ports, &port_pulse_ids, p->precision, S,
               p->extra ? ((all_bits & BC_M_EXT) ? kParamStride : kParamStrideExtra) : kParamStrideCore};
   std::vector<TileOut> outs;
   outs.reserve(builds.size());
@@ -1832,7 +1823,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   p->tile_stats.clear();
   for (size_t k = 0; k < tord.size(); ++k) {
     const TileDesc& d = p->tiles[k];
-    p->tile_stats.push_back({int64_t(d.n_real_nodes), int64_t(d.n_chains), int64_t(d.n_phases),
+    p->tile_stats.push_back({int64_t(d.n_real_nodes), int64_t(d.n_segs), int64_t(d.n_phases),
                              int64_t(outs_crit[tord[k]]), int64_t(builds[tord[k]].cls),
                              int64_t(d.blob_bytes) + int64_t(d.scratch_bytes)});
   }

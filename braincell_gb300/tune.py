@@ -3,8 +3,7 @@
 The step kernel's speed depends on four plan options:
 - ``tile_nodes``: how many cells share a CTA, hence CTAs per SM;
 - ``threads_per_tile``: warps that take warp slots in parallel;
-- ``lane_nodes``: the switch between shuffle-scanned chains and chains walked
-  serially by one lane;
+- ``lane_nodes``: the longest unbranched run one lane eliminates in one piece;
 - ``steps_per_launch``: how many steps one launch fuses.
 
 Their best values depend on the morphologies of the batch.  :func:`autotune` times

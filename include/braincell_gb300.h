@@ -394,8 +394,8 @@ typedef struct bc_plan_options {
   int32_t precision;        /* BC_PREC_*                                             */
   int32_t threads_per_tile; /* CTA size (multiple of 32, <= 1024); 0 = auto          */
   int32_t tile_nodes;       /* node budget per tile (shared-memory size); 0 = auto   */
-  int32_t lane_nodes;       /* nodes a lane walks serially inside a warp slot; longer
-                               chains are spread over lanes joined by shuffle scans;
+  int32_t lane_nodes;       /* unbranched runs of more nodes are cut into about
+                               sqrt(nodes / 3.2) pieces, each walked by one lane;
                                0 = auto (10)                                         */
   int32_t steps_per_launch; /* time steps fused per kernel launch; 0 = auto          */
   int32_t record_every;     /* probe sampling period in steps (>= 1)                 */
@@ -408,8 +408,8 @@ typedef struct bc_plan_options {
   int32_t threads_big;      /* CTA size for tiles holding one cell larger than
                                tile_nodes; 0 = auto                                   */
   int32_t threads_global;   /* CTA size for global-memory tiles; 0 = auto            */
-  int32_t narrow_lane_nodes; /* lane_nodes for narrow phases (fewer nodes than one
-                               warp slot per warp); 0 = auto (1)                  */
+  int32_t narrow_lane_nodes; /* accepted and without effect: all runs of a tile are
+                               eliminated in one pass, so there are no narrow phases */
   float reserved_b;         /* must be 0                                             */
   int32_t dry_run;          /* 1: lower and schedule only (no CUDA calls); the plan
                                answers bc_plan_info / bc_plan_tile_stats only         */
