@@ -65,6 +65,10 @@ constexpr int kParamStrideCore = BC_P_CA_CI0 + 2;
 // nodes, grouped by the warp that sweeps them and, inside a group, by level
 // (children before parents).
 // The root, whose row needs no elimination, has a segment of no nodes to itself.
+//
+// Cells of at most kCellLaneNodes nodes are not cut: a lane solves a whole one, its
+// nodes in the order of elimination (runs bottom -> top, child runs first) and stored
+// jagged like a segment's.
 struct alignas(16) SegRec {
   uint16_t t, s;   // upper / lower separator (tile separator index); s = kLinkNone at a leaf
   uint16_t len;    // nodes
@@ -74,11 +78,15 @@ struct alignas(16) SegRec {
 };
 struct alignas(16) SlotRec {
   int32_t n_begin;   // first node
-  int32_t seg0;      // first segment (lane 0)
+  int32_t seg0;      // first segment (lane 0); whole cells: first of the slot's max_len + 1 row starts
   int16_t n_lanes;
   uint16_t max_len;
-  int32_t lower;     // 1: the slot's segments have a lower separator
+  int32_t kind;      // kSlotLeaf, kSlotLower: segments without / with a lower separator; kSlotCell: whole cells
 };
+constexpr int32_t kSlotLeaf = 0, kSlotLower = 1, kSlotCell = 2;
+// On the GB300, 1,000 network cells of 9 nodes x 400 steps: 7.19 ms cut into segments, 6.77 ms whole; 20,000 cells of
+// 8 to 100 nodes x 401 steps: 8.79 ms with all of them cut, 9.14 / 9.64 ms with those of up to 10 / 16 nodes whole.
+constexpr int kCellLaneNodes = 10;
 // A separator's inbox holds an entry per segment below it, padded to pairs.
 struct alignas(16) SepRec {
   int32_t in0;     // first pair of inbox entries
@@ -92,7 +100,13 @@ struct alignas(8) GroupRec {
   int32_t lv0, n_lv;
 };
 constexpr uint32_t kLinkNone = 0xFFFF;
-constexpr uint32_t kLinkSelf = 0xFFFE;  // lower half of a separator node's own link
+// Upper halves of the other links: a separator node's own; a whole cell's node, whose
+// lower half is its parent's row of the slot (kLinkNoParent at the root), plus
+// kLinkOnlyChild when the parent has no other child (it is the next row then).
+constexpr uint32_t kLinkSelf = 0xFFFE;
+constexpr uint32_t kLinkCell = 0xFFFD;
+constexpr uint32_t kLinkNoParent = 0xFF;
+constexpr uint32_t kLinkOnlyChild = 0x100;
 
 // Per-tile descriptor (global memory, read-only).
 struct TileDesc {
@@ -115,13 +129,14 @@ struct TileDesc {
   int64_t state_offset;     // elements into the plan's global mechanism-state array ([slot][n_nodes])
   int32_t off_ab;           // (alpha, beta) pairs
   int32_t off_pidx, off_spec, off_specs;
-  int32_t off_segs, off_slots, off_seps, off_levels, off_groups, off_link;
+  int32_t off_segs, off_slots, off_seps, off_levels, off_groups, off_link, off_rows, off_diag0;
   int32_t off_crec, off_params, off_mech;
   int32_t scratch_bytes;    // solver scratch (shared memory after the blob)
   int32_t off_dr;           // rows, inside the scratch area
   int32_t off_q, off_inbox, off_srow, off_own, off_xsep;  // inside the scratch area
   int32_t n_slots;          // warp slots of the segment elimination
   int32_t n_groups;
+  int32_t cell0;            // first node of the cells solved whole
   int32_t sep0;             // first separator node
   int32_t n_seps;
   int32_t n_inbox;          // inbox entries

@@ -142,6 +142,8 @@ struct TileView {
   const SepRec* seps;
   const int32_t* levels;       // separator levels: [level] first separator, one past the last level at the end
   const GroupRec* groups;
+  const int32_t* rows;         // row starts of the slots of whole cells
+  const Real* diag0;           // their nodes' axial diagonal
   const uint32_t* link;        // per node: upper separator | lower separator << 16 (kLinkNone, kLinkSelf)
   const uint16_t *pidx, *spec, *crec;  // crec: lane tiles only
   const SpecRec* specs;
@@ -155,7 +157,7 @@ struct TileView {
   const uint16_t* ncell;    // per node: tile-local cell (spike-source tiles only)
   const int32_t* srccell;   // per tile cell: global id of a spike source, -1 otherwise
   int32_t* stamp;           // per tile cell: last step with a crossing
-  int N, n_real, n_cells, n_slots, n_groups, sep0, n_seps, n_inbox;
+  int N, n_real, n_cells, n_slots, n_groups, cell0, sep0, n_seps, n_inbox;
   int pstride;  // reals per parameter record
   bool has_src;
 
@@ -171,6 +173,8 @@ struct TileView {
     levels = reinterpret_cast<const int32_t*>(base + td.off_levels);
     groups = reinterpret_cast<const GroupRec*>(base + td.off_groups);
     link = reinterpret_cast<const uint32_t*>(base + td.off_link);
+    rows = reinterpret_cast<const int32_t*>(base + td.off_rows);
+    diag0 = reinterpret_cast<const Real*>(base + td.off_diag0);
     crec = reinterpret_cast<const uint16_t*>(base + td.off_crec);
     pidx = reinterpret_cast<const uint16_t*>(base + td.off_pidx);
     spec = reinterpret_cast<const uint16_t*>(base + td.off_spec);
@@ -192,6 +196,7 @@ struct TileView {
     n_real = td.n_real_nodes;
     n_slots = td.n_slots;
     n_groups = td.n_groups;
+    cell0 = td.cell0;
     sep0 = td.sep0;
     n_seps = td.n_seps;
     n_inbox = td.n_inbox;
@@ -203,6 +208,10 @@ struct TileView {
 // the denormal range); FP64: IEEE round-to-nearest.
 __device__ __forceinline__ float pivot_rcp(float d) { return rcp_approx(d); }
 __device__ __forceinline__ double pivot_rcp(double d) { return __drcp_rn(d); }
+
+// a * b rounded (never part of a fused multiply-add).
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 // float-float accumulation: (hi, lo) += d
 template <typename Real>
@@ -941,13 +950,22 @@ __device__ __forceinline__ void steady_states(const Real* P, uint32_t m, Real* s
 
 // Row i of the next linear system without its axial part: excess = diagonal minus
 // the row's axial coefficients = 1 + dt G / cm, rhs = dt I / cm on membrane rows;
-// 0, 0 on boundary rows.
+// 0, 0 on boundary rows.  Cells solved whole take the diagonal, 1 + dt (D + G / cm).
 template <typename Real>
 __device__ __forceinline__ void write_row(const TileView<Real>& tv, int i, uint16_t pr, Real dt, Real G, Real I) {
-  if (pr == kBoundary) {
+  const Real* P = tv.params + size_t(pr) * tv.pstride;
+  if (i >= tv.cell0 && i < tv.sep0) {
+    const Real d0 = tv.diag0[i - tv.cell0];
+    if (pr == kBoundary) {
+      tv.dr[i] = make_pair(dt * d0, Real(0));
+    } else {
+      const Real invcm = P[BC_P_INVCM];
+      tv.dr[i] = make_pair(Real(1) + dt * (d0 + invcm * G), dt * invcm * I);
+    }
+  } else if (pr == kBoundary) {
     tv.dr[i] = make_pair(Real(0), Real(0));
   } else {
-    const Real invcm = tv.params[size_t(pr) * tv.pstride + BC_P_INVCM];
+    const Real invcm = P[BC_P_INVCM];
     tv.dr[i] = make_pair(Real(1) + dt * (invcm * G), dt * invcm * I);
   }
 }
@@ -1148,14 +1166,66 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
   }
 }
 
+// One slot of whole cells: lane l eliminates and back-substitutes its cell, in the
+// diagonal form.  A parent with one child is the next row and takes its child's terms
+// from registers; other parents collect them in their rows, child by child.  For cells
+// this small the separators are as many as the segments, and their sweep, inboxes and
+// records cost more than the walk.
+template <typename Real, bool kPre>
+__device__ __forceinline__ void solve_cells(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
+  const int32_t* rows = tv.rows + sr.seg0;
+  bool carry = false;
+  Pair<Real> pc = make_pair(Real(0), Real(0));
+  Real pw = Real(0), pR = Real(0), pd = Real(0);
+  for (int k = 0; k < sr.max_len; ++k) {
+    const int i = rows[k] + lane;
+    if (i >= rows[k + 1]) break;  // the lanes with more nodes come first
+    const uint32_t lk = tv.link[i];
+    const uint32_t par = lk & 0xFF;
+    const Pair<Real> q = tv.dr[i], c = coef<Real, kPre>(tv, i, dt), v = tv.v[i];
+    const int ip = par == kLinkNoParent ? i : rows[par] + lane;
+    Real D = q.x, R = q.y;
+    if (carry) {
+      D = q.x - pc.x * pw;
+      R = q.y + pw * pR + pc.y * pd;
+    }
+    const Real inv = pivot_rcp(D);
+    const Real delta = vdelta<Real>(v, tv.v[ip]);
+    R -= c.x * delta;
+    tv.dr[i] = make_pair(inv, R);
+    const Real w = c.y * inv;
+    carry = (lk & kLinkOnlyChild) != 0;
+    if (!carry && par != kLinkNoParent) {
+      Pair<Real> pp = tv.dr[ip];
+      pp.x -= mul_rn(c.x, w);
+      pp.y += w * R + c.y * delta;
+      tv.dr[ip] = pp;
+    }
+    pc = c;
+    pw = w;
+    pR = R;
+    pd = delta;
+  }
+  for (int k = sr.max_len - 1; k >= 0; --k) {
+    const int i = rows[k] + lane;
+    if (i >= rows[k + 1]) continue;
+    const uint32_t par = tv.link[i] & 0xFF;
+    const Pair<Real> q = tv.dr[i];
+    const Real xp = par == kLinkNoParent ? Real(0) : tv.dr[rows[par] + lane].y;
+    tv.dr[i].y = (q.y + coef<Real, kPre>(tv, i, dt).x * xp) * q.x;
+  }
+}
+
 template <typename Real, bool kPre>
 __device__ __forceinline__ void eliminate_segments(const TileView<Real>& tv, int warp, int n_warps, int lane, Real dt) {
   for (int s = warp; s < tv.n_slots; s += n_warps) {
     const SlotRec sr = tv.slots[s];
-    if (sr.lower)
+    if (sr.kind == kSlotLower)
       eliminate_slot<Real, kPre, true>(tv, sr, lane, dt);
-    else
+    else if (sr.kind == kSlotLeaf)
       eliminate_slot<Real, kPre, false>(tv, sr, lane, dt);
+    else
+      solve_cells<Real, kPre>(tv, sr, lane, dt);
   }
 }
 
@@ -1243,9 +1313,10 @@ __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int w
 template <typename Real>
 __device__ __forceinline__ Real node_increment(const TileView<Real>& tv, int i) {
   const uint32_t lk = tv.link[i], s = lk >> 16;
+  const Pair<Real> d = tv.dr[i];
+  if (s == kLinkCell) return d.y;
   const Real xt = tv.xsep[lk & 0xFFFF];
   if (s == kLinkSelf) return xt;
-  const Pair<Real> d = tv.dr[i];
   const Real x = d.x + d.y * xt;
   return s == kLinkNone ? x : x + tv.q[i] * tv.xsep[s];
 }

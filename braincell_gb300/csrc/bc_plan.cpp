@@ -290,6 +290,8 @@ struct CellSched {
   // lowered root .. tree root of the solve; the edges along it are turned around
   std::vector<int32_t> path;
   int32_t n_levels = 0;
+  // a cell solved whole (no segments or separators): its nodes in the order of elimination
+  std::vector<int32_t> order;
 };
 
 // fn(i) for i in [0, n) on up to BC_PLAN_THREADS host threads (default: the
@@ -325,6 +327,39 @@ static void parallel_for(int64_t n, F&& fn) {
   for (auto& th : pool) th.join();
 }
 
+// Elimination order of a cell solved whole: runs bottom -> top, the runs below a
+// branch point before it, in the order of their bottom nodes.
+static void order_whole(const LoweredCell& lc, CellSched& cs) {
+  const int32_t n = lc.n_node;
+  std::vector<std::vector<int32_t>> kids(n);
+  int32_t root = 0;
+  for (int32_t i = 0; i < n; ++i) {
+    if (lc.parent[i] < 0)
+      root = i;
+    else
+      kids[lc.parent[i]].push_back(i);
+  }
+  auto bottom = [&](int32_t v) {
+    while (kids[v].size() == 1) v = kids[v][0];
+    return v;
+  };
+  std::vector<std::pair<int32_t, bool>> todo{{root, false}};  // (top of a run, its branches done)
+  while (!todo.empty()) {
+    const auto [top, done] = todo.back();
+    todo.pop_back();
+    const int32_t b = bottom(top);
+    if (!done) {
+      todo.push_back({top, true});
+      std::vector<int32_t> below = kids[b];
+      std::sort(below.begin(), below.end(), [&](int32_t x, int32_t y) { return bottom(x) > bottom(y); });
+      for (const int32_t k : below) todo.push_back({k, false});
+    } else {
+      for (int32_t v = b; v != top; v = lc.parent[v]) cs.order.push_back(v);
+      cs.order.push_back(top);
+    }
+  }
+}
+
 // Segments and separators of one cell.  Runs of more than lane_nodes nodes are cut:
 // a lane's walk costs about 60 cycles a node and a further separator level about
 // 190, so a run of L nodes is cut into about sqrt(L / 3.2) pieces (measured on the
@@ -332,6 +367,10 @@ static void parallel_for(int64_t n, F&& fn) {
 // its results do not depend on its tile mates or on the launch shape.
 static void decompose(const LoweredCell& lc, int lane_nodes, CellSched& cs) {
   const int32_t n = lc.n_node;
+  if (n <= kCellLaneNodes) {
+    order_whole(lc, cs);
+    return;
+  }
   std::vector<std::array<int32_t, 2>> kid(n, {-1, -1});
   std::vector<int32_t> nchild(n, 0), parent(lc.parent);
   int32_t root = 0;
@@ -484,7 +523,8 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   std::vector<GroupRec> groups;
   std::vector<int32_t> levels;
   std::vector<uint32_t> link;
-  int32_t next_node = 0, sep0 = 0, n_inbox = 0;
+  std::vector<int32_t> rows;  // row starts of the slots of whole cells
+  int32_t next_node = 0, cell0 = 0, sep0 = 0, n_inbox = 0;
   int n_levels = 0;
   int64_t crit = 0, n_lower = 0;  // nodes of segments with a lower separator (they come first)
   if (!lane) {
@@ -496,13 +536,18 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     };
     std::vector<Cost> by_cost;
     size_t n_sep = 0;
+    std::vector<size_t> whole;  // cells of one lane each
     for (size_t li = 0; li < cell_list.size(); ++li) {
+      if (!sched_of(li).order.empty()) {
+        whole.push_back(li);
+        continue;
+      }
       by_cost.push_back({int64_t(sched_of(li).n_levels) + int64_t(sched_of(li).seps.size()) / 32, li});
       n_sep += sched_of(li).seps.size();
     }
-    if (n_sep >= kLinkSelf) return fail(BC_ERR_CAPACITY, "too many branch points in one tile");
+    if (n_sep >= kLinkCell) return fail(BC_ERR_CAPACITY, "too many branch points in one tile");
     std::stable_sort(by_cost.begin(), by_cost.end(), [](const Cost& a, const Cost& b) { return a.cost > b.cost; });
-    const size_t n_groups = std::min(cell_list.size(), size_t(W));
+    const size_t n_groups = std::min(by_cost.size(), size_t(W));
     std::vector<std::vector<size_t>> members(n_groups);
     std::vector<int64_t> group_seps(n_groups, 0);
     for (size_t k = 0; k < by_cost.size(); ++k) {
@@ -560,14 +605,15 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
         for (size_t k = 0; k < sched_of(li).segs.size(); ++k)
           if ((sched_of(li).segs[k].s >= 0) == (lower == 1)) v.push_back({li, int32_t(k)});
       // the roots' segments to themselves (k = -1)
-      for (size_t li = 0; lower == 1 && li < cell_list.size(); ++li) v.push_back({li, -1});
+      for (const Cost& c : by_cost)
+        if (lower == 1) v.push_back({c.li, -1});
       auto len = [&](const std::pair<size_t, int32_t>& x) {
         return x.second < 0 ? size_t(0) : sched_of(x.first).segs[x.second].nodes.size();
       };
       std::stable_sort(v.begin(), v.end(), [&](const auto& x, const auto& y) { return len(x) > len(y); });
       for (size_t q = 0; q < v.size(); q += 32) {
         const size_t n_lanes = std::min<size_t>(32, v.size() - q);
-        SlotRec sr{next_node, int32_t(segs.size()), int16_t(n_lanes), uint16_t(len(v[q])), lower};
+        SlotRec sr{next_node, int32_t(segs.size()), int16_t(n_lanes), uint16_t(len(v[q])), lower ? kSlotLower : kSlotLeaf};
         for (size_t l = 0; l < n_lanes; ++l) {
           const auto& st = sep_tile[v[q + l].first];
           if (v[q + l].second < 0) {
@@ -593,9 +639,34 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
       }
       if (lower == 1) n_lower = next_node;
     }
+    // -------- whole cells, largest first
+    cell0 = next_node;
+    std::stable_sort(whole.begin(), whole.end(),
+                     [&](size_t x, size_t y) { return sched_of(x).order.size() > sched_of(y).order.size(); });
+    for (size_t q = 0; q < whole.size(); q += 32) {
+      const size_t n_lanes = std::min<size_t>(32, whole.size() - q);
+      const size_t max_len = sched_of(whole[q]).order.size();
+      slots.push_back(SlotRec{next_node, int32_t(rows.size()), int16_t(n_lanes), uint16_t(max_len), kSlotCell});
+      for (size_t k = 0; k < max_len; ++k) {
+        rows.push_back(next_node);
+        for (size_t l = 0; l < n_lanes && sched_of(whole[q + l]).order.size() > k; ++l) {
+          const LoweredCell& lc = (*cx.cells)[cell_list[whole[q + l]]];
+          const std::vector<int32_t>& ord = sched_of(whole[q + l]).order;
+          const int32_t p = lc.parent[ord[k]];
+          uint32_t lk = kLinkNoParent;
+          if (p >= 0) {
+            lk = uint32_t(std::find(ord.begin(), ord.end(), p) - ord.begin());
+            if (std::count(lc.parent.begin(), lc.parent.end(), p) == 1) lk |= kLinkOnlyChild;
+          }
+          link.push_back(lk | (kLinkCell << 16));
+          node_tile[whole[q + l]][ord[k]] = next_node++;
+        }
+      }
+      rows.push_back(next_node);
+    }
     // warp w takes slots w, w + W, ...: the dearest first
     std::stable_sort(slots.begin(), slots.end(), [](const SlotRec& a, const SlotRec& b) {
-      return int(a.max_len) + 2 * a.lower > int(b.max_len) + 2 * b.lower;
+      return int(a.max_len) + 2 * a.kind > int(b.max_len) + 2 * b.kind;
     });
     sep0 = next_node;
     for (size_t j = 0; j < sep_src.size(); ++j) {
@@ -624,6 +695,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     n_real = int64_t(lane_kmax) * T;
     out.crit = lane_kmax;
   }
+  if (lane) cell0 = sep0 = int32_t(n_real);  // rows in the excess form
   std::vector<uint16_t> crec;
   if (lane) {  // lane tiles: the parent's node index v within the cell (0xFFFF at the root)
     crec.assign(size_t(n_real), 0);
@@ -694,6 +766,10 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   off = align16(off + levels.size() * 4);
   d.off_groups = int32_t(off);
   off = align16(off + groups.size() * sizeof(GroupRec));
+  d.off_rows = int32_t(off);
+  off = align16(off + rows.size() * 4);
+  d.off_diag0 = int32_t(off);
+  off = align16(off + size_t(sep0 - cell0) * rs);
   d.off_crec = int32_t(off);
   off = align16(off + crec.size() * 2);
   d.off_params = int32_t(off);
@@ -755,6 +831,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   d.n_seps = int32_t(seps.size());
   d.n_inbox = n_inbox;
   d.n_groups = int32_t(groups.size());
+  d.cell0 = cell0;
   d.sep0 = sep0;
   d.n_params = int32_t(n_params);
   // -------- fill
@@ -784,7 +861,9 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
       std::memcpy(b.data() + d.off_pidx + size_t(j) * 2, &pi, 2);
       out.vinit[j] = lc.node_vrest[v];
     }
-    if (!lane) {
+    if (!lane && !sched_of(li).order.empty()) {
+      for (int32_t v = 0; v < lc.n_node; ++v) putr(d.off_diag0, size_t(node_tile[li][v] - cell0), lc.diag[v]);
+    } else if (!lane) {
       // the solve's root is path.back(): along the path the old parent is the child
       const std::vector<int32_t>& path = sched_of(li).path;
       for (size_t k = 0; k < path.size(); ++k) {
@@ -931,6 +1010,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   put_all(d.off_seps, seps.data(), seps.size() * sizeof(SepRec));
   put_all(d.off_levels, levels.data(), levels.size() * 4);
   put_all(d.off_groups, groups.data(), groups.size() * sizeof(GroupRec));
+  put_all(d.off_rows, rows.data(), rows.size() * 4);
   put_all(d.off_crec, crec.data(), crec.size() * 2);
   out.desc = d;
   return BC_OK;
