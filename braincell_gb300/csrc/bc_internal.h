@@ -77,8 +77,8 @@ struct alignas(16) SegRec {
   int32_t pad2;
 };
 struct alignas(16) SlotRec {
-  int32_t n_begin;   // first node
-  int32_t seg0;      // first segment (lane 0); whole cells: first of the slot's max_len + 1 row starts
+  int32_t rows0;     // row starts: node k of lane l is rows[rows0 + k] + l (a multiple of 4, max_len + 1 entries, padded)
+  int32_t seg0;      // first segment (lane 0)
   int16_t n_lanes;
   uint16_t max_len;
   int32_t kind;      // kSlotLeaf, kSlotLower: segments without / with a lower separator; kSlotCell: whole cells
@@ -87,7 +87,7 @@ constexpr int32_t kSlotLeaf = 0, kSlotLower = 1, kSlotCell = 2;
 // On the GB300, 1,000 network cells of 9 nodes x 400 steps: 7.19 ms cut into segments, 6.77 ms whole; 20,000 cells of
 // 8 to 100 nodes x 401 steps: 8.79 ms with all of them cut, 9.14 / 9.64 ms with those of up to 10 / 16 nodes whole.
 constexpr int kCellLaneNodes = 10;
-// A separator's inbox holds an entry per segment below it, padded to pairs.
+// A separator's inbox holds an entry per segment below it, padded to pairs, two or more.
 struct alignas(16) SepRec {
   int32_t in0;     // first pair of inbox entries
   int32_t inbox;   // this separator's entry in its upper separator's inbox (one nobody reads at a root)
@@ -95,10 +95,15 @@ struct alignas(16) SepRec {
   uint16_t t;      // upper separator (itself at a root)
   int32_t pad;
 };
-// Separator levels [lv0, lv0 + n_lv) swept by one warp.
+// The separators one warp sweeps, in chunks of at most 32 of one level: chunk c starts
+// at separator levels[lv0 + c], c < n_chunks (kChunkMore set: one of its inboxes has
+// more than two pairs), and ends where the next starts (levels[lv0 + n_chunks]: the end).
 struct alignas(8) GroupRec {
-  int32_t lv0, n_lv;
+  int32_t lv0, n_chunks;
 };
+constexpr uint32_t kChunkMore = 0x80000000u;
+// Entries past the last separator that the padding of a tile's nodes (to a multiple of 4) reads.
+constexpr int kSepPad = 4;
 constexpr uint32_t kLinkNone = 0xFFFF;
 // Upper halves of the other links: a separator node's own; a whole cell's node, whose
 // lower half is its parent's row of the slot (kLinkNoParent at the root), plus
@@ -129,13 +134,16 @@ struct TileDesc {
   int64_t state_offset;     // elements into the plan's global mechanism-state array ([slot][n_nodes])
   int32_t off_ab;           // (alpha, beta) pairs
   int32_t off_pidx, off_spec, off_specs;
-  int32_t off_segs, off_slots, off_seps, off_levels, off_groups, off_link, off_rows, off_diag0;
+  int32_t off_segs, off_slots, off_seps, off_levels, off_groups, off_link, off_rows, off_diag0, off_heavy;
   int32_t off_crec, off_params, off_mech;
   int32_t scratch_bytes;    // solver scratch (shared memory after the blob)
   int32_t off_dr;           // rows, inside the scratch area
   int32_t off_q, off_inbox, off_srow, off_own, off_xsep;  // inside the scratch area
+  int32_t off_wparams;      // global-memory tiles: the launch's parameter records (scratch)
   int32_t n_slots;          // warp slots of the segment elimination
   int32_t n_groups;
+  int32_t n_heavy;          // nodes with heavy mechanisms
+  int32_t n_lower;          // nodes of segments with a lower separator (they come first)
   int32_t cell0;            // first node of the cells solved whole
   int32_t sep0;             // first separator node
   int32_t n_seps;

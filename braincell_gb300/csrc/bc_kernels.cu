@@ -140,10 +140,11 @@ struct TileView {
   const SlotRec* slots;        // warp slots of the segment elimination
   const SegRec* segs;
   const SepRec* seps;
-  const int32_t* levels;       // separator levels: [level] first separator, one past the last level at the end
+  const int32_t* levels;       // chunks of the separator sweeps (see GroupRec)
   const GroupRec* groups;
-  const int32_t* rows;         // row starts of the slots of whole cells
-  const Real* diag0;           // their nodes' axial diagonal
+  const int32_t* rows;         // row starts of the slots
+  const Real* diag0;           // axial diagonal of the whole cells' nodes
+  const int32_t* heavy;        // nodes with heavy mechanisms
   const uint32_t* link;        // per node: upper separator | lower separator << 16 (kLinkNone, kLinkSelf)
   const uint16_t *pidx, *spec, *crec;  // crec: lane tiles only
   const SpecRec* specs;
@@ -157,7 +158,7 @@ struct TileView {
   const uint16_t* ncell;    // per node: tile-local cell (spike-source tiles only)
   const int32_t* srccell;   // per tile cell: global id of a spike source, -1 otherwise
   int32_t* stamp;           // per tile cell: last step with a crossing
-  int N, n_real, n_cells, n_slots, n_groups, cell0, sep0, n_seps, n_inbox;
+  int N, n_real, n_cells, n_slots, n_groups, n_lower, cell0, sep0, n_seps, n_inbox, n_heavy;
   int pstride;  // reals per parameter record
   bool has_src;
 
@@ -175,6 +176,8 @@ struct TileView {
     link = reinterpret_cast<const uint32_t*>(base + td.off_link);
     rows = reinterpret_cast<const int32_t*>(base + td.off_rows);
     diag0 = reinterpret_cast<const Real*>(base + td.off_diag0);
+    heavy = reinterpret_cast<const int32_t*>(base + td.off_heavy);
+    n_heavy = td.n_heavy;
     crec = reinterpret_cast<const uint16_t*>(base + td.off_crec);
     pidx = reinterpret_cast<const uint16_t*>(base + td.off_pidx);
     spec = reinterpret_cast<const uint16_t*>(base + td.off_spec);
@@ -196,6 +199,7 @@ struct TileView {
     n_real = td.n_real_nodes;
     n_slots = td.n_slots;
     n_groups = td.n_groups;
+    n_lower = td.n_lower;
     cell0 = td.cell0;
     sep0 = td.sep0;
     n_seps = td.n_seps;
@@ -209,9 +213,15 @@ struct TileView {
 __device__ __forceinline__ float pivot_rcp(float d) { return rcp_approx(d); }
 __device__ __forceinline__ double pivot_rcp(double d) { return __drcp_rn(d); }
 
-// a * b rounded (never part of a fused multiply-add).
+// a * b and a + b rounded (never parts of a fused multiply-add), and a * b + c fused:
+// where the same sum stands in several copies of the code (the two nodes of a lane, the
+// forms of a warp), so that a node's result does not depend on which copy it met.
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // float-float accumulation: (hi, lo) += d
 template <typename Real>
@@ -225,33 +235,54 @@ __device__ __forceinline__ void ff_add(Real& hi, Real& lo, Real d) {
 }
 
 // ------------------------------------------------------------------ mechanisms
-// The mechanism states of one node, held in registers (absent ones are 0).
-template <typename Real>
+// The mechanism states of W consecutive nodes, in registers (absent ones are undefined).
+template <typename Real, int W>
 struct NodeStates {
-  Real nap, naq, kdrp, calp, calq, catp, catq, hcnp, ahpp, cahi, calo;
+  Real nap[W], naq[W], kdrp[W], calp[W], calq[W], catp[W], catq[W], hcnp[W], ahpp[W], cahi[W], calo[W];
 };
 
-template <typename Real>
-__device__ __forceinline__ void load_states(const Real* st, int N, uint32_t m, NodeStates<Real>& s) {
-  s.nap = s.naq = s.kdrp = s.calp = s.calq = s.catp = s.catq = s.hcnp = s.ahpp = s.cahi = s.calo = Real(0);
-  if (m & BC_M_NA) {
-    s.nap = st[kSlotNaP * N];
-    s.naq = st[kSlotNaQ * N];
+// Loaded by group: a state that is absent but in a present group is read and not used.
+constexpr uint32_t kSpikeGroup = BC_M_NA | BC_M_KDR;
+constexpr uint32_t kShellGroup = BC_M_CAT | BC_M_AHP | BC_M_CADET;
+
+// W consecutive values of a per-node array (W = 2: one vector access; the arrays keep
+// an even node on an 8-byte boundary).
+template <int W, typename Real>
+__device__ __forceinline__ void load_w(const Real* p, Real (&x)[W]) {
+  if constexpr (W == 2) {
+    const Pair<Real> t = *reinterpret_cast<const Pair<Real>*>(p);
+    x[0] = t.x;
+    x[1] = t.y;
+  } else {
+    x[0] = p[0];
   }
-  if (m & BC_M_KDR) s.kdrp = st[kSlotKdrP * N];
+}
+template <int W, typename Real>
+__device__ __forceinline__ void store_w(Real* p, const Real (&x)[W]) {
+  if constexpr (W == 2)
+    *reinterpret_cast<Pair<Real>*>(p) = make_pair<Real>(x[0], x[1]);
+  else
+    p[0] = x[0];
+}
+
+template <int W, typename Real>
+__device__ __forceinline__ void load_states(const Real* st, int N, uint32_t m, NodeStates<Real, W>& s) {
   if (m & BC_M_CAL) {
-    s.calp = st[kSlotCalP * N];
-    s.calq = st[kSlotCalQ * N];
+    load_w<W>(st + kSlotCalP * N, s.calp);
+    load_w<W>(st + kSlotCalQ * N, s.calq);
   }
-  if (m & BC_M_CAT) {
-    s.catp = st[kSlotCatP * N];
-    s.catq = st[kSlotCatQ * N];
+  if (m & BC_M_HCN) load_w<W>(st + kSlotHcnP * N, s.hcnp);
+  if (m & kSpikeGroup) {
+    load_w<W>(st + kSlotNaP * N, s.nap);
+    load_w<W>(st + kSlotNaQ * N, s.naq);
+    load_w<W>(st + kSlotKdrP * N, s.kdrp);
   }
-  if (m & BC_M_HCN) s.hcnp = st[kSlotHcnP * N];
-  if (m & BC_M_AHP) s.ahpp = st[kSlotAhpP * N];
-  if (m & BC_M_CADET) {
-    s.cahi = st[kSlotCaHi * N];
-    s.calo = st[kSlotCaLo * N];
+  if (m & kShellGroup) {
+    load_w<W>(st + kSlotCatP * N, s.catp);
+    load_w<W>(st + kSlotCatQ * N, s.catq);
+    load_w<W>(st + kSlotAhpP * N, s.ahpp);
+    load_w<W>(st + kSlotCaHi * N, s.cahi);
+    load_w<W>(st + kSlotCaLo * N, s.calo);
   }
 }
 
@@ -689,137 +720,242 @@ __device__ __noinline__ void extra_channels(Real* st, int N, const Real* P, uint
   }
 }
 
-// One node's mechanisms.  `st` points at the node's slot-0 state (stride N).
-// With advance = true the states move from (v_old) to (v_new) first: calcium
-// from the step-start current (old gates, old V, old Ci), then every gate at
-// v_new (and the new Ci).  Returns the membrane conductance G (mS/cm^2) and
-// ionic current I (uA/cm^2) at v_new with the resulting states.
-template <typename Real, bool kExtra = true>
-__device__ __forceinline__ void node_mechanisms_loaded(const NodeStates<Real>& s0, Real* st, int N, const Real* P,
-                                                       uint32_t m, Real v_old, Real v_new, Real dt, bool advance,
-                                                       Real& G, Real& I) {
-  Real nap = s0.nap, naq = s0.naq, kdrp = s0.kdrp, calp = s0.calp, calq = s0.calq, catp = s0.catp, catq = s0.catq,
-       hcnp = s0.hcnp, ahpp = s0.ahpp, cahi = s0.cahi, calo = s0.calo;
+// Parameter records of a launch: the main mix's entries that only ever appear with dt
+// are replaced by what the step needs (kDer), once per launch, in the records' shared-
+// memory copy or in a copy in the tile's scratch:
+//   PHI entries -> -dt phi;  CA_TAU -> c = 1 - exp(-dt / tau);  CA_D -> the shell's gain
+//   c tau 10 / (2 F d), so that the calcium step is Ci += max(gain ICa, 0) + c (C_rest - Ci).
+template <typename Real>
+__device__ __forceinline__ Real launch_param(const Real* P, uint32_t m, int k, Real dt) {
+  switch (k) {
+    case BC_P_NA_PHI:
+    case BC_P_KDR_PHI:
+    case BC_P_CAL_PHIP:
+    case BC_P_CAL_PHIQ:
+    case BC_P_CAT_PHIP:
+    case BC_P_CAT_PHIQ:
+    case BC_P_HCN_PHI:
+    case BC_P_AHP_PHI:
+      return -dt * P[k];
+    case BC_P_CA_TAU:
+      return (m & BC_M_CADET) ? -dexpm1(-dt / P[k]) : P[k];
+    case BC_P_CA_D:
+      return (m & BC_M_CADET) ? -dexpm1(-dt / P[BC_P_CA_TAU]) * P[BC_P_CA_TAU] * Real(kCaDrive) / P[k] : P[k];
+    default:
+      return P[k];
+  }
+}
+template <typename Real, bool kDer>
+__device__ __forceinline__ Real step_param(const Real* P, uint32_t m, int k, Real dt) {
+  return kDer ? P[k] : launch_param(P, m, k, dt);
+}
 
-  if (advance) {
-    if (m & BC_M_CADET) {
-      const Real ci = cahi + calo;
-      const Real eca = Real(kNernstCa) * P[BC_P_CA_TEMP] * dlog(P[BC_P_CA_CO] / ci);
-      Real ica = Real(0);
-      if (m & BC_M_CAL) ica += P[BC_P_CAL_G] * calp * calp * calq * (eca - v_old);
-      if (m & BC_M_CAT) ica += P[BC_P_CAT_G] * catp * catp * catq * (eca - v_old);
-      if (kExtra && (m & kCerebellarCaChannels)) ica += cerebellar_ca_current(st, N, P, m, v_old, eca, (Real*)nullptr);
-      if (kExtra && (m & BC_M_EXT)) ica += ext_ca_current(st, N, P, v_old, ci, eca);
-      Real drive = ica * Real(kCaDrive) / P[BC_P_CA_D];
-      drive = drive > Real(0) ? drive : Real(0);
-      const Real tau = P[BC_P_CA_TAU];
-      const Real f = drive + (P[BC_P_CA_CREST] - ci) / tau;
-      ff_add(cahi, calo, dt * exprel(-dt / tau) * f);
-      st[kSlotCaHi * N] = cahi;
-      st[kSlotCaLo * N] = calo;
+// The mechanisms of W consecutive nodes.  `st` points at the first node's slot-0 state
+// (stride N).  With kAdv the states move from (v_old) to (v) first: calcium from the
+// step-start current (old gates, old V, old Ci), then every gate at v (and the new Ci).
+// Returns the membrane conductance G (mS/cm^2) and ionic current I (uA/cm^2) at v with
+// the resulting states.  kDer: P are a launch's records (see launch_param).
+//
+// kHeavy: nodes may have heavy mechanisms (kHeavyMech) too.
+// mu is the union of m over the warp (or the node's m): a mechanism's block is entered
+// by the whole warp, a uniform branch.  Nodes without the mechanism keep its terms to
+// themselves; a pair's states are stored together (pair) when either node has the
+// mechanism (a state that a node does not have is never read), unless one of the two is
+// another lane's.
+template <typename Real, int W, bool kHeavy, bool kExtra, bool kAdv, bool kDer>
+__device__ __forceinline__ void node_mechanisms(const NodeStates<Real, W>& s0, Real* st, int N,
+                                                const Real* const (&P)[W], const uint32_t (&m)[W], uint32_t mu, bool pair,
+                                                const Real (&v_old)[W], const Real (&v)[W], Real dt, Real (&G)[W],
+                                                Real (&I)[W]) {
+  uint32_t m_any = m[0];
+  if constexpr (W == 2) m_any |= m[1];
+  auto keep = [&](int slot, uint32_t bit, const Real(&x)[W]) {
+    if (W == 1 || pair) {
+      if (m_any & bit) store_w<W>(st + slot * N, x);
+    } else {
+      for (int j = 0; j < W; ++j)
+        if (m[j] & bit) st[slot * N + j] = x[j];
     }
-    if (m & BC_M_NA) {
-      const NaRates<Real> r(v_new, P[BC_P_NA_VSH]);
-      const Real phi = P[BC_P_NA_PHI];
-      nap = gate_ab<Real, true>(nap, r.ap, r.bp, phi, dt);
-      naq = gate_ab<Real, true>(naq, r.aq, r.bq, phi, dt);
-      st[kSlotNaP * N] = nap;
-      st[kSlotNaQ * N] = naq;
+  };
+  auto k_of = [&](int j, int k) { return step_param<Real, kDer>(P[j], m[j], k, dt); };
+  // selects instead of branches: the two nodes' chains interleave
+  auto add = [&](int j, uint32_t bit, Real g, Real e) {
+    const bool on = (m[j] & bit) != 0;
+    const Real i = mul_rn(g, e - v[j]);
+    G[j] = add_rn(G[j], on ? g : Real(0));
+    I[j] = add_rn(I[j], on ? i : Real(0));
+  };
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    G[j] = I[j] = Real(0);
+    add(j, BC_M_IL, P[j][BC_P_IL_G], P[j][BC_P_IL_E]);
+    add(j, BC_M_KLEAK, P[j][BC_P_KLEAK_G], P[j][BC_P_EK]);
+  }
+  Real ci[W];
+#pragma unroll
+  for (int j = 0; j < W; ++j) ci[j] = Real(0);
+  if ((kHeavy && kExtra) || (mu & (BC_M_CAL | kShellGroup))) {
+    Real eca[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      ci[j] = P[j][BC_P_CA_CI0];
+      eca[j] = P[j][BC_P_ECA];
     }
-    if (m & BC_M_KDR) {
-      const KdrRates<Real> r(v_new, P[BC_P_KDR_VSH]);
-      kdrp = gate_ab<Real, true>(kdrp, r.a, r.b, P[BC_P_KDR_PHI], dt);
-      st[kSlotKdrP * N] = kdrp;
+    if (mu & BC_M_CADET) {
+      Real cahi[W], calo[W];
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        const bool on = (m[j] & BC_M_CADET) != 0;
+        cahi[j] = s0.cahi[j];
+        calo[j] = s0.calo[j];
+        const Real co = P[j][BC_P_CA_CO], nernst = Real(kNernstCa) * P[j][BC_P_CA_TEMP];
+        Real c = cahi[j] + calo[j], E = nernst * dlog(adiv(co, c));
+        if (kAdv) {
+          Real ica = Real(0);
+          if (mu & BC_M_CAL) {
+            const Real i = P[j][BC_P_CAL_G] * s0.calp[j] * s0.calp[j] * s0.calq[j] * (E - v_old[j]);
+            ica = add_rn(ica, (m[j] & BC_M_CAL) ? i : Real(0));
+          }
+          if (mu & BC_M_CAT) {
+            const Real i = P[j][BC_P_CAT_G] * s0.catp[j] * s0.catp[j] * s0.catq[j] * (E - v_old[j]);
+            ica = add_rn(ica, (m[j] & BC_M_CAT) ? i : Real(0));
+          }
+          if (kHeavy && kExtra && (m[j] & kCerebellarCaChannels))
+            ica += cerebellar_ca_current(st + j, N, P[j], m[j], v_old[j], E, (Real*)nullptr);
+          if (kHeavy && kExtra && (m[j] & BC_M_EXT)) ica += ext_ca_current(st + j, N, P[j], v_old[j], c, E);
+          const Real drive = ica * k_of(j, BC_P_CA_D);
+          ff_add(cahi[j], calo[j],
+                 (drive > Real(0) ? drive : Real(0)) + k_of(j, BC_P_CA_TAU) * (P[j][BC_P_CA_CREST] - c));
+          c = cahi[j] + calo[j];
+          E = nernst * dlog(adiv(co, c));
+        }
+        ci[j] = on ? c : ci[j];
+        eca[j] = on ? E : eca[j];
+      }
+      if (kAdv) keep(kSlotCaHi, BC_M_CADET, cahi);
+      if (kAdv) keep(kSlotCaLo, BC_M_CADET, calo);
     }
-    if (m & BC_M_CAL) {
-      const CaLRates<Real> r(v_new, P[BC_P_CAL_VSH]);
-      calp = gate_it(calp, r.pinf, r.ptau, P[BC_P_CAL_PHIP], dt);
-      calq = gate_it(calq, r.qinf, r.qtau, P[BC_P_CAL_PHIQ], dt);
-      st[kSlotCalP * N] = calp;
-      st[kSlotCalQ * N] = calq;
+    if (mu & BC_M_CAL) {
+      Real p[W], q[W];
+#pragma unroll
+      for (int j = 0; j < W; ++j) {
+        p[j] = s0.calp[j];
+        q[j] = s0.calq[j];
+        if (kAdv) {
+          const Real vs = v[j] - P[j][BC_P_CAL_VSH];
+          p[j] = cal_p_step(vs, k_of(j, BC_P_CAL_PHIP)).step(p[j]);
+          q[j] = cal_q_step(vs, k_of(j, BC_P_CAL_PHIQ)).step(q[j]);
+        }
+        add(j, BC_M_CAL, P[j][BC_P_CAL_G] * p[j] * p[j] * q[j], eca[j]);
+      }
+      if (kAdv) keep(kSlotCalP, BC_M_CAL, p);
+      if (kAdv) keep(kSlotCalQ, BC_M_CAL, q);
     }
-    if (m & BC_M_CAT) {
-      const CaTRates<Real> r(v_new, P[BC_P_CAT_VSH]);
-      catp = gate_it(catp, r.pinf, r.ptau, P[BC_P_CAT_PHIP], dt);
-      catq = gate_it(catq, r.qinf, r.qtau, P[BC_P_CAT_PHIQ], dt);
-      st[kSlotCatP * N] = catp;
-      st[kSlotCatQ * N] = catq;
-    }
-    if (m & BC_M_HCN) {
-      const HcnRates<Real> r(v_new);
-      hcnp = gate_it(hcnp, r.pinf, r.ptau, P[BC_P_HCN_PHI], dt);
-      st[kSlotHcnP * N] = hcnp;
-    }
-    if (m & BC_M_AHP) {
-      const Real ci = (m & BC_M_CADET) ? cahi + calo : P[BC_P_CA_CI0];
-      const Real n = P[BC_P_AHP_N];
-      const Real ci_n = n == Real(2) ? ci * ci : dpow(ci, n);
-      ahpp = gate_ab(ahpp, P[BC_P_AHP_ALPHA] * ci_n, P[BC_P_AHP_BETA], P[BC_P_AHP_PHI], dt);
-      st[kSlotAhpP * N] = ahpp;
+    if (mu & (BC_M_CAT | BC_M_AHP)) {
+      if (mu & BC_M_CAT) {
+        Real p[W], q[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          p[j] = s0.catp[j];
+          q[j] = s0.catq[j];
+          if (kAdv) {
+            const Real vs = v[j] - P[j][BC_P_CAT_VSH];
+            p[j] = cat_p_step(vs, k_of(j, BC_P_CAT_PHIP)).step(p[j]);
+            q[j] = cat_q_step(vs, k_of(j, BC_P_CAT_PHIQ)).step(q[j]);
+          }
+          add(j, BC_M_CAT, P[j][BC_P_CAT_G] * p[j] * p[j] * q[j], eca[j]);
+        }
+        if (kAdv) keep(kSlotCatP, BC_M_CAT, p);
+        if (kAdv) keep(kSlotCatQ, BC_M_CAT, q);
+      }
+      if (mu & BC_M_AHP) {
+        Real p[W];
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+          p[j] = s0.ahpp[j];
+          const bool on = (m[j] & BC_M_AHP) != 0;
+          if (kAdv) {
+            const Real n = P[j][BC_P_AHP_N];
+            const Real a = P[j][BC_P_AHP_ALPHA] * (n == Real(2) || !on ? ci[j] * ci[j] : dpow(ci[j], n));
+            const Real s = a + P[j][BC_P_AHP_BETA];
+            p[j] = p[j] - decay_em1(k_of(j, BC_P_AHP_PHI) * s) * (rdiv(a, s) - p[j]);
+          }
+          add(j, BC_M_AHP, P[j][BC_P_AHP_G] * p[j] * p[j], P[j][BC_P_EK]);
+        }
+        if (kAdv) keep(kSlotAhpP, BC_M_AHP, p);
+      }
     }
   }
-  // currents at v_new
-  const Real v = v_new;
-  G = Real(0);
-  I = Real(0);
-  if (m & BC_M_IL) {
-    const Real g = P[BC_P_IL_G];
-    G += g;
-    I += g * (P[BC_P_IL_E] - v);
-  }
-  if (m & BC_M_KLEAK) {
-    const Real g = P[BC_P_KLEAK_G];
-    G += g;
-    I += g * (P[BC_P_EK] - v);
-  }
-  if (m & BC_M_NA) {
-    const Real g = P[BC_P_NA_G] * nap * nap * nap * naq;
-    G += g;
-    I += g * (P[BC_P_ENA] - v);
-  }
-  if (m & BC_M_KDR) {
-    const Real p2 = kdrp * kdrp;
-    const Real g = P[BC_P_KDR_G] * p2 * p2;
-    G += g;
-    I += g * (P[BC_P_EK] - v);
-  }
-  if (m & (BC_M_CAL | BC_M_CAT)) {
-    Real eca = P[BC_P_ECA];
-    if (m & BC_M_CADET) eca = Real(kNernstCa) * P[BC_P_CA_TEMP] * dlog(P[BC_P_CA_CO] / (cahi + calo));
-    if (m & BC_M_CAL) {
-      const Real g = P[BC_P_CAL_G] * calp * calp * calq;
-      G += g;
-      I += g * (eca - v);
+  if (mu & BC_M_HCN) {
+    Real p[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      p[j] = s0.hcnp[j];
+      if (kAdv) p[j] = hcn_step(v[j], k_of(j, BC_P_HCN_PHI)).step(p[j]);
+      add(j, BC_M_HCN, P[j][BC_P_HCN_G] * p[j], P[j][BC_P_HCN_E]);
     }
-    if (m & BC_M_CAT) {
-      const Real g = P[BC_P_CAT_G] * catp * catp * catq;
-      G += g;
-      I += g * (eca - v);
+    if (kAdv) keep(kSlotHcnP, BC_M_HCN, p);
+  }
+  // the spike-generating gates: accurate forms, and few nodes, so per node
+  if (kHeavy && (mu & kSpikeGroup)) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      if (m[j] & BC_M_NA) {
+        Real p = s0.nap[j], q = s0.naq[j];
+        if (kAdv) {
+          const NaRates<Real> r(v[j], P[j][BC_P_NA_VSH]);
+          const Real k = k_of(j, BC_P_NA_PHI), sp = r.ap + r.bp, sq = r.aq + r.bq;
+          p = p - dexpm1(k * sp) * (adiv(r.ap, sp) - p);
+          q = q - dexpm1(k * sq) * (adiv(r.aq, sq) - q);
+          st[kSlotNaP * N + j] = p;
+          st[kSlotNaQ * N + j] = q;
+        }
+        add(j, BC_M_NA, P[j][BC_P_NA_G] * p * p * p * q, P[j][BC_P_ENA]);
+      }
+      if (m[j] & BC_M_KDR) {
+        Real p = s0.kdrp[j];
+        if (kAdv) {
+          const KdrRates<Real> r(v[j], P[j][BC_P_KDR_VSH]);
+          const Real s = r.a + r.b;
+          p = p - dexpm1(k_of(j, BC_P_KDR_PHI) * s) * (adiv(r.a, s) - p);
+          st[kSlotKdrP * N + j] = p;
+        }
+        const Real p2 = p * p;
+        add(j, BC_M_KDR, P[j][BC_P_KDR_G] * p2 * p2, P[j][BC_P_EK]);
+      }
     }
   }
-  if (m & BC_M_HCN) {
-    const Real g = P[BC_P_HCN_G] * hcnp;
-    G += g;
-    I += g * (P[BC_P_HCN_E] - v);
-  }
-  if (m & BC_M_AHP) {
-    const Real g = P[BC_P_AHP_G] * ahpp * ahpp;
-    G += g;
-    I += g * (P[BC_P_EK] - v);
-  }
-  if (kExtra && (m & kExtraChannels)) {
-    // the calcium the Markov Kca channels bind: the new Ci of a dynamic ion, else the fixed one
-    const Real ci = (m & BC_M_CADET) ? cahi + calo : P[BC_P_CA_CI0];
-    extra_channels(st, N, P, m, v_new, ci, dt, advance, G, I);
+  // the Markov Kca channels bind the new Ci of a dynamic ion, else the fixed one
+  if constexpr (kHeavy && kExtra) {
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (m[j] & kExtraChannels) extra_channels(st + j, N, P[j], m[j], v[j], ci[j], dt, kAdv, G[j], I[j]);
   }
 }
 
-template <typename Real, bool kExtra = true>
-__device__ __forceinline__ void node_mechanisms(Real* st, int N, const Real* P, uint32_t m, Real v_old, Real v_new,
-                                                Real dt, bool advance, Real& G, Real& I) {
-  NodeStates<Real> s;
+// Mechanisms whose nodes are updated in a list of their own, one to a lane: the spike-
+// generating gates with their accurate functions, and all out-of-line channels.
+constexpr uint32_t kHeavyMech = kSpikeGroup | kExtraChannels;
+
+// The same for one node by itself: its currents as they are, or one step on.
+template <typename Real, bool kExtra, bool kAdv>
+__device__ __forceinline__ void one_node(const NodeStates<Real, 1>& s, Real* st, int N, const Real* P, uint32_t m,
+                                         Real v_old, Real v, Real dt, Real& G, Real& I) {
+  const Real* const Pa[1] = {P};
+  const uint32_t ma[1] = {m};
+  const Real vo[1] = {v_old}, va[1] = {v};
+  Real g[1], i[1];
+  node_mechanisms<Real, 1, true, kExtra, kAdv, false>(s, st, N, Pa, ma, m, true, vo, va, dt, g, i);
+  G = g[0];
+  I = i[0];
+}
+
+template <typename Real, bool kExtra>
+__device__ __forceinline__ void node_currents(Real* st, int N, const Real* P, uint32_t m, Real v, Real dt, Real& G,
+                                              Real& I) {
+  NodeStates<Real, 1> s;
   load_states(st, N, m, s);
-  node_mechanisms_loaded<Real, kExtra>(s, st, N, P, m, v_old, v_new, dt, advance, G, I);
+  one_node<Real, kExtra, false>(s, st, N, P, m, v, v, dt, G, I);
 }
 
 // Steady state of every gate at v (HH.reset_state), Ci = Ci0.
@@ -951,23 +1087,17 @@ __device__ __forceinline__ void steady_states(const Real* P, uint32_t m, Real* s
 // Row i of the next linear system without its axial part: excess = diagonal minus
 // the row's axial coefficients = 1 + dt G / cm, rhs = dt I / cm on membrane rows;
 // 0, 0 on boundary rows.  Cells solved whole take the diagonal, 1 + dt (D + G / cm).
+// pr: the node's parameter record, negative on boundary rows.
 template <typename Real>
-__device__ __forceinline__ void write_row(const TileView<Real>& tv, int i, uint16_t pr, Real dt, Real G, Real I) {
-  const Real* P = tv.params + size_t(pr) * tv.pstride;
+__device__ __forceinline__ Pair<Real> node_row(const TileView<Real>& tv, int i, int pr, Real dt, Real G, Real I) {
+  const Real invcm = tv.params[size_t(max(pr, 0)) * tv.pstride + BC_P_INVCM];
+  Real e = fma_rn(dt, mul_rn(invcm, G), Real(1)), r = mul_rn(mul_rn(dt, invcm), I);
+  if (pr < 0) e = r = Real(0);
   if (i >= tv.cell0 && i < tv.sep0) {
     const Real d0 = tv.diag0[i - tv.cell0];
-    if (pr == kBoundary) {
-      tv.dr[i] = make_pair(dt * d0, Real(0));
-    } else {
-      const Real invcm = P[BC_P_INVCM];
-      tv.dr[i] = make_pair(Real(1) + dt * (d0 + invcm * G), dt * invcm * I);
-    }
-  } else if (pr == kBoundary) {
-    tv.dr[i] = make_pair(Real(0), Real(0));
-  } else {
-    const Real invcm = P[BC_P_INVCM];
-    tv.dr[i] = make_pair(Real(1) + dt * (invcm * G), dt * invcm * I);
+    e = pr < 0 ? mul_rn(dt, d0) : fma_rn(dt, fma_rn(invcm, G, d0), Real(1));
   }
+  return make_pair(e, r);
 }
 
 // ExpSyn synapses of a node (synapse/markov.py:65-117).  `g` is stored as the
@@ -1006,11 +1136,11 @@ __device__ __forceinline__ void node_synapses(const LaunchArgs& a, const TileVie
 // Clamp pulses active at `step` on node i (the thread that wrote row i adds them).
 template <typename Real>
 __device__ __forceinline__ void add_node_pulses(const TileView<Real>& tv, const PulseRec* pulses, const SpecRec& sr,
-                                                int i, uint16_t pr, int64_t step, Real dt) {
+                                                int i, int pr, int64_t step, Real dt) {
   for (int k = sr.pulse_begin; k < sr.pulse_end; ++k) {
     const PulseRec p = pulses[k];
     if (step < p.on_step || step >= p.off_step) continue;
-    if (pr == kBoundary)
+    if (pr < 0)
       tv.dr[i].y += dt * Real(p.amp);
     else
       tv.dr[i].y += dt * tv.params[size_t(pr) * tv.pstride + BC_P_INVCM] * Real(p.amp);
@@ -1063,25 +1193,21 @@ __device__ __forceinline__ Real vdelta(const Pair<Real>& v, const Pair<Real>& up
 }
 
 // One warp slot: lane l eliminates segment seg0 + l.  kLower: the slot's segments
-// have a lower separator.  Nodes are taken kBatch at a time, all loads of a batch
-// issued together: taken one by one, each node cost about 250 cycles of exposed
-// shared-memory latency on each of the two walks.  A lane past its segment's end
-// reads its upper separator's node and drops the result.
+// have a lower separator.  Nodes are taken four at a time: one read of their row
+// starts, all loads of the batch issued together, and no branch inside it (a lane past
+// its segment's end reads its upper separator's node and keeps what it had).  Node by
+// node, each took about 250 cycles a walk, most of it exposed shared-memory latency and
+// divergent branches; the dependent arithmetic of a node is about 45.
 template <typename Real, bool kPre, bool kLower>
 __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  constexpr int kBatch = 4;
   const bool valid = lane < sr.n_lanes;
   const SegRec sg = tv.segs[sr.seg0 + (valid ? lane : 0)];
+  const int4* rq = reinterpret_cast<const int4*>(tv.rows + sr.rows0);
+  int4 r = rq[0];
   const int len = valid ? int(sg.len) : 0;
   const int max_len = sr.max_len;
   const int nt = tv.sep0 + sg.t;
-  int off = sr.n_begin;  // first node of row k of the slot
-  auto next_id = [&](int k) {
-    const int id = len > k ? off + lane : nt;
-    off += __popc(__ballot_sync(kFullMask, len > k));
-    return id;
-  };
-  int id0 = next_id(0);
+  int id0 = len > 0 ? r.x + lane : nt;
   Pair<Real> v0 = tv.v[id0];
   Real wE = Real(0), wF = Real(0), wR = Real(0), as = Real(0), ds = Real(0);
   Pair<Real> row_s = make_pair(Real(0), Real(0));
@@ -1094,64 +1220,61 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
     wE = wF = cs.y;
     wR = cs.y * ds;
   }
-  for (int k = 0; k < max_len; k += kBatch) {
-    int id[kBatch + 1];
-    Pair<Real> row[kBatch], c[kBatch], v[kBatch + 1];
-    id[0] = id0;
+  for (int k = 0; k < max_len; k += 4) {
+    const int4 rn = rq[k / 4 + 1];
+    const int id[5] = {id0, len > k + 1 ? r.y + lane : nt, len > k + 2 ? r.z + lane : nt, len > k + 3 ? r.w + lane : nt,
+                       len > k + 4 ? rn.x + lane : nt};
+    Pair<Real> row[4], c[4], v[5];
     v[0] = v0;
 #pragma unroll
-    for (int j = 1; j <= kBatch; ++j) id[j] = next_id(k + j);
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
+    for (int j = 0; j < 4; ++j) {
       row[j] = tv.dr[id[j]];
       c[j] = coef<Real, kPre>(tv, id[j], dt);
       v[j + 1] = tv.v[id[j + 1]];
     }
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
+    for (int j = 0; j < 4; ++j) {
+      const bool act = len > k + j;
       const Real delta = vdelta<Real>(v[j], v[j + 1]);
       const Real E = row[j].x + wE;
       const Real R = (row[j].y + wR) - c[j].x * delta;
       const Real inv = pivot_rcp(E + c[j].x);
-      if (len > k + j) {
-        tv.dr[id[j]] = make_pair(inv * R, c[j].x * inv);
-        const Real g = c[j].y * inv;
-        if (kLower) {
-          tv.q[id[j]] = inv * wF;
-          wF *= g;
-        }
-        wE = (c[j].y * E) * inv;
-        wR = g * R + c[j].y * delta;
+      const Real g = c[j].y * inv;
+      if (act) tv.dr[id[j]] = make_pair(inv * R, c[j].x * inv);
+      if (kLower) {
+        if (act) tv.q[id[j]] = inv * wF;
+        wF = act ? g * wF : wF;
       }
+      wE = act ? (c[j].y * E) * inv : wE;
+      wR = act ? g * R + c[j].y * delta : wR;
     }
-    id0 = id[kBatch];
-    v0 = v[kBatch];
+    id0 = id[4];
+    v0 = v[4];
+    r = rn;
   }
   if (!kLower && valid) tv.inbox[sg.inbox] = make_pair(wE, wR);
-  // back down (off is one past the slot's last node): x_k = p + q x_s + u x_t
+  // back down: x_k = p + q x_s + u x_t
   Real p = Real(0), q = Real(0), u = Real(1);
-  for (int k = max_len - 1; k >= 0; k -= kBatch) {
-    int id[kBatch];
-    Pair<Real> d[kBatch];
-    Real f[kBatch];
+  for (int k = (max_len - 1) & ~3; k >= 0; k -= 4) {
+    r = rq[k / 4];
+    const int id[4] = {r.x + lane, r.y + lane, r.z + lane, r.w + lane};
+    Pair<Real> d[4];
+    Real f[4];
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      off -= k >= j ? __popc(__ballot_sync(kFullMask, len > k - j)) : 0;
-      id[j] = k >= j && len > k - j ? off + lane : -1;
+    for (int j = 0; j < 4; ++j) {
+      const int i = len > k + j ? id[j] : nt;
+      d[j] = tv.dr[i];
+      f[j] = kLower ? tv.q[len > k + j ? id[j] : 0] : Real(0);
     }
 #pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      d[j] = id[j] >= 0 ? tv.dr[id[j]] : make_pair(Real(0), Real(1));
-      f[j] = kLower && id[j] >= 0 ? tv.q[id[j]] : Real(0);
-    }
-#pragma unroll
-    for (int j = 0; j < kBatch; ++j) {
-      p = d[j].x + d[j].y * p;
-      u = d[j].y * u;
-      q = f[j] + d[j].y * q;
-      if (id[j] >= 0) {
-        tv.dr[id[j]] = make_pair(p, u);
-        if (kLower) tv.q[id[j]] = q;
+    for (int j = 3; j >= 0; --j) {
+      const bool act = len > k + j;
+      p = act ? d[j].x + d[j].y * p : p;
+      u = act ? d[j].y * u : u;
+      if (act) tv.dr[id[j]] = make_pair(p, u);
+      if (kLower) {
+        q = act ? f[j] + d[j].y * q : q;
+        if (act) tv.q[id[j]] = q;
       }
     }
   }
@@ -1173,7 +1296,7 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
 // records cost more than the walk.
 template <typename Real, bool kPre>
 __device__ __forceinline__ void solve_cells(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
-  const int32_t* rows = tv.rows + sr.seg0;
+  const int32_t* rows = tv.rows + sr.rows0;
   bool carry = false;
   Pair<Real> pc = make_pair(Real(0), Real(0));
   Real pw = Real(0), pR = Real(0), pd = Real(0);
@@ -1246,60 +1369,59 @@ __device__ __forceinline__ SepItem<Real> load_sep(const TileView<Real>& tv, int 
   return it;
 }
 
-template <typename Real>
-__device__ __forceinline__ void eliminate_sep(const TileView<Real>& tv, int j, const SepItem<Real>& it) {
-  const InPair<Real>* in = reinterpret_cast<const InPair<Real>*>(tv.inbox) + it.rec.in0;
-  InPair<Real> c = in[0];
-  Real E = it.row.e + (c.e0 + c.e1), R = it.row.r + (c.r0 + c.r1);
-  for (int k = 1; k < it.rec.n_in; ++k) {
-    c = in[k];
-    E += c.e0 + c.e1;
-    R += c.r0 + c.r1;
-  }
-  const Real inv = pivot_rcp(E + it.row.a);
-  const Real w = it.row.b * inv;
-  tv.inbox[it.rec.inbox] = make_pair(it.own.x + w * E, it.own.y + w * R);
-  tv.dr[tv.sep0 + j] = make_pair(it.row.a * inv, R * inv);
-}
-
-// The separator tree: a warp per group of cells, lanes over the separators of a
-// level.  A level's own data are loaded while the level before is eliminated, so
-// what is left per level is the inbox, one reciprocal and two stores: the sweep is
-// one warp's chain of dependent instructions, and every one of them counts.
+// The separator tree: a warp per group of cells, up to 32 separators of a level at a
+// time.  A chunk's own data are loaded while the chunk before is eliminated, inboxes of
+// up to four entries are read unconditionally, and the only branches are the loops':
+// this is one warp's chain of dependent instructions, where a branch costs 15 to 25
+// cycles and a chunk's arithmetic about 100.
 template <typename Real>
 __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int warp, int n_warps, int lane) {
+  const InPair<Real>* inbox = reinterpret_cast<const InPair<Real>*>(tv.inbox);
+  const int j_last = tv.n_seps - 1;
   for (int g = warp; g < tv.n_groups; g += n_warps) {
     const GroupRec gr = tv.groups[g];
     const int32_t* lv = tv.levels + gr.lv0;
-    int b = lv[0], e = lv[1];
-    SepItem<Real> it = load_sep(tv, min(b + lane, e - 1));
-    for (int l = 0; l < gr.n_lv; ++l) {
-      const int e1 = lv[min(l + 2, gr.n_lv)];
-      const SepItem<Real> nx = load_sep(tv, min(e + lane, tv.n_seps - 1));
-      if (b + lane < e) eliminate_sep(tv, b + lane, it);
-      for (int j = b + lane + 32; j < e; j += 32) eliminate_sep(tv, j, load_sep(tv, j));
+    uint32_t cb = uint32_t(lv[0]), ce = uint32_t(lv[1]);
+    int b = int(cb & ~kChunkMore);
+    SepItem<Real> it = load_sep(tv, min(b + lane, j_last));
+    for (int l = 0; l < gr.n_chunks; ++l) {
+      const uint32_t cn = uint32_t(lv[min(l + 2, gr.n_chunks)]);
+      const int e = int(ce & ~kChunkMore);
+      const SepItem<Real> nx = load_sep(tv, min(e + lane, j_last));
+      const InPair<Real> c0 = inbox[it.rec.in0], c1 = inbox[it.rec.in0 + 1];
+      Real E = it.row.e + ((c0.e0 + c0.e1) + (c1.e0 + c1.e1));
+      Real R = it.row.r + ((c0.r0 + c0.r1) + (c1.r0 + c1.r1));
+      if (cb & kChunkMore) {
+        for (int k = 2; k < it.rec.n_in; ++k) {
+          const InPair<Real> c = inbox[it.rec.in0 + k];
+          E += c.e0 + c.e1;
+          R += c.r0 + c.r1;
+        }
+      }
+      const Real inv = pivot_rcp(E + it.row.a);
+      const Real w = it.row.b * inv;
+      const bool valid = b + lane < e;
+      if (valid) tv.inbox[it.rec.inbox] = make_pair(it.own.x + w * E, it.own.y + w * R);
+      if (valid) tv.dr[tv.sep0 + b + lane] = make_pair(it.row.a * inv, R * inv);
       __syncwarp();
       b = e;
-      e = e1;
+      cb = ce;
+      ce = cn;
       it = nx;
     }
-    // back down: x = R / D + A / D x_t (A = 0 and t = itself at a root), the next
-    // level's pairs loaded ahead
-    e = lv[gr.n_lv];
-    b = lv[gr.n_lv - 1];
-    int j = min(b + lane, e - 1);
+    // back down: x = R / D + A / D x_t (A = 0 and t = itself at a root)
+    int e = b;
+    b = lv[gr.n_chunks - 1] & int(~kChunkMore);
+    int j = min(b + lane, j_last);
     uint32_t t = tv.seps[j].t;
     Pair<Real> d = tv.dr[tv.sep0 + j];
-    for (int l = gr.n_lv - 1; l >= 0; --l) {
-      const int b1 = lv[max(l - 1, 0)];
-      const int j1 = min(b1 + lane, e - 1);
+    for (int l = gr.n_chunks - 1; l >= 0; --l) {
+      const int b1 = lv[max(l - 1, 0)] & int(~kChunkMore);
+      const int j1 = min(b1 + lane, j_last);
       const uint32_t t1 = tv.seps[j1].t;
       const Pair<Real> d1 = tv.dr[tv.sep0 + j1];
-      if (b + lane < e) tv.xsep[b + lane] = d.y + d.x * tv.xsep[t];
-      for (int i = b + lane + 32; i < e; i += 32) {
-        const Pair<Real> di = tv.dr[tv.sep0 + i];
-        tv.xsep[i] = di.y + di.x * tv.xsep[tv.seps[i].t];
-      }
+      const Real x = d.y + d.x * tv.xsep[t];
+      if (b + lane < e) tv.xsep[b + lane] = x;
       __syncwarp();
       e = b;
       b = b1;
@@ -1309,16 +1431,33 @@ __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int w
   }
 }
 
-// The solved increment of node i.
-template <typename Real>
-__device__ __forceinline__ Real node_increment(const TileView<Real>& tv, int i) {
-  const uint32_t lk = tv.link[i], s = lk >> 16;
-  const Pair<Real> d = tv.dr[i];
-  if (s == kLinkCell) return d.y;
-  const Real xt = tv.xsep[lk & 0xFFFF];
-  if (s == kLinkSelf) return xt;
-  const Real x = d.x + d.y * xt;
-  return s == kLinkNone ? x : x + tv.q[i] * tv.xsep[s];
+// The solved increments of nodes i .. i + W - 1; i0: the warp's first node.
+template <typename Real, int W>
+__device__ __forceinline__ void node_increments(const TileView<Real>& tv, int i, int i0, Real (&x)[W]) {
+  if (i0 + 32 * W <= tv.cell0) {  // segment nodes
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      const Pair<Real> d = tv.dr[i + j];
+      const uint32_t lk = tv.link[i + j];
+      x[j] = fma_rn(d.y, tv.xsep[lk & 0xFFFF], d.x);
+      if (i + j < tv.n_lower) x[j] = fma_rn(tv.q[i + j], tv.xsep[lk >> 16], x[j]);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+      const int k = i + j;
+      const Pair<Real> d = tv.dr[k];
+      if (k >= tv.sep0) {
+        x[j] = tv.xsep[k - tv.sep0];  // (0 in the padding)
+      } else if (k >= tv.cell0) {
+        x[j] = d.y;
+      } else {
+        const uint32_t lk = tv.link[k];
+        x[j] = fma_rn(d.y, tv.xsep[lk & 0xFFFF], d.x);
+        if (k < tv.n_lower) x[j] = fma_rn(tv.q[k], tv.xsep[lk >> 16], x[j]);
+      }
+    }
+  }
 }
 
 // ------------------------------------------------------------ surrogate ports
@@ -1503,6 +1642,124 @@ __device__ __forceinline__ bool is_finite_real(Real x) {
   return isfinite(x);
 }
 
+// ------------------------------------------------------------------ the update pass
+struct StepCtx {
+  int64_t step, rec_slot;
+  bool last, record;
+};
+
+// One warp's turn of the update: the lane's nodes i .. i + W - 1 (ok: it has any; a lane
+// without works on another's and stores nothing), i0 the warp's first node.  V += x, the
+// mechanisms, the next step's row, probes, spikes and the pulses of the next step.
+// Returns whether a voltage is not finite.
+//
+// Light nodes go two to a lane in FP32 (kHeavy = false, W = 2): half the loads, stores,
+// branches and address arithmetic a node, and two independent chains.  The tile's node
+// count is a multiple of 4 and its padding is boundary nodes that move nothing.  Heavy
+// nodes (a few somas, or every node of a cell) have a list of their own, one to a lane:
+// spread over the light nodes' warps, each made its warp the last at the barrier, with
+// about 3 thousand cycles of dependent accurate functions on top of its share.
+template <typename Real, int W, bool kHeavy, bool kExtra>
+__device__ __forceinline__ bool update_nodes(const LaunchArgs& a, const TileView<Real>& tv, const PulseRec* pulses,
+                                             const StepCtx& c, int i, bool ok, int i0, Real dt) {
+  int pr[W];
+  uint32_t m[W], m_any = 0;
+  const Real* P[W];
+  bool mine[W], all_mine = ok, any_mine = false;
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const uint16_t rec = tv.pidx[i + j];
+    pr[j] = rec == kBoundary ? -1 : int(rec);
+    m[j] = pr[j] >= 0 ? tv.mech[pr[j]] : 0u;
+    mine[j] = ok && (kHeavy || !(m[j] & kHeavyMech));
+    all_mine = all_mine && mine[j];
+    any_mine = any_mine || mine[j];
+    if (!mine[j]) m[j] = 0u;
+    m_any |= m[j];
+    P[j] = tv.params + size_t(max(pr[j], 0)) * tv.pstride;
+  }
+  const uint32_t mu = __reduce_or_sync(kFullMask, m_any);
+  // the states live in global memory (L2): read first, needed after the voltage
+  NodeStates<Real, W> st;
+  load_states(tv.state + i, tv.N, mu, st);
+  Real hi[W], lo[W], v_old[W], lo_old[W], x[W], G[W], I[W];
+  node_increments<Real, W>(tv, i, i0, x);
+  bool bad = false;
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const Pair<Real> vv = tv.v[i + j];
+    hi[j] = v_old[j] = vv.x;
+    lo[j] = lo_old[j] = vv.y;
+    ff_add(hi[j], lo[j], x[j]);
+    bad = bad || (mine[j] && !is_finite_real(hi[j]));
+  }
+  if (all_mine) {
+#pragma unroll
+    for (int j = 0; j < W; ++j) tv.v[i + j] = make_pair(hi[j], lo[j]);
+  } else if (any_mine) {
+    for (int j = 0; j < W; ++j)
+      if (mine[j]) tv.v[i + j] = make_pair(hi[j], lo[j]);
+  }
+  if (c.last) {  // last_V of the per-CV spike indicator (cell.py:2384-2386)
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (mine[j]) {
+        tv.state[size_t(kSlotVLastHi) * tv.N + i + j] = v_old[j];
+        tv.state[size_t(kSlotVLastLo) * tv.N + i + j] = lo_old[j];
+      }
+  }
+  node_mechanisms<Real, W, kHeavy, kExtra, true, true>(st, tv.state + i, tv.N, P, m, mu, all_mine, v_old, hi, dt, G, I);
+  Pair<Real> row[W];
+  uint16_t spec[W];
+  bool special = false;
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    row[j] = node_row(tv, i + j, pr[j], dt, G[j], I[j]);
+    spec[j] = mine[j] ? tv.spec[i + j] : kNoSpecial;
+    special = special || spec[j] != kNoSpecial;
+  }
+  if (!c.last) {
+    if (all_mine) {
+#pragma unroll
+      for (int j = 0; j < W; ++j) tv.dr[i + j] = row[j];
+    } else if (any_mine) {
+      for (int j = 0; j < W; ++j)
+        if (mine[j]) tv.dr[i + j] = row[j];
+    }
+  }
+  if (special) {
+    for (int j = 0; j < W; ++j) {
+      if (spec[j] == kNoSpecial) continue;
+      const SpecRec sr = tv.specs[spec[j]];
+      if (kExtra && sr.syn_begin < sr.syn_end) {
+        node_synapses(a, tv, sr, hi[j], dt, true, c.last, c.step + 1, G[j], I[j]);
+        if (!c.last) tv.dr[i + j] = node_row(tv, i + j, pr[j], dt, G[j], I[j]);
+      }
+      if (sr.probe >= 0) {
+        const double v1 = double(hi[j]) + double(lo[j]), v0 = double(v_old[j]) + double(lo_old[j]);
+        if (v0 < 0.0 && v1 >= 0.0) {
+          const int n = a.spike_count[sr.probe];
+          if (n < a.max_spikes)
+            a.spike_times[int64_t(sr.probe) * a.max_spikes + n] =
+                double(c.step) * a.dt + a.dt * (0.0 - v0) / (v1 - v0);
+          a.spike_count[sr.probe] = n + 1;
+        }
+        if (c.record && c.rec_slot < a.trace_cap) a.traces[c.rec_slot * a.n_probes_total + sr.probe] = v1;
+      }
+      if (!c.last) add_node_pulses(tv, pulses, sr, i + j, pr[j], c.step + 1, dt);
+    }
+  }
+  if (kExtra && tv.has_src) {
+    // a spike of the cell: any of its CVs crossing 0 mV upward in this step
+    for (int j = 0; j < W; ++j) {
+      const uint16_t lc = tv.ncell[i + j];
+      if (mine[j] && pr[j] >= 0 && lc != 0xFFFF && Real(v_old[j] + lo_old[j]) < Real(0) && Real(hi[j] + lo[j]) >= Real(0))
+        tv.stamp[lc] = int32_t(c.step & 0x7fffffff);
+    }
+  }
+  return bad;
+}
+
 // ------------------------------------------------------------------ the step kernel
 // kVar: 0 = lean (no optional mechanism), 1 = extra (synapses, network,
 // out-of-line channels), 2 = extra + subtree-surrogate ports, 3 = lean + ports
@@ -1575,20 +1832,38 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
     Real G = Real(0), I = Real(0);
     if (pr != kBoundary) {
       const Real v = tv.v[i].x;
-      node_mechanisms<Real, kExtra>(tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride, tv.mech[pr], v, v, dt,
-                                    false, G, I);
+      node_currents<Real, kExtra>(tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride, tv.mech[pr], v, dt, G, I);
     }
     const uint16_t sp = tv.spec[i];
     if (sp != kNoSpecial) {
       const SpecRec sr = tv.specs[sp];
       if (kExtra && sr.syn_begin < sr.syn_end) node_synapses(a, tv, sr, tv.v[i].x, dt, false, false, a.step0, G, I);
     }
-    write_row(tv, i, pr, dt, G, I);
-    if (sp != kNoSpecial) add_node_pulses(tv, pulses, tv.specs[sp], i, pr, a.step0, dt);
+    const int rec = pr == kBoundary ? -1 : int(pr);
+    tv.dr[i] = node_row(tv, i, rec, dt, G, I);
+    if (sp != kNoSpecial) add_node_pulses(tv, pulses, tv.specs[sp], i, rec, a.step0, dt);
+  }
+  {
+    // the launch's parameter records: in place in shared memory, in the scratch otherwise
+    Real* rec = kSmem ? const_cast<Real*>(tv.params) : reinterpret_cast<Real*>(scratch + td.off_wparams);
+    if (!kSmem)
+      for (int k = tid; k < td.n_params * tv.pstride; k += T) rec[k] = tv.params[k];
+    __syncthreads();  // the rows above read the records as they were
+    for (int r = tid; r < td.n_params; r += T) {
+      const Real* P = tv.params + size_t(r) * tv.pstride;
+      Real* L = rec + size_t(r) * tv.pstride;
+      const uint32_t m = tv.mech[r];
+      constexpr int keys[] = {BC_P_CA_D,    BC_P_CA_TAU,  BC_P_NA_PHI,  BC_P_KDR_PHI, BC_P_CAL_PHIP,
+                              BC_P_CAL_PHIQ, BC_P_CAT_PHIP, BC_P_CAT_PHIQ, BC_P_HCN_PHI, BC_P_AHP_PHI};
+#pragma unroll
+      for (int k : keys) L[k] = launch_param(P, m, k, dt);  // CA_D first: it reads CA_TAU
+    }
+    tv.params = rec;
   }
   // inbox entries that no segment fills stay 0; a root reads its own xsep times 0
   for (int i = tid; i < tv.n_inbox; i += T) tv.inbox[i] = make_pair(Real(0), Real(0));
-  for (int i = tid; i < tv.n_seps; i += T) tv.xsep[i] = Real(0);
+  for (int i = tid; i < tv.n_seps + kSepPad; i += T) tv.xsep[i] = Real(0);
+  for (int i = tv.n_real + tid; i < tv.N; i += T) tv.dr[i] = make_pair(Real(0), Real(0));
   if (tv.has_src)
     for (int c = tid; c < tv.n_cells; c += T) tv.stamp[c] = -1;
   __syncthreads();
@@ -1628,6 +1903,14 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
   do {                \
   } while (0)
 #endif
+  // steps to the next trace record, and its index
+  int rec_in = 0;
+  int64_t rec_slot = 0;
+  if (a.record_every > 0) {
+    const int64_t since = a.step0 - a.trace_base;
+    rec_in = a.record_every - 1 - int(since % a.record_every);
+    rec_slot = since / a.record_every;
+  }
   for (int s = 0; s < a.n_steps; ++s) {
     const int64_t step = a.step0 + s;
     eliminate_segments<Real, kSmem>(tv, warp, n_warps, lane, dt);
@@ -1638,79 +1921,26 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
     BC_TICK(1);
     // V update, mechanism states, next row, probes and next pulses
     const bool last = s + 1 == a.n_steps;
-    const int64_t k_since = step + 1 - a.trace_base;
-    const bool record = a.record_every > 0 && k_since % a.record_every == 0;
-    // The states live in global memory (L2): the next node's are loaded one
-    // iteration ahead so that their latency overlaps this node's arithmetic.
-    NodeStates<Real> cur;
-    uint16_t pr_cur = kBoundary;
-    if (tid < tv.n_real) {
-      pr_cur = tv.pidx[tid];
-      if (pr_cur != kBoundary) load_states(tv.state + tid, tv.N, tv.mech[pr_cur], cur);
-    }
-    for (int i = tid; i < tv.n_real; i += T) {
-      NodeStates<Real> nxt;
-      uint16_t pr_nxt = kBoundary;
-      if (i + T < tv.n_real) {
-        pr_nxt = tv.pidx[i + T];
-        if (pr_nxt != kBoundary) load_states(tv.state + i + T, tv.N, tv.mech[pr_nxt], nxt);
-      }
-      const Pair<Real> vv = tv.v[i];
-      Real hi = vv.x, lo = vv.y;
-      const Real v_old = hi, lo_old = lo;
-      ff_add(hi, lo, node_increment(tv, i));
-      tv.v[i] = make_pair(hi, lo);
-      if (last) {  // last_V of the per-CV spike indicator (cell.py:2384-2386)
-        tv.state[size_t(kSlotVLastHi) * tv.N + i] = v_old;
-        tv.state[size_t(kSlotVLastLo) * tv.N + i] = lo_old;
-      }
-      if (!is_finite_real(hi)) s_status = kStatusNonfinite;
-      const uint16_t pr = pr_cur;
-      Real G = Real(0), I = Real(0);
-      if (pr != kBoundary)
-        node_mechanisms_loaded<Real, kExtra>(cur, tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride, tv.mech[pr],
-                                             v_old, hi, dt, true, G, I);
-      cur = nxt;
-      pr_cur = pr_nxt;
-      const uint16_t sp = tv.spec[i];
-      SpecRec sr;
-      if (sp != kNoSpecial) {
-        sr = tv.specs[sp];
-        if (kExtra && sr.syn_begin < sr.syn_end) node_synapses(a, tv, sr, hi, dt, true, last, step + 1, G, I);
-      }
-      if (!last) write_row(tv, i, pr, dt, G, I);
-      if (kExtra && tv.has_src && pr != kBoundary) {
-        // a spike of the cell: any of its CVs crossing 0 mV upward in this step
-        const uint16_t lc = tv.ncell[i];
-        if (lc != 0xFFFF && Real(v_old + lo_old) < Real(0) && Real(hi + lo) >= Real(0))
-          tv.stamp[lc] = int32_t(step & 0x7fffffff);
-      }
-      if (sp != kNoSpecial) {
-        if (sr.probe >= 0) {
-          const double v1 = double(hi) + double(lo), v0 = double(v_old) + double(lo_old);
-          if (v0 < 0.0 && v1 >= 0.0) {
-            const int n = a.spike_count[sr.probe];
-            if (n < a.max_spikes)
-              a.spike_times[int64_t(sr.probe) * a.max_spikes + n] = double(step) * a.dt + a.dt * (0.0 - v0) / (v1 - v0);
-            a.spike_count[sr.probe] = n + 1;
-          }
-          if (record) {
-            const int64_t slot = k_since / a.record_every - 1;
-            if (slot >= 0 && slot < a.trace_cap) a.traces[slot * a.n_probes_total + sr.probe] = v1;
-          }
-        }
-        if (!last) add_node_pulses(tv, pulses, sr, i, pr, step + 1, dt);
-      }
-    }
+    const bool record = a.record_every > 0 && rec_in == 0;
+    const StepCtx ctx{step, rec_slot, last, record};
+    constexpr int W = sizeof(Real) == 4 ? 2 : 1;
+    bool bad = false;
+    for (int h0 = (n_warps - 1 - warp) * 32; h0 < tv.n_heavy; h0 += T)
+      bad |= update_nodes<Real, 1, true, kExtra>(a, tv, pulses, ctx, tv.heavy[min(h0 + lane, tv.n_heavy - 1)],
+                                                 h0 + lane < tv.n_heavy, tv.N, dt);
+    if (tv.n_heavy < tv.n_real)
+      for (int i0 = warp * (32 * W); i0 < tv.N; i0 += W * T)
+        bad |= update_nodes<Real, W, false, kExtra>(a, tv, pulses, ctx, min(i0 + W * lane, tv.N - W),
+                                                    i0 + W * lane < tv.N, i0, dt);
+    if (bad) s_status = kStatusNonfinite;
     __syncthreads();
     if (kExtra && record && td.n_xprobes > 0) {
       // mechanism probes (plans with them run the extra variant): state views after the update
       const ProbeRef* pl = reinterpret_cast<const ProbeRef*>(reinterpret_cast<const unsigned char*>(tv.specs) +
                                                              (td.off_plist - td.off_specs));
-      const int64_t slot = k_since / a.record_every - 1;
       for (int q = tid; q < td.n_xprobes; q += T) {
         const ProbeRef r = pl[q];
-        if (slot < 0 || slot >= a.trace_cap) continue;
+        if (rec_slot >= a.trace_cap) continue;
         double val;
         if (r.field >= BC_PROBE_CURRENT) {
           const uint16_t pr = tv.pidx[r.node];
@@ -1720,7 +1950,7 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
         } else {
           val = probe_state(tv.state + r.node, tv.N, r.field);
         }
-        a.traces[slot * a.n_probes_total + r.id] = val;
+        a.traces[rec_slot * a.n_probes_total + r.id] = val;
       }
     }
     if (kExtra && tv.has_src)
@@ -1734,6 +1964,10 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
             s_status = kStatusRecordOverflow;
           }
         }
+    if (--rec_in < 0) {
+      rec_in = a.record_every - 1;
+      ++rec_slot;
+    }
     BC_TICK(2);
     if constexpr (kPorts) {
       if (td.n_ports > 0 && !last) {
@@ -1799,15 +2033,13 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
     const uint16_t pr = tv.pidx[i];
     Real G = Real(0), I = Real(0);
     if (pr != kBoundary) {
-      NodeStates<Real> st;
-      load_states(tv.state + i, tv.N, tv.mech[pr], st);
-      const Real v = tv.v[i].x;
-      node_mechanisms_loaded<Real, kExtra>(st, tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride, tv.mech[pr],
-                                           v, v, dt, false, G, I);
+      node_currents<Real, kExtra>(tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride, tv.mech[pr], tv.v[i].x, dt,
+                                  G, I);
     }
-    write_row(tv, i, pr, dt, G, I);
+    const int rec = pr == kBoundary ? -1 : int(pr);
+    tv.dr[i] = node_row(tv, i, rec, dt, G, I);
     const uint16_t sp = tv.spec[i];
-    if (sp != kNoSpecial) add_node_pulses(tv, pulses, tv.specs[sp], i, pr, a.step0, dt);
+    if (sp != kNoSpecial) add_node_pulses(tv, pulses, tv.specs[sp], i, rec, a.step0, dt);
   }
   for (int s = 0; s < a.n_steps; ++s) {
     const int64_t step = a.step0 + s;
@@ -1899,7 +2131,7 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
     const bool last = s + 1 == a.n_steps;
     const int64_t k_since = step + 1 - a.trace_base;
     const bool record = a.record_every > 0 && k_since % a.record_every == 0;
-    NodeStates<Real> cur;
+    NodeStates<Real, 1> cur;
     uint16_t pr_cur = kBoundary;
     if (n > 0) {
       pr_cur = tv.pidx[lane];
@@ -1907,7 +2139,7 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
     }
     for (int k = 0; k < n; ++k) {
       const int i = k * L + lane;
-      NodeStates<Real> nxt;
+      NodeStates<Real, 1> nxt;
       uint16_t pr_nxt = kBoundary;
       if (k + 1 < n) {
         pr_nxt = tv.pidx[i + L];
@@ -1926,11 +2158,12 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
       const uint16_t pr = pr_cur;
       Real G = Real(0), I = Real(0);
       if (pr != kBoundary)
-        node_mechanisms_loaded<Real, kExtra>(cur, tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride,
-                                             tv.mech[pr], v_old, hi, dt, true, G, I);
+        one_node<Real, kExtra, true>(cur, tv.state + i, tv.N, tv.params + size_t(pr) * tv.pstride, tv.mech[pr], v_old,
+                                     hi, dt, G, I);
       cur = nxt;
       pr_cur = pr_nxt;
-      if (!last) write_row(tv, i, pr, dt, G, I);
+      const int rec = pr == kBoundary ? -1 : int(pr);
+      if (!last) tv.dr[i] = node_row(tv, i, rec, dt, G, I);
       const uint16_t sp = tv.spec[i];
       if (sp != kNoSpecial) {
         const SpecRec sr = tv.specs[sp];
@@ -1948,7 +2181,7 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
             if (slot >= 0 && slot < a.trace_cap) a.traces[slot * a.n_probes_total + sr.probe] = v1;
           }
         }
-        if (!last) add_node_pulses(tv, pulses, sr, i, pr, step + 1, dt);
+        if (!last) add_node_pulses(tv, pulses, sr, i, rec, step + 1, dt);
       }
     }
   }

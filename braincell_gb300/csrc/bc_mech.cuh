@@ -35,7 +35,8 @@ __device__ __forceinline__ float dexpm1(float x) { return expm1f(x); }
 __host__ __device__ __forceinline__ double dexpm1(double x) { return expm1(x); }
 __device__ __forceinline__ float dlog(float x) { return logf(x); }
 __host__ __device__ __forceinline__ double dlog(double x) { return log(x); }
-__device__ __forceinline__ float dpow(float x, float y) { return powf(x, y); }
+// x^y, out of line: the step only takes it for a calcium exponent other than 2.
+static __device__ __noinline__ float dpow(float x, float y) { return powf(x, y); }
 __host__ __device__ __forceinline__ double dpow(double x, double y) { return pow(x, y); }
 // The FP64 forms and the rate structures are also host functions, so that a host
 // build of this header can check the FP64 rates against the oracle on a CPU; the
@@ -55,21 +56,83 @@ __device__ __forceinline__ float rcp_approx(float x) {
 __device__ __forceinline__ float rdiv(float a, float b) { return a * rcp_approx(b); }
 __host__ __device__ __forceinline__ double rdiv(double a, double b) { return a / b; }
 
+// a / b to about half an ulp, for finite non-zero b: one Newton correction of
+// a * rcp(b) (the IEEE division takes about three times the instructions and a
+// branch to a subroutine).
+__device__ __forceinline__ float adiv(float a, float b) {
+  const float r = rcp_approx(b);
+  const float q = a * r;
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+__host__ __device__ __forceinline__ double adiv(double a, double b) { return a / b; }
+
+// 1 / x for the step's rate forms.  FP64: two Newton-Raphson steps from the hardware
+// estimate, r += r (1 - x r) (x normal and finite: the forms below see to it); on the
+// host, and where the estimate does not exist, the division.
+__device__ __forceinline__ float srcp(float x) { return rcp_approx(x); }
+__host__ __device__ __forceinline__ double srcp(double x) {
+#ifdef __CUDA_ARCH__
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+#else
+  return 1.0 / x;
+#endif
+}
+
+// exp(k v + c) with constant k and c.  FP32: one multiply-add into the base-2
+// exponential, so the result may overflow to infinity (rcp makes it 0 again) but is
+// never wrong by a denormal's worth.  FP64: the exponent is capped at 700.
+constexpr double kLog2E = 1.4426950408889634;
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float lin_exp(float v, double k, double c) {
+  return ex2_ftz(fmaf(v, float(k * kLog2E), float(c * kLog2E)));
+}
+__host__ __device__ __forceinline__ double lin_exp(double v, double k, double c) { return exp(fmin(fma(v, k, c), 700.0)); }
+// exp(-|x| k), k > 0: at most 1, so squares and sums of it stay in range.
+__device__ __forceinline__ float exp_neg_abs(float x, double k) { return ex2_ftz(fabsf(x) * float(-k * kLog2E)); }
+__host__ __device__ __forceinline__ double exp_neg_abs(double x, double k) { return exp(fabs(x) * -k); }
+
 // e^x - 1 for the exp-Euler decay of a gate (x = dt * lambda <= 0).  FP32: for
 // |x| < 1/4 the Taylor series of e^x - 1 to x^6 (truncation < 5e-8 relative, the
-// float rounding level); otherwise __expf(x) - 1, which has no cancellation there.
-// FP64: expm1.
+// float rounding level); otherwise exp(x) - 1, which has no cancellation there.
+// FP64: the series to x^9 below 1/64 and to x^12 below 1/8 (truncation below 1e-18 of
+// the result), expm1 above.
 __device__ __forceinline__ float decay_em1(float x) {
   const float p = x * (1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f + x * (1.0f / 720.0f))))));
-  return fabsf(x) < 0.25f ? p : __expf(x) - 1.0f;
+  return fabsf(x) < 0.25f ? p : ex2_ftz(x * float(kLog2E)) - 1.0f;
 }
-__host__ __device__ __forceinline__ double decay_em1(double x) { return expm1(x); }
+__host__ __device__ __forceinline__ double decay_em1(double x) {
+  if (!(fabs(x) < 0.125)) return expm1(x);
+  double s = 1.0 / 362880;
+  if (fabs(x) >= 0.015625) s += x * (1.0 / 3628800 + x * (1.0 / 39916800 + x * (1.0 / 479001600)));
+  return x * (1.0 + x * (1.0 / 2 + x * (1.0 / 6 + x * (1.0 / 24 + x * (1.0 / 120 + x * (1.0 / 720 +
+         x * (1.0 / 5040 + x * (1.0 / 40320 + x * s))))))));
+}
 
 // exprel(x) = (e^x - 1) / x, exprel(0) = 1
 template <typename Real>
 __host__ __device__ __forceinline__ Real exprel(Real x) {
   return x == Real(0) ? Real(1) : dexpm1(x) / x;
 }
+
+// c / exprel(x) = c x / (e^x - 1), c at x = 0, with one division; FP32: x is capped at
+// 80, where the quotient is below 1e-32 of c.
+__device__ __forceinline__ float over_exprel(float c, float x) {
+  const float y = fminf(x, 80.0f);
+  return fabsf(y) < 1e-30f ? c : adiv(c * y, dexpm1(y));
+}
+__host__ __device__ __forceinline__ double over_exprel(double c, double x) {
+  return x == 0.0 ? c : c * (x / dexpm1(x));
+}
+// c / (1 + e^x), accurate; FP32: x capped at 80.
+__device__ __forceinline__ float over_1pexp(float c, float x) { return adiv(c, 1.0f + aexp(fminf(x, 80.0f))); }
+__host__ __device__ __forceinline__ double over_1pexp(double c, double x) { return c / (1.0 + aexp(x)); }
 
 // One exp-Euler step y += dt * exprel(dt * lam) * f of a gate whose right-hand
 // side is affine in the gate: with lam = -phi (a + b) and f = -lam (x_inf - x) the
@@ -78,7 +141,7 @@ __host__ __device__ __forceinline__ Real exprel(Real x) {
 template <typename Real, bool kExact = false>
 __device__ __forceinline__ Real gate_ab(Real x, Real a, Real b, Real phi, Real dt) {
   const Real s = a + b;
-  if (kExact) return x - dexpm1(-dt * phi * s) * (a / s - x);
+  if (kExact) return x - dexpm1(-dt * phi * s) * (adiv(a, s) - x);
   const Real xinf = rdiv(a, s);
   return x - decay_em1(-dt * phi * s) * (xinf - x);
 }
@@ -94,10 +157,10 @@ struct NaRates {
   Real ap, bp, aq, bq;
   __host__ __device__ __forceinline__ NaRates(Real v, Real vsh) {
     const Real vp = v - vsh;
-    ap = Real(0.32 * 4.0) / exprel(-(vp - Real(13)) * Real(1.0 / 4));
-    bp = Real(0.28 * 5.0) / exprel((vp - Real(40)) * Real(1.0 / 5));
+    ap = over_exprel(Real(0.32 * 4.0), -(vp - Real(13)) * Real(1.0 / 4));
+    bp = over_exprel(Real(0.28 * 5.0), (vp - Real(40)) * Real(1.0 / 5));
     aq = Real(0.128) * aexp(-(vp - Real(17)) * Real(1.0 / 18));
-    bq = Real(4) / (Real(1) + aexp(-(vp - Real(40)) * Real(1.0 / 5)));
+    bq = over_1pexp(Real(4), -(vp - Real(40)) * Real(1.0 / 5));
   }
 };
 
@@ -106,7 +169,7 @@ struct KdrRates {
   Real a, b;
   __host__ __device__ __forceinline__ KdrRates(Real v, Real vsh) {
     const Real vp = v - vsh;
-    a = Real(0.032 * 5.0) / exprel(-(vp - Real(15)) * Real(1.0 / 5));
+    a = over_exprel(Real(0.032 * 5.0), -(vp - Real(15)) * Real(1.0 / 5));
     b = Real(0.5) * aexp(-(vp - Real(10)) * Real(1.0 / 40));
   }
 };
@@ -151,15 +214,57 @@ struct HcnRates {
   }
 };
 
+// The main mix's steps take a gate's steady state and its exponent x = -dt phi / tau
+// (k = -dt phi) instead of tau: the reciprocals of the time constants' sums cancel, and
+// a CaL gate takes two exponentials and two reciprocals instead of two and three plus a
+// division of the bell; the bells' exponentials are taken of -|y|, so that nothing
+// overflows.
+template <typename Real>
+struct GateStep {
+  Real inf, x;
+  __host__ __device__ __forceinline__ Real step(Real g) const { return g - decay_em1(x) * (inf - g); }
+};
+template <typename Real>
+__host__ __device__ __forceinline__ Real bell_rate(Real k, Real y, double inv_width, double base, double height) {
+  const Real z = exp_neg_abs(y, inv_width);
+  const Real w = Real(1) + z * z;  // tau = base + height z / w
+  return k * w * srcp(Real(base) * w + Real(height) * z);
+}
+template <typename Real>
+__host__ __device__ __forceinline__ GateStep<Real> cal_p_step(Real vs, Real k) {
+  return {srcp(Real(1) + lin_exp(vs, -1.0 / 4, -10.0 / 4)), bell_rate(k, vs + Real(5), 1.0 / 15, 0.4, 0.7)};
+}
+template <typename Real>
+__host__ __device__ __forceinline__ GateStep<Real> cal_q_step(Real vs, Real k) {
+  return {srcp(Real(1) + lin_exp(vs, 1.0 / 2, 25.0 / 2)), bell_rate(k, vs + Real(40), 1.0 / 9.5, 300.0, 100.0)};
+}
+template <typename Real>
+__host__ __device__ __forceinline__ GateStep<Real> cat_p_step(Real vs, Real k) {
+  // tau = 1 / s + 0.612; s is capped where 1 / s no longer counts
+  Real s = lin_exp(vs, -1.0 / 16.7, -132.0 / 16.7) + lin_exp(vs, 1.0 / 18.2, 16.8 / 18.2);
+  s = s < Real(1e18) ? s : Real(1e18);
+  return {srcp(Real(1) + lin_exp(vs, -1.0 / 6.2, -59.0 / 6.2)), k * s * srcp(Real(1) + Real(0.612) * s)};
+}
+template <typename Real>
+__host__ __device__ __forceinline__ GateStep<Real> cat_q_step(Real vs, Real k) {
+  const Real tau = vs >= Real(-80) ? lin_exp(vs, -1.0 / 10.5, -22.0 / 10.5) + Real(28) : lin_exp(vs, 1.0 / 66.6, 467.0 / 66.6);
+  return {srcp(Real(1) + lin_exp(vs, 1.0 / 4, 83.0 / 4)), k * srcp(tau)};
+}
+template <typename Real>
+__host__ __device__ __forceinline__ GateStep<Real> hcn_step(Real v, Real k) {
+  return {srcp(Real(1) + lin_exp(v, 1.0 / 5.5, 75.0 / 5.5)),
+          k * (lin_exp(v, -0.086, -14.59) + lin_exp(v, 0.0701, -1.87))};
+}
+
 template <typename Real>
 struct NaHHRates {
   Real ap, bp, aq, bq;
   __host__ __device__ __forceinline__ NaHHRates(Real v, Real vsh) {
     const Real vp = v - vsh;
-    ap = Real(1) / exprel(-(vp - Real(5)) * Real(0.1));
+    ap = over_exprel(Real(1), -(vp - Real(5)) * Real(0.1));
     bp = Real(4) * aexp(-(vp + Real(20)) * Real(1.0 / 18));
     aq = Real(0.07) * aexp(-(vp + Real(20)) * Real(0.05));
-    bq = Real(1) / (Real(1) + aexp(-(vp - Real(10)) * Real(0.1)));
+    bq = over_1pexp(Real(1), -(vp - Real(10)) * Real(0.1));
   }
 };
 
@@ -168,7 +273,7 @@ struct KHHRates {
   Real a, b;
   __host__ __device__ __forceinline__ KHHRates(Real v, Real vsh) {
     const Real vp = v - vsh;
-    a = Real(0.1) / exprel(-(vp + Real(10)) * Real(0.1));
+    a = over_exprel(Real(0.1), -(vp + Real(10)) * Real(0.1));
     b = Real(0.125) * aexp(-(vp + Real(20)) * Real(1.0 / 80));
   }
 };

@@ -62,6 +62,9 @@ constexpr int kDefaultLaneNodes = 10;
 constexpr uint32_t kMarkovBits = BC_M_NAV16 | BC_M_KCA22 | BC_M_KCA11;
 constexpr uint32_t kCerebellarBits = BC_M_KV34 | BC_M_KV43 | BC_M_KV11 | BC_M_KIR23 | BC_M_HCN1F | BC_M_HCN1H |
                                      BC_M_CAHVA | BC_M_CAV23 | BC_M_CAV32;
+// mechanisms outside the main mix (the extra kernel variants)
+constexpr uint32_t kOutOfLineBits = BC_M_NAHH | BC_M_KHH | BC_M_KM | BC_M_KA1 | BC_M_KA2 | BC_M_KK2A | BC_M_KK2B |
+                                    BC_M_KNI | kMarkovBits | kCerebellarBits | BC_M_EXT;
 
 namespace bc {
 
@@ -523,7 +526,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   std::vector<GroupRec> groups;
   std::vector<int32_t> levels;
   std::vector<uint32_t> link;
-  std::vector<int32_t> rows;  // row starts of the slots of whole cells
+  std::vector<int32_t> rows;  // row starts of the slots
   int32_t next_node = 0, cell0 = 0, sep0 = 0, n_inbox = 0;
   int n_levels = 0;
   int64_t crit = 0, n_lower = 0;  // nodes of segments with a lower separator (they come first)
@@ -566,25 +569,30 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
         if (lv.size() < size_t(cs.n_levels)) lv.resize(cs.n_levels);
         for (size_t j = 0; j < cs.seps.size(); ++j) lv[cs.seps[j].level].push_back({li, int32_t(j)});
       }
-      groups.push_back({int32_t(levels.size()), int32_t(lv.size())});
+      GroupRec gr{int32_t(levels.size()), 0};
       n_levels = std::max(n_levels, int(lv.size()));
-      for (auto& v : lv) {
-        levels.push_back(int32_t(sep_src.size()));
-        for (auto& x : v) {
+      for (auto& v : lv)
+        for (size_t k = 0; k < v.size(); ++k) {
+          const auto& x = v[k];
+          if (k % 32 == 0) {
+            levels.push_back(int32_t(sep_src.size()));
+            ++gr.n_chunks;
+          }
+          if (sched_of(x.first).seps[x.second].in.size() > 4) levels.back() |= int32_t(kChunkMore);
           sep_tile[x.first][x.second] = int32_t(sep_src.size());
           sep_src.push_back(x);
         }
-      }
       levels.push_back(int32_t(sep_src.size()));
+      groups.push_back(gr);
     }
-    // -------- inboxes: one entry per segment, consecutive per upper separator, padded to pairs
+    // -------- inboxes: one entry per segment, consecutive per upper separator, padded to two or more pairs
     std::vector<std::vector<int32_t>> seg_inbox(cell_list.size());
     for (size_t li = 0; li < cell_list.size(); ++li) seg_inbox[li].resize(sched_of(li).segs.size());
     seps.resize(sep_src.size());
     for (size_t j = 0; j < sep_src.size(); ++j) {
       const auto [li, q] = sep_src[j];
       const Sep& sp = sched_of(li).seps[q];
-      const size_t pairs = std::max<size_t>(1, (sp.in.size() + 1) / 2);
+      const size_t pairs = std::max<size_t>(2, (sp.in.size() + 1) / 2);
       if (pairs > 0xFFFF) return fail(BC_ERR_CAPACITY, "too many branches at one point");
       seps[j] = SepRec{n_inbox / 2, -1, uint16_t(pairs), uint16_t(sp.t >= 0 ? size_t(sep_tile[li][sp.t]) : j), 0};
       for (size_t k = 0; k < sp.in.size(); ++k) seg_inbox[li][sp.in[k]] = n_inbox + int32_t(k);
@@ -597,6 +605,12 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
       }
     for (SepRec& sp : seps)
       if (sp.inbox < 0) sp.inbox = n_inbox++;
+    // the end of a slot's rows, and what the kernel's reads of four rows at a time may touch past it
+    auto end_rows = [&]() {
+      rows.push_back(next_node);
+      while (rows.size() % 4 != 0) rows.push_back(next_node);
+      rows.insert(rows.end(), 4, next_node);
+    };
     // -------- warp slots: segments with a lower separator first, then the leaves', longest first
     std::vector<std::pair<size_t, int32_t>> seg_src;
     for (int lower = 1; lower >= 0; --lower) {
@@ -613,7 +627,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
       std::stable_sort(v.begin(), v.end(), [&](const auto& x, const auto& y) { return len(x) > len(y); });
       for (size_t q = 0; q < v.size(); q += 32) {
         const size_t n_lanes = std::min<size_t>(32, v.size() - q);
-        SlotRec sr{next_node, int32_t(segs.size()), int16_t(n_lanes), uint16_t(len(v[q])), lower ? kSlotLower : kSlotLeaf};
+        SlotRec sr{int32_t(rows.size()), int32_t(segs.size()), int16_t(n_lanes), uint16_t(len(v[q])), lower ? kSlotLower : kSlotLeaf};
         for (size_t l = 0; l < n_lanes; ++l) {
           const auto& st = sep_tile[v[q + l].first];
           if (v[q + l].second < 0) {
@@ -628,13 +642,16 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
           segs.push_back(SegRec{uint16_t(st[sg.t]), uint16_t(sg.s >= 0 ? uint32_t(st[sg.s]) : kLinkNone),
                                 uint16_t(sg.nodes.size()), 0, seg_inbox[v[q + l].first][v[q + l].second], 0});
         }
-        for (size_t k = 0; k < sr.max_len; ++k)
+        for (size_t k = 0; k < sr.max_len; ++k) {
+          rows.push_back(next_node);
           for (size_t l = 0; l < n_lanes && len(v[q + l]) > k; ++l) {
             const Seg& sg = sched_of(v[q + l].first).segs[v[q + l].second];
             node_tile[v[q + l].first][sg.nodes[k]] = next_node++;
             const SegRec& rec = segs[sr.seg0 + l];
             link.push_back(uint32_t(rec.t) | (uint32_t(rec.s) << 16));
           }
+        }
+        end_rows();
         slots.push_back(sr);
       }
       if (lower == 1) n_lower = next_node;
@@ -646,7 +663,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     for (size_t q = 0; q < whole.size(); q += 32) {
       const size_t n_lanes = std::min<size_t>(32, whole.size() - q);
       const size_t max_len = sched_of(whole[q]).order.size();
-      slots.push_back(SlotRec{next_node, int32_t(rows.size()), int16_t(n_lanes), uint16_t(max_len), kSlotCell});
+      slots.push_back(SlotRec{int32_t(rows.size()), 0, int16_t(n_lanes), uint16_t(max_len), kSlotCell});
       for (size_t k = 0; k < max_len; ++k) {
         rows.push_back(next_node);
         for (size_t l = 0; l < n_lanes && sched_of(whole[q + l]).order.size() > k; ++l) {
@@ -662,7 +679,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
           node_tile[whole[q + l]][ord[k]] = next_node++;
         }
       }
-      rows.push_back(next_node);
+      end_rows();
     }
     // warp w takes slots w, w + W, ...: the dearest first
     std::stable_sort(slots.begin(), slots.end(), [](const SlotRec& a, const SlotRec& b) {
@@ -696,6 +713,20 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     out.crit = lane_kmax;
   }
   if (lane) cell0 = sep0 = int32_t(n_real);  // rows in the excess form
+  // -------- nodes with heavy mechanisms, ordered by their mechanisms, so that the lanes of a warp share them
+  std::vector<int32_t> heavy;
+  if (!lane) {
+    std::vector<std::pair<uint32_t, int32_t>> v;
+    for (size_t li = 0; li < cell_list.size(); ++li) {
+      const LoweredCell& lc = (*cx.cells)[cell_list[li]];
+      for (int32_t n = 0; n < lc.n_node; ++n) {
+        const uint32_t m = lc.region[n] >= 0 ? s.region_mech[cell_list[li] * R + lc.region[n]] : 0u;
+        if (m & (BC_M_NA | BC_M_KDR | kOutOfLineBits)) v.push_back({m, node_tile[li][n]});
+      }
+    }
+    std::sort(v.begin(), v.end());
+    for (const auto& x : v) heavy.push_back(x.second);
+  }
   std::vector<uint16_t> crec;
   if (lane) {  // lane tiles: the parent's node index v within the cell (0xFFFF at the root)
     crec.assign(size_t(n_real), 0);
@@ -770,6 +801,8 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   off = align16(off + rows.size() * 4);
   d.off_diag0 = int32_t(off);
   off = align16(off + size_t(sep0 - cell0) * rs);
+  d.off_heavy = int32_t(off);
+  off = align16(off + heavy.size() * 4);
   d.off_crec = int32_t(off);
   off = align16(off + crec.size() * 2);
   d.off_params = int32_t(off);
@@ -809,7 +842,9 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   d.off_q = int32_t(so);
   so = align16(so + size_t(n_lower) * rs);
   d.off_xsep = int32_t(so);
-  so = align16(so + seps.size() * rs);
+  so = align16(so + (seps.size() + kSepPad) * rs);
+  d.off_wparams = int32_t(so);
+  if (tb.cls == 2) so = align16(so + size_t(n_params) * cx.param_stride * rs);
   d.off_stamp = -1;
   if (has_src) {
     d.off_stamp = int32_t(so);
@@ -831,6 +866,8 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   d.n_seps = int32_t(seps.size());
   d.n_inbox = n_inbox;
   d.n_groups = int32_t(groups.size());
+  d.n_heavy = int32_t(heavy.size());
+  d.n_lower = int32_t(n_lower);
   d.cell0 = cell0;
   d.sep0 = sep0;
   d.n_params = int32_t(n_params);
@@ -838,9 +875,9 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   std::vector<unsigned char>& b = out.blob;
   b.assign(d.blob_bytes, 0);
   out.vinit.assign(n_real, 0.0);
-  if (lane) {  // holes of the lane grid are boundary rows the kernel never visits
-    std::vector<uint16_t> hole(size_t(N), 0xFFFF);
-    std::memcpy(b.data() + d.off_pidx, hole.data(), hole.size() * 2);
+  // the holes of a lane grid and the padding of a tile are boundary rows
+  std::memset(b.data() + d.off_pidx, 0xFF, size_t(N) * 2);
+  if (lane) {
     std::memcpy(b.data() + d.off_lane_n, lane_n.data(), lane_n.size() * 4);
   }
   auto putr = [&](size_t base_off, size_t idx, double v) {
@@ -1011,6 +1048,7 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   put_all(d.off_levels, levels.data(), levels.size() * 4);
   put_all(d.off_groups, groups.data(), groups.size() * sizeof(GroupRec));
   put_all(d.off_rows, rows.data(), rows.size() * 4);
+  put_all(d.off_heavy, heavy.data(), heavy.size() * 4);
   put_all(d.off_crec, crec.data(), crec.size() * 2);
   out.desc = d;
   return BC_OK;
@@ -1387,8 +1425,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   p->cell_ncv.resize(s.n_cells);
   for (int64_t c = 0; c < s.n_cells; ++c) p->cell_ncv[c] = cells[c].n_cv;
   for (int64_t k = 0; k < s.n_cells * s.n_regions; ++k)
-    p->extra = p->extra || (s.region_mech[k] & (BC_M_NAHH | BC_M_KHH | BC_M_KM | BC_M_KA1 | BC_M_KA2 | BC_M_KK2A |
-                                                 BC_M_KK2B | BC_M_KNI | kMarkovBits | kCerebellarBits | BC_M_EXT)) != 0;
+    p->extra = p->extra || (s.region_mech[k] & kOutOfLineBits) != 0;
   for (int64_t k = 0; k < s.n_cells * s.n_regions; ++k) {
     if (s.region_mech[k] & ~BC_M_ALL) {
       delete p;
