@@ -138,7 +138,12 @@ struct TileDesc {
   int32_t off_crec, off_params, off_mech;
   int32_t scratch_bytes;    // solver scratch (shared memory after the blob)
   int32_t off_dr;           // rows, inside the scratch area
-  int32_t off_q, off_inbox, off_srow, off_own, off_xsep;  // inside the scratch area
+  int32_t off_q;
+  // the separators' work area: off_sep .. off_sep + sep_bytes of the scratch, or the first
+  // sep_bytes of shared memory, with the records (off_seps .. off_rows of the blob) after
+  // them, when sep_in_smem (global-memory tiles)
+  int32_t off_sep, sep_bytes, sep_in_smem;
+  int32_t off_inbox, off_srow, off_own, off_xsep;  // inside the work area
   int32_t off_wparams;      // global-memory tiles: the launch's parameter records (scratch)
   int32_t n_slots;          // warp slots of the segment elimination
   int32_t n_groups;
@@ -300,6 +305,7 @@ struct ProbeRef {
 struct LaunchArgs {
   const TileDesc* tiles;
   int32_t n_tiles;
+  int32_t cluster;            // CTAs per tile (global-memory tiles; 1 otherwise)
   unsigned char* blob;        // plan blob buffer
   unsigned char* scratch;     // global scratch (global-resident tiles)
   void* state;                // mechanism states, [slot][node] per tile (Real)
@@ -345,7 +351,9 @@ struct LaunchArgs {
 // whose only optional feature is its ports).
 int launch_tiles(const LaunchArgs& a, int precision, bool smem, int threads, size_t smem_bytes, int variant,
                  void* stream);
-// Kernel-node parameters of the same launch for a CUDA graph.  kernelParams
+// Largest cluster, a power of two up to `want`, at which `count` global-memory tiles run at once.
+int tile_cluster(int precision, int variant, int want, int count, int threads, size_t smem_bytes);
+// Kernel-node parameters of the same launch for a CUDA graph (clusters of 1).  kernelParams
 // points at *hold, which points at *a: both must stay valid until the graph
 // call that consumes the parameters returns (it copies the argument).
 int tile_node_params(const LaunchArgs* a, int precision, bool smem, int threads, size_t smem_bytes, int variant,

@@ -162,7 +162,16 @@ struct TileView {
   int pstride;  // reals per parameter record
   bool has_src;
 
-  __device__ __forceinline__ void bind(const TileDesc& td, unsigned char* base, unsigned char* scratch, void* gstate) {
+  __device__ __forceinline__ void bind_seps(const TileDesc& td, unsigned char* sepw) {
+    inbox = reinterpret_cast<Pair<Real>*>(sepw + td.off_inbox);
+    srow = reinterpret_cast<SepRow<Real>*>(sepw + td.off_srow);
+    own = reinterpret_cast<Pair<Real>*>(sepw + td.off_own);
+  }
+
+  // sepw, sepr: the separators' work area and records (in the scratch and the blob, or
+  // both in shared memory for a global-memory tile)
+  __device__ __forceinline__ void bind(const TileDesc& td, unsigned char* base, unsigned char* scratch,
+                                       unsigned char* sepw, const unsigned char* sepr, void* gstate) {
     v = reinterpret_cast<Pair<Real>*>(base + td.off_v);
     ab = reinterpret_cast<Pair<Real>*>(base + td.off_ab);
     dr = reinterpret_cast<Pair<Real>*>(scratch + td.off_dr);
@@ -170,9 +179,9 @@ struct TileView {
     params = reinterpret_cast<const Real*>(base + td.off_params);
     slots = reinterpret_cast<const SlotRec*>(base + td.off_slots);
     segs = reinterpret_cast<const SegRec*>(base + td.off_segs);
-    seps = reinterpret_cast<const SepRec*>(base + td.off_seps);
-    levels = reinterpret_cast<const int32_t*>(base + td.off_levels);
-    groups = reinterpret_cast<const GroupRec*>(base + td.off_groups);
+    seps = reinterpret_cast<const SepRec*>(sepr);
+    levels = reinterpret_cast<const int32_t*>(sepr + (td.off_levels - td.off_seps));
+    groups = reinterpret_cast<const GroupRec*>(sepr + (td.off_groups - td.off_seps));
     link = reinterpret_cast<const uint32_t*>(base + td.off_link);
     rows = reinterpret_cast<const int32_t*>(base + td.off_rows);
     diag0 = reinterpret_cast<const Real*>(base + td.off_diag0);
@@ -184,10 +193,8 @@ struct TileView {
     specs = reinterpret_cast<const SpecRec*>(base + td.off_specs);
     mech = reinterpret_cast<const uint32_t*>(base + td.off_mech);
     q = reinterpret_cast<Real*>(scratch + td.off_q);
-    inbox = reinterpret_cast<Pair<Real>*>(scratch + td.off_inbox);
-    srow = reinterpret_cast<SepRow<Real>*>(scratch + td.off_srow);
-    own = reinterpret_cast<Pair<Real>*>(scratch + td.off_own);
-    xsep = reinterpret_cast<Real*>(scratch + td.off_xsep);
+    bind_seps(td, sepw);
+    xsep = reinterpret_cast<Real*>(sepw + td.off_xsep);
     syn = reinterpret_cast<const int32_t*>(base + td.off_syn);
     has_src = td.off_ncell >= 0;
     ncell = has_src ? reinterpret_cast<const uint16_t*>(base + td.off_ncell) : nullptr;
@@ -206,6 +213,17 @@ struct TileView {
     n_inbox = td.n_inbox;
   }
 };
+
+// Address of `p`, in this CTA's shared memory, in that of CTA `rank` of its cluster.
+__device__ __forceinline__ unsigned char* cluster_map(unsigned char* p, uint32_t rank) {
+  uint64_t out;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(out) : "l"(reinterpret_cast<uint64_t>(p)), "r"(rank));
+  return reinterpret_cast<unsigned char*>(out);
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 
 // Reciprocal of a Hines pivot.  FP32: the hardware approximation (about 1 ulp;
 // pivots are >= 1 on membrane rows and O(dt * g / C) on boundary rows, far from
@@ -1402,7 +1420,7 @@ __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int w
       const Real w = it.row.b * inv;
       const bool valid = b + lane < e;
       if (valid) tv.inbox[it.rec.inbox] = make_pair(it.own.x + w * E, it.own.y + w * R);
-      if (valid) tv.dr[tv.sep0 + b + lane] = make_pair(it.row.a * inv, R * inv);
+      if (valid) *reinterpret_cast<Pair<Real>*>(tv.srow + b + lane) = make_pair(it.row.a * inv, R * inv);
       __syncwarp();
       b = e;
       cb = ce;
@@ -1414,12 +1432,12 @@ __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int w
     b = lv[gr.n_chunks - 1] & int(~kChunkMore);
     int j = min(b + lane, j_last);
     uint32_t t = tv.seps[j].t;
-    Pair<Real> d = tv.dr[tv.sep0 + j];
+    Pair<Real> d = *reinterpret_cast<const Pair<Real>*>(tv.srow + j);
     for (int l = gr.n_chunks - 1; l >= 0; --l) {
       const int b1 = lv[max(l - 1, 0)] & int(~kChunkMore);
       const int j1 = min(b1 + lane, j_last);
       const uint32_t t1 = tv.seps[j1].t;
-      const Pair<Real> d1 = tv.dr[tv.sep0 + j1];
+      const Pair<Real> d1 = *reinterpret_cast<const Pair<Real>*>(tv.srow + j1);
       const Real x = d.y + d.x * tv.xsep[t];
       if (b + lane < e) tv.xsep[b + lane] = x;
       __syncwarp();
@@ -1774,7 +1792,17 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int s_status;
-  const TileDesc td = a.tiles[blockIdx.x];
+  // A global-memory tile runs on a cluster of a.cluster CTAs: warps and threads are
+  // counted through the cluster, and the barriers between phases are the cluster's.
+  const int csize = kSmem || kPorts ? 1 : a.cluster;
+  const int rank = csize == 1 ? 0 : int(blockIdx.x) % csize;
+  auto tile_sync = [&]() {
+    if (csize == 1)
+      __syncthreads();
+    else
+      cluster_sync();
+  };
+  const TileDesc td = a.tiles[csize == 1 ? int(blockIdx.x) : int(blockIdx.x) / csize];
   unsigned char* gblob = a.blob + td.blob_offset;
   unsigned char* base;
   unsigned char* scratch;
@@ -1810,11 +1838,24 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
     scratch = a.scratch + td.scratch_offset;
     __syncthreads();
   }
-  TileView<Real> tv;
-  tv.bind(td, base, scratch, a.state);
   const Real dt = Real(a.dt);
-  const int T = blockDim.x, tid = threadIdx.x;
+  const int T = blockDim.x * csize, tid = rank * blockDim.x + threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, n_warps = T >> 5;
+  TileView<Real> tv;
+  if constexpr (kSmem) {
+    tv.bind(td, base, scratch, scratch + td.off_sep, base + td.off_seps, a.state);
+  } else if (td.sep_in_smem) {
+    // the separators of a global-memory tile are swept in shared memory (by CTA 0 of a
+    // cluster, whose copy the segments of all CTAs fill; xsep is every CTA's own)
+    unsigned char* rec = smem + td.sep_bytes;
+    for (int k = threadIdx.x; k < (td.off_rows - td.off_seps) / 4; k += blockDim.x)
+      reinterpret_cast<int32_t*>(rec)[k] = reinterpret_cast<const int32_t*>(base + td.off_seps)[k];
+    tv.bind(td, base, scratch, smem, rec, a.state);
+    if (rank > 0) tv.bind_seps(td, cluster_map(smem, 0));
+    __syncthreads();
+  } else {
+    tv.bind(td, base, scratch, scratch + td.off_sep, base + td.off_seps, a.state);
+  }
   const PulseRec* pulses = a.pulses + td.pulse_offset;
   if constexpr (kSmem) {
     // the staged axial coefficients become (alpha dt, beta dt) for this launch
@@ -1848,7 +1889,7 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
     Real* rec = kSmem ? const_cast<Real*>(tv.params) : reinterpret_cast<Real*>(scratch + td.off_wparams);
     if (!kSmem)
       for (int k = tid; k < td.n_params * tv.pstride; k += T) rec[k] = tv.params[k];
-    __syncthreads();  // the rows above read the records as they were
+    tile_sync();  // the rows above read the records as they were
     for (int r = tid; r < td.n_params; r += T) {
       const Real* P = tv.params + size_t(r) * tv.pstride;
       Real* L = rec + size_t(r) * tv.pstride;
@@ -1861,12 +1902,13 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
     tv.params = rec;
   }
   // inbox entries that no segment fills stay 0; a root reads its own xsep times 0
-  for (int i = tid; i < tv.n_inbox; i += T) tv.inbox[i] = make_pair(Real(0), Real(0));
-  for (int i = tid; i < tv.n_seps + kSepPad; i += T) tv.xsep[i] = Real(0);
+  if (rank == 0)
+    for (int i = threadIdx.x; i < tv.n_inbox; i += blockDim.x) tv.inbox[i] = make_pair(Real(0), Real(0));
+  for (int i = threadIdx.x; i < tv.n_seps + kSepPad; i += blockDim.x) tv.xsep[i] = Real(0);
   for (int i = tv.n_real + tid; i < tv.N; i += T) tv.dr[i] = make_pair(Real(0), Real(0));
   if (tv.has_src)
     for (int c = tid; c < tv.n_cells; c += T) tv.stamp[c] = -1;
-  __syncthreads();
+  tile_sync();
   PortStage* pstage = nullptr;
   PortLocal* plocal = nullptr;
   uint2* wfrag = nullptr;
@@ -1914,10 +1956,19 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
   for (int s = 0; s < a.n_steps; ++s) {
     const int64_t step = a.step0 + s;
     eliminate_segments<Real, kSmem>(tv, warp, n_warps, lane, dt);
-    __syncthreads();
+    tile_sync();
     BC_TICK(0);
-    sweep_separators<Real>(tv, warp, n_warps, lane);
-    __syncthreads();
+    if (rank == 0) sweep_separators<Real>(tv, threadIdx.x >> 5, blockDim.x >> 5, lane);
+    if (csize > 1) {
+      if (rank == 0) {
+        __syncthreads();
+        for (int r = 1; r < csize; ++r) {
+          Real* xr = reinterpret_cast<Real*>(cluster_map(reinterpret_cast<unsigned char*>(tv.xsep), r));
+          for (int j = threadIdx.x; j < tv.n_seps; j += blockDim.x) xr[j] = tv.xsep[j];
+        }
+      }
+    }
+    tile_sync();
     BC_TICK(1);
     // V update, mechanism states, next row, probes and next pulses
     const bool last = s + 1 == a.n_steps;
@@ -1933,7 +1984,7 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
         bad |= update_nodes<Real, W, false, kExtra>(a, tv, pulses, ctx, min(i0 + W * lane, tv.N - W),
                                                     i0 + W * lane < tv.N, i0, dt);
     if (bad) s_status = kStatusNonfinite;
-    __syncthreads();
+    tile_sync();
     if (kExtra && record && td.n_xprobes > 0) {
       // mechanism probes (plans with them run the extra variant): state views after the update
       const ProbeRef* pl = reinterpret_cast<const ProbeRef*>(reinterpret_cast<const unsigned char*>(tv.specs) +
@@ -2019,7 +2070,7 @@ __global__ void __launch_bounds__(kLaneThreads, sizeof(Real) == 4 ? 8 : 4) lane_
   const TileDesc td = a.tiles[blockIdx.x];
   unsigned char* base = a.blob + td.blob_offset;
   TileView<Real> tv;
-  tv.bind(td, base, a.scratch + td.scratch_offset, a.state);
+  tv.bind(td, base, a.scratch + td.scratch_offset, a.scratch + td.scratch_offset, base, a.state);
   const int L = blockDim.x, lane = threadIdx.x;
   const int n = reinterpret_cast<const int32_t*>(base + td.off_lane_n)[lane];
   const uint16_t* par = tv.crec;  // parent v of each node
@@ -2234,7 +2285,7 @@ __global__ void reset_kernel(LaunchArgs a, const double* vinit, const int64_t* v
   const TileDesc td = a.tiles[blockIdx.x];
   unsigned char* base = a.blob + td.blob_offset;
   TileView<Real> tv;
-  tv.bind(td, base, base, a.state);  // scratch unused
+  tv.bind(td, base, base, base, base, a.state);  // scratch unused
   const double* vi = vinit + vinit_off[blockIdx.x];
   for (int i = threadIdx.x; i < tv.n_real; i += blockDim.x) {
     const Real v = Real(vi[i]);
@@ -2274,16 +2325,66 @@ __global__ void view_kernel(unsigned char* blob, unsigned char* state, const int
 }
 
 // ------------------------------------------------------------------ launchers
+static void cluster_config(const LaunchArgs& a, int threads, size_t smem_bytes, cudaStream_t st, cudaLaunchConfig_t& cfg,
+                           cudaLaunchAttribute& attr) {
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = unsigned(a.cluster);
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(unsigned(a.n_tiles) * unsigned(a.cluster), 1, 1);
+  cfg.blockDim = dim3(unsigned(threads), 1, 1);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+}
+
 template <typename Real, bool kSmem, int kVar>
 static int launch_impl(const LaunchArgs& a, int threads, size_t smem_bytes, cudaStream_t st) {
   auto k = tile_step_kernel<Real, kSmem, kVar>;
-  if (kSmem) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
-    if (e != cudaSuccess) return int(e);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
+  if (e != cudaSuccess) return int(e);
+  if (!kSmem && a.cluster > 1) {
+    if (a.cluster > 8) {
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return int(e);
+    }
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    cluster_config(a, threads, smem_bytes, st, cfg, attr);
+    return int(cudaLaunchKernelEx(&cfg, k, a));
   }
-  dim3 grid(a.n_tiles, 1, 1);
-  k<<<grid, threads, kSmem ? smem_bytes : 0, st>>>(a);
+  k<<<a.n_tiles, threads, smem_bytes, st>>>(a);
   return int(cudaGetLastError());
+}
+
+// The largest power of two up to `want` at which `count` clusters are resident at once.
+template <typename Real, int kVar>
+static int usable_cluster(int want, int count, int threads, size_t smem_bytes) {
+  auto k = tile_step_kernel<Real, false, kVar>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes)) != cudaSuccess) return 1;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) want = std::min(want, 8);
+  for (int c = want; c > 1; c /= 2) {
+    LaunchArgs a{};
+    a.n_tiles = 1;
+    a.cluster = c;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    cluster_config(a, threads, smem_bytes, nullptr, cfg, attr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= count) return c;
+    (void)cudaGetLastError();
+  }
+  return 1;
+}
+
+int tile_cluster(int precision, int variant, int want, int count, int threads, size_t smem_bytes) {
+  if (variant > 1) return 1;
+  if (precision == BC_PREC_F64)
+    return variant ? usable_cluster<double, 1>(want, count, threads, smem_bytes)
+                   : usable_cluster<double, 0>(want, count, threads, smem_bytes);
+  return variant ? usable_cluster<float, 1>(want, count, threads, smem_bytes)
+                 : usable_cluster<float, 0>(want, count, threads, smem_bytes);
 }
 
 template <int kVar>
@@ -2318,14 +2419,12 @@ int launch_tiles(const LaunchArgs& a, int precision, bool smem, int threads, siz
 template <typename Real, bool kSmem, int kVar>
 static int node_impl(const LaunchArgs* a, int threads, size_t smem_bytes, cudaKernelNodeParams* np) {
   auto k = tile_step_kernel<Real, kSmem, kVar>;
-  if (kSmem) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
-    if (e != cudaSuccess) return int(e);
-  }
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
+  if (e != cudaSuccess) return int(e);
   np->func = reinterpret_cast<void*>(k);
   np->gridDim = dim3(a->n_tiles, 1, 1);
   np->blockDim = dim3(threads, 1, 1);
-  np->sharedMemBytes = kSmem ? unsigned(smem_bytes) : 0u;
+  np->sharedMemBytes = unsigned(smem_bytes);
   np->extra = nullptr;
   return 0;
 }

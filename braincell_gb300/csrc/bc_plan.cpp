@@ -56,6 +56,8 @@ struct CellSched;
 // launch classes: 0 packed shared-memory tiles, 1 one big cell per shared-memory
 // tile, 2 global-memory tiles, 3 lane tiles (one small cell per thread)
 constexpr int kMaxClasses = 4;
+// Shared memory that a global-memory tile may take for its separators: two CTAs to an SM.
+constexpr size_t kSepSmemLimit = 110 * 1024;
 // Longest unbranched run that one lane eliminates in one piece (lane_nodes).
 constexpr int kDefaultLaneNodes = 10;
 
@@ -124,6 +126,7 @@ struct LaunchClass {
   int first = 0, count = 0, threads = 256;
   bool smem = true;
   bool lane = false;  // lane tiles: one cell per thread (lane_step_kernel)
+  int cluster = 1;  // CTAs per tile (global-memory tiles)
   size_t smem_bytes = 0;
 };
 
@@ -363,11 +366,33 @@ static void order_whole(const LoweredCell& lc, CellSched& cs) {
   }
 }
 
-// Segments and separators of one cell.  Runs of more than lane_nodes nodes are cut:
-// a lane's walk costs about 60 cycles a node and a further separator level about
-// 190, so a run of L nodes is cut into about sqrt(L / 3.2) pieces (measured on the
-// 2,500-node tiles of the uneven population).  The cuts depend on the cell alone, so
-// its results do not depend on its tile mates or on the launch shape.
+// Levels of the separators, children before parents.
+static void set_levels(CellSched& cs) {
+  const int32_t ns = int32_t(cs.seps.size());
+  std::vector<int32_t> waits(ns, 0), ready;
+  for (Sep& sp : cs.seps) {
+    sp.level = 0;
+    if (sp.t >= 0) waits[sp.t]++;
+  }
+  for (int32_t j = 0; j < ns; ++j)
+    if (waits[j] == 0) ready.push_back(j);
+  cs.n_levels = 0;
+  for (size_t k = 0; k < ready.size(); ++k) {
+    const Sep& sp = cs.seps[ready[k]];
+    cs.n_levels = std::max(cs.n_levels, sp.level + 1);
+    if (sp.t < 0) continue;
+    cs.seps[sp.t].level = std::max(cs.seps[sp.t].level, sp.level + 1);
+    if (--waits[sp.t] == 0) ready.push_back(sp.t);
+  }
+}
+
+// Segments and separators of one cell.  Runs of more than lane_nodes nodes are cut.  A
+// lane's walk costs about 100 cycles a node, all runs at once; a further separator on a
+// run costs about 400 on every path through it, so with d branch levels a run of L nodes
+// is best cut into sqrt(L / (4 d)) pieces: long unbranched cells are cut, the 50-node
+// branches of a 20-level tree are not (256 such cells x 100 steps: 33.3 ms with every run
+// cut into sqrt(L / 3.2) pieces).  The cuts depend on the cell alone, so its
+// results do not depend on its tile mates or on the launch shape.
 static void decompose(const LoweredCell& lc, int lane_nodes, CellSched& cs) {
   const int32_t n = lc.n_node;
   if (n <= kCellLaneNodes) {
@@ -413,30 +438,40 @@ static void decompose(const LoweredCell& lc, int lane_nodes, CellSched& cs) {
   const int64_t room = std::max<int64_t>(0, 60000 - int64_t(cs.seps.size()));
   const int64_t most_per_run = std::max<int64_t>(1, 1 + room / std::max<int64_t>(1, int64_t(start.size())));
   const int64_t whole = std::min(std::max(lane_nodes, 1), 4096);
-  std::vector<int32_t> run;
-  for (const int32_t v0 : start) {
-    // the run from a leaf (itself the bottom node) or above a separator, up to the next separator
-    run.clear();
-    int32_t lower = sep_of[v0], v = lower >= 0 ? parent[v0] : v0;
-    for (; sep_of[v] < 0; v = parent[v]) run.push_back(v);
-    const int32_t upper = sep_of[v];
-    const int64_t L = int64_t(run.size());
+  // the run from a leaf (itself the bottom node) or above a separator, up to the next separator
+  struct Run {
+    int32_t lower, upper;
+    std::vector<int32_t> nodes;
+  };
+  std::vector<Run> runs(start.size());
+  for (size_t k = 0; k < start.size(); ++k) {
+    const int32_t v0 = start[k];
+    runs[k].lower = sep_of[v0];
+    int32_t v = runs[k].lower >= 0 ? parent[v0] : v0;
+    for (; sep_of[v] < 0; v = parent[v]) runs[k].nodes.push_back(v);
+    runs[k].upper = sep_of[v];
+    if (runs[k].lower >= 0) cs.seps[runs[k].lower].t = runs[k].upper;
+  }
+  set_levels(cs);
+  const double d = std::max(1, cs.n_levels);
+  for (const Run& run : runs) {
+    int32_t lower = run.lower;
+    const int64_t L = int64_t(run.nodes.size());
     int64_t pieces = 1;
-    if (L > whole) pieces = std::max<int64_t>(1, std::llround(std::sqrt(double(L) / 3.2)));
-    pieces = std::min({pieces, most_per_run, (L + 1) / 2});
-    pieces = std::max<int64_t>(pieces, 1);
+    if (L > whole) pieces = std::llround(std::sqrt(double(L) / (4.0 * d)));
+    pieces = std::max<int64_t>(1, std::min({pieces, most_per_run, (L + 1) / 2}));
     int64_t k0 = 0;
     for (int64_t q = 0; q < pieces; ++q) {
       // pieces - 1 of the L nodes become separators; the others are shared out evenly
       const int64_t k1 = k0 + (L - (pieces - 1)) * (q + 1) / pieces - (L - (pieces - 1)) * q / pieces;
       Seg sg;
-      sg.nodes.assign(run.begin() + k0, run.begin() + k1);
+      sg.nodes.assign(run.nodes.begin() + k0, run.nodes.begin() + k1);
       sg.s = lower;
       if (q + 1 < pieces) {
-        add_sep(run[k1]);
-        sg.t = sep_of[run[k1]];
+        add_sep(run.nodes[k1]);
+        sg.t = sep_of[run.nodes[k1]];
       } else {
-        sg.t = upper;
+        sg.t = run.upper;
       }
       if (sg.s >= 0) cs.seps[sg.s].t = sg.t;
       lower = sg.t;
@@ -445,20 +480,7 @@ static void decompose(const LoweredCell& lc, int lane_nodes, CellSched& cs) {
     }
   }
   for (size_t k = 0; k < cs.segs.size(); ++k) cs.seps[cs.segs[k].t].in.push_back(int32_t(k));
-  // levels, children before parents
-  const int32_t ns = int32_t(cs.seps.size());
-  std::vector<int32_t> waits(ns, 0), ready;
-  for (const Sep& sp : cs.seps)
-    if (sp.t >= 0) waits[sp.t]++;
-  for (int32_t j = 0; j < ns; ++j)
-    if (waits[j] == 0) ready.push_back(j);
-  for (size_t k = 0; k < ready.size(); ++k) {
-    const Sep& sp = cs.seps[ready[k]];
-    cs.n_levels = std::max(cs.n_levels, sp.level + 1);
-    if (sp.t < 0) continue;
-    cs.seps[sp.t].level = std::max(cs.seps[sp.t].level, sp.level + 1);
-    if (--waits[sp.t] == 0) ready.push_back(sp.t);
-  }
+  set_levels(cs);
 }
 
 // ------------------------------------------------------------------ tile building
@@ -692,8 +714,8 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     }
     // relative length of a step (it orders tiles): the walks of the dearest warp, the sweep, the update
     std::vector<int64_t> warp_cost(W, 0);
-    for (size_t k = 0; k < slots.size(); ++k) warp_cost[k % W] += 2 * slots[k].max_len;
-    crit = *std::max_element(warp_cost.begin(), warp_cost.end()) + 2 * n_levels + n_real / 32;
+    for (size_t k = 0; k < slots.size(); ++k) warp_cost[k % W] += slots[k].max_len;
+    crit = *std::max_element(warp_cost.begin(), warp_cost.end()) + 4 * n_levels + n_real / 32;
   }
   out.crit = crit;
   // lane tile: node v of the cell in lane l is tile node v * T + l
@@ -833,16 +855,8 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
   size_t so = 0;
   d.off_dr = int32_t(so);
   so = align16(so + 2 * N * rs);
-  d.off_inbox = int32_t(so);
-  so = align16(so + 2 * size_t(n_inbox) * rs);
-  d.off_srow = int32_t(so);
-  so = align16(so + 4 * seps.size() * rs);
-  d.off_own = int32_t(so);
-  so = align16(so + 2 * seps.size() * rs);
   d.off_q = int32_t(so);
   so = align16(so + size_t(n_lower) * rs);
-  d.off_xsep = int32_t(so);
-  so = align16(so + (seps.size() + kSepPad) * rs);
   d.off_wparams = int32_t(so);
   if (tb.cls == 2) so = align16(so + size_t(n_params) * cx.param_stride * rs);
   d.off_stamp = -1;
@@ -857,6 +871,21 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     d.off_pstage = int32_t(so);
     so = align16(so + size_t(kGruSmemBytes) + n_tile_ports * (sizeof(PortStage) + sizeof(PortLocal)));
   }
+  // the separators' work area
+  d.off_sep = int32_t(so);
+  size_t sw = 0;
+  d.off_inbox = int32_t(sw);
+  sw = align16(sw + 2 * size_t(n_inbox) * rs);
+  d.off_srow = int32_t(sw);
+  sw = align16(sw + 4 * seps.size() * rs);
+  d.off_own = int32_t(sw);
+  sw = align16(sw + 2 * seps.size() * rs);
+  d.off_xsep = int32_t(sw);
+  sw = align16(sw + (seps.size() + kSepPad) * rs);
+  d.sep_bytes = int32_t(sw);
+  so += sw;
+  // in shared memory for a global-memory tile whose CTAs still fit twice on an SM that way
+  d.sep_in_smem = tb.cls == 2 && n_tile_ports == 0 && sw + size_t(d.off_rows - d.off_seps) <= kSepSmemLimit;
   d.scratch_bytes = int32_t(so);
   d.n_nodes = int32_t(N);
   d.n_real_nodes = int32_t(n_real);
@@ -1139,6 +1168,7 @@ static LaunchArgs base_args(bc_plan* p) {
   a.spike_times = p->d_spike_times;
   a.status = p->d_status;
   a.state_slots = p->state_slots;
+  a.cluster = 1;
   a.timers = p->d_timers;
   a.syn_g = p->d_syn_g;
   a.syn_tau = p->d_syn_tau;
@@ -1317,6 +1347,7 @@ static bc_status enqueue_run(bc_plan* p, int64_t n_steps, double dt, void* strea
       }
       a.tiles = p->d_tiles + lcz.first;
       a.n_tiles = lcz.count;
+      a.cluster = lcz.cluster;
       int e = lcz.lane ? launch_lanes(a, p->precision, lcz.threads, p->extra, st)
                        : launch_tiles(a, p->precision, lcz.smem, lcz.threads, lcz.smem_bytes, kernel_variant(p), st);
       if (e) return fail(BC_ERR_CUDA, std::string("tile kernel launch: ") + cudaGetErrorString(cudaError_t(e)));
@@ -1692,13 +1723,24 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   const double bpn = 6.0 * double(rs) + 8.0 + (16.0 + 2.0 * double(rs)) / 6.4 + (20.0 + 9.0 * double(rs)) / 16.0 +
                      double(rs) / 3.0;
   int tile_nodes = opts.tile_nodes;
+  int n_sm = 152;
+  if (!dry && cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, opts.device) != cudaSuccess) n_sm = 152;
+  // 0 = auto: two tiles to an SM, so that a small population is spread over the whole GPU, up to the size that
+  // ran best on large ones (FP32; FP64 tiles take twice the shared memory).  A step's time is its tile's latency:
+  // 300 uneven cells ran 16.2 us a step in 900-node tiles; 16 cells of 129 nodes 6.6 us in three tiles.
+  const bool auto_shape = tile_nodes <= 0 && s.n_ports == 0;
+  if (auto_shape)
+    tile_nodes = int(std::min<int64_t>(std::max<int64_t>((p->n_nodes + 2 * n_sm - 1) / (2 * n_sm), 128),
+                                       opts.precision == BC_PREC_F64 ? 1250 : 2500));
   if (tile_nodes <= 0) tile_nodes = 900;
   tile_nodes = std::max(tile_nodes, 16);
   p->tile_nodes = tile_nodes;
   // Launch classes: 0 = packed shared-memory tiles (cells <= tile_nodes), 1 = one big
   // cell per shared-memory tile, 2 = global-memory tiles (too big for shared memory).
-  const int T_packed = opts.threads_per_tile > 0 ? opts.threads_per_tile : 128;
-  const int T_big = opts.threads_big > 0 ? opts.threads_big : 256;
+  // (a thread for every pair of nodes and a warp for the heavy ones, up to 512: two such tiles fill an SM's registers)
+  const int T_auto = auto_shape ? std::min(512, (tile_nodes / 2 + 31) / 32 * 32 + 32) : 128;
+  const int T_packed = opts.threads_per_tile > 0 ? opts.threads_per_tile : T_auto;
+  const int T_big = opts.threads_big > 0 ? opts.threads_big : (auto_shape ? 512 : 256);
   const int T_glob = opts.threads_global > 0 ? opts.threads_global : (s.n_ports > 0 ? BC_PORT_MAX_THREADS : 512);
   if (T_big % 32 || T_big > 1024 || T_glob % 32 || T_glob > 1024) {
     delete p;
@@ -1850,6 +1892,9 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
         tord.push_back(t);
         const size_t need = size_t(outs[t].desc.blob_bytes) + size_t(outs[t].desc.scratch_bytes);
         if (lcz.smem) lcz.smem_bytes = std::max(lcz.smem_bytes, need);
+        const TileDesc& d = outs[t].desc;
+        if (cl == 2 && d.sep_in_smem)
+          lcz.smem_bytes = std::max(lcz.smem_bytes, size_t(d.sep_bytes) + size_t(d.off_rows - d.off_seps));
       }
     if (opts.tile_order == 1) {
       // longest estimated step first: the block scheduler hands out CTAs in index
@@ -1860,6 +1905,15 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
       });
     }
     lcz.count = int(tord.size()) - lcz.first;
+    if (cl == 2 && lcz.count > 0 && !dry && s.n_ports == 0 && !p->use_graph) {
+      // few global-memory tiles: on each the largest cluster of CTAs at which they all run at once (one cell of
+      // 18,700 nodes: 127 us a step on one CTA, 41 on 16; 16 cells on clusters of 16, more than fit: 81)
+      bool seps_fit = true;
+      for (size_t t = 0; t < builds.size(); ++t) seps_fit = seps_fit && (builds[t].cls != 2 || outs[t].desc.sep_in_smem);
+      if (seps_fit && 2 * lcz.count <= 2 * n_sm)
+        lcz.cluster = tile_cluster(p->precision, p->extra ? BC_VARIANT_EXTRA : BC_VARIANT_LEAN, 16, lcz.count, lcz.threads,
+                                   lcz.smem_bytes);
+    }
     if (lcz.count > 0) p->classes.push_back(lcz);
   }
   p->n_smem_tiles = 0;

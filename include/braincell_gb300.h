@@ -394,9 +394,8 @@ typedef struct bc_plan_options {
   int32_t precision;        /* BC_PREC_*                                             */
   int32_t threads_per_tile; /* CTA size (multiple of 32, <= 1024); 0 = auto          */
   int32_t tile_nodes;       /* node budget per tile (shared-memory size); 0 = auto   */
-  int32_t lane_nodes;       /* unbranched runs of more nodes are cut into about
-                               sqrt(nodes / 3.2) pieces, each walked by one lane;
-                               0 = auto (10)                                         */
+  int32_t lane_nodes;       /* unbranched runs of more nodes may be cut into pieces,
+                               each walked by one lane; 0 = auto (10)                */
   int32_t steps_per_launch; /* time steps fused per kernel launch; 0 = auto          */
   int32_t record_every;     /* probe sampling period in steps (>= 1)                 */
   int32_t max_spikes;       /* spike times kept per probe                            */

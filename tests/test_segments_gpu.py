@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from braincell_gb300 import Branch, Cell, Morphology
+from braincell_gb300 import workloads as W
 from braincell_gb300.batch import concat_batches, lower_cell
 from braincell_gb300.mech import AllRegion, CableProperty, Channel, CurrentClamp, CVPerBranchList, RootLocation, StateProbe
 from braincell_gb300.runtime import Plan
@@ -57,3 +58,21 @@ def test_segment_shapes_match_the_oracle(native_lib, cuda_device, precision, tol
         assert np.abs(got - oc.V[0]).max() <= tol, name
         off += oc.V.shape[1]
     assert off == V.size
+
+
+@pytest.mark.parametrize("n_cells", [1, 3, 20])
+@pytest.mark.parametrize("precision", ["f32", "f64"])
+def test_clusters_do_not_change_a_global_memory_cell(native_lib, cuda_device, n_cells, precision):
+    # cells too large for shared memory run on clusters of CTAs when they are few; a CUDA-graph
+    # plan runs the same tiles on one CTA each: bit-identical
+    descs = W.large(n_cells, n_range=(6000, 6400), n_branches=60, n_pulses=40, duration=4.0)
+    out = []
+    for use_graph in (False, True):
+        p = Plan(W.descs_to_batch(descs), precision=precision, record_every=4, use_graph=use_graph, device=cuda_device)
+        assert (p.tile_stats()[:, 4] == 2).any()
+        for n in (60, 1, 39):
+            p.run(n, DT)
+        out.append((p.state("V"), p.state("Ci"), p.traces()))
+        p.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
