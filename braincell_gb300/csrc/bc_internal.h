@@ -365,10 +365,20 @@ int lane_node_params(const LaunchArgs* a, int precision, int threads, bool extra
                      const LaunchArgs** hold);
 int launch_reset_impl(const LaunchArgs& a, int precision, int threads, const double* vinit, const int64_t* voff,
                       void* stream);
-// View offsets: byte offsets into the blob, or kStateTag + byte offset into the state array.
-constexpr int64_t kStateTag = int64_t(1) << 62;
-int launch_view_impl(unsigned char* blob, unsigned char* state, int precision, const int64_t* off_hi,
-                     const int64_t* off_lo, double* view, int64_t n, bool write, void* stream);
+// One state view: slot of its high word in the state array (-1: the voltage, in the blob)
+// and of its low word (-1: none), and the mechanism bits that own it (region_bits layout;
+// 0: every CV has it).  kViewSpike tests V_last < v_th <= V instead.
+enum : int32_t { kViewRead = 0, kViewWrite = 1, kViewSpike = 2 };
+struct ViewArgs {
+  int32_t mode, slot, slot_lo;
+  uint64_t owner;
+  double v_th;
+};
+// cv: (tile, node) of every CV.
+int launch_view_impl(const TileDesc* tiles, unsigned char* blob, unsigned char* state, int precision, const int2* cv,
+                     const ViewArgs& va, double* view, int64_t n, void* stream);
+int launch_pulse_amp_impl(PulseRec* pulses, const int32_t* src, const double* scale, const double* amp, int64_t n,
+                          void* stream);
 // Event delivery after a launch: every spike record in [*rec_done, *rec_count)
 // adds the weights of its source cell's connections into the arrival ring.
 int launch_deliver_impl(int precision, const int32_t* rec_cell, const int64_t* rec_step,
@@ -376,8 +386,7 @@ int launch_deliver_impl(int precision, const int32_t* rec_cell, const int64_t* r
                         const int64_t* out_ptr, const int64_t* out_syn, const void* out_w, const int32_t* out_d,
                         void* arrivals, int64_t arr_slots, int64_t n_syn, void* stream);
 // Device address (on the current device) of the fixed scratch behind
-// bc_state_download_noalloc: [hi offsets | lo offsets | values], BC_NOALLOC_MAX_CV
-// 8-byte entries each.  Returns the cudaError_t of cudaGetSymbolAddress.
+// bc_state_download_noalloc: BC_NOALLOC_MAX_CV 8-byte values.  Returns the cudaError_t of cudaGetSymbolAddress.
 int noalloc_view_scratch_address(void** out);
 
 }  // namespace bc

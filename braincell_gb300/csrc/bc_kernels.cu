@@ -2299,29 +2299,63 @@ __global__ void reset_kernel(LaunchArgs a, const double* vinit, const int64_t* v
   }
 }
 
-// Gather (write = false) or scatter (write = true) one named view.
-__device__ __forceinline__ unsigned char* view_addr(unsigned char* blob, unsigned char* state, int64_t off) {
-  return off >= kStateTag ? state + (off - kStateTag) : blob + off;
-}
-
+// Reads, writes or tests one named view of every CV, in the reference's CV order
+// (view_args): the addresses come from the plan's CV map and tile descriptors, so that a
+// call uploads nothing and allocates nothing (tables of byte offsets, built on the host
+// and copied on every call, took 24 ms for 5.8 million CVs).
 template <typename Real>
-__global__ void view_kernel(unsigned char* blob, unsigned char* state, const int64_t* off_hi, const int64_t* off_lo,
-                            double* view, int64_t n, bool write) {
+__global__ void view_kernel(const TileDesc* tiles, unsigned char* blob, Real* state, const int2* cv, ViewArgs va,
+                            double* view, int64_t n) {
   for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t oh = off_hi[k], ol = off_lo[k];
-    if (oh < 0) {
-      if (!write) view[k] = __longlong_as_double(0x7ff8000000000000LL);
+    const int2 c = cv[k];
+    const TileDesc& d = tiles[c.x];
+    const unsigned char* base = blob + d.blob_offset;
+    Pair<Real>& v = reinterpret_cast<Pair<Real>*>(blob + d.blob_offset + d.off_v)[c.y];
+    Real* st = state + d.state_offset + c.y;
+    const int64_t N = d.n_nodes;
+    if (va.mode == kViewSpike) {
+      const double last = double(st[kSlotVLastHi * N]) + double(st[kSlotVLastLo * N]), now = double(v.x) + double(v.y);
+      view[k] = last < va.v_th && now >= va.v_th ? 1.0 : 0.0;
       continue;
     }
-    Real* hi = reinterpret_cast<Real*>(view_addr(blob, state, oh));
-    Real* lo = ol >= 0 ? reinterpret_cast<Real*>(view_addr(blob, state, ol)) : nullptr;
-    if (write) {
-      *hi = Real(view[k]);
-      if (lo) *lo = Real(view[k] - double(*hi));
+    bool present = true;
+    if (va.owner != 0) {
+      const uint16_t pr = reinterpret_cast<const uint16_t*>(base + d.off_pidx)[c.y];
+      present = pr != kBoundary;
+      if (present) {
+        const uint32_t m = reinterpret_cast<const uint32_t*>(base + d.off_mech)[pr];
+        uint64_t bits = m;
+        if (m & BC_M_EXT)
+          bits |= uint64_t(ext_mask(reinterpret_cast<const Real*>(base + d.off_params) + size_t(pr) * d.param_stride))
+                  << 32;
+        present = (bits & va.owner) != 0;
+      }
+    }
+    if (!present) {
+      if (va.mode == kViewRead) view[k] = __longlong_as_double(0x7ff8000000000000LL);
+      continue;
+    }
+    Real* hi = va.slot < 0 ? &v.x : st + va.slot * N;
+    Real* lo = va.slot < 0 ? &v.y : (va.slot_lo >= 0 ? st + va.slot_lo * N : nullptr);
+    if (va.mode == kViewWrite) {
+      const double x = view[k];
+      *hi = Real(x);
+      if (lo) *lo = Real(x - double(*hi));
+      if (va.slot < 0) {  // a new voltage starts a fresh history: no step has crossed anything since
+        st[kSlotVLastHi * N] = *hi;
+        st[kSlotVLastLo * N] = *lo;
+      }
     } else {
       view[k] = double(*hi) + (lo ? double(*lo) : 0.0);
     }
   }
+}
+
+// New amplitudes (nA, batch order) into the pulse records.
+__global__ void pulse_amp_kernel(PulseRec* pulses, const int32_t* src, const double* scale, const double* amp,
+                                 int64_t n) {
+  for (int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x)
+    pulses[k].amp = amp[src[k]] * scale[k];
 }
 
 // ------------------------------------------------------------------ launchers
@@ -2510,22 +2544,32 @@ int launch_reset_impl(const LaunchArgs& a, int precision, int threads, const dou
   return int(cudaGetLastError());
 }
 
-int launch_view_impl(unsigned char* blob, unsigned char* state, int precision, const int64_t* off_hi,
-                     const int64_t* off_lo, double* view, int64_t n, bool write, void* stream) {
+static int grid_for(int64_t n, int threads) { return int(std::min<int64_t>((n + threads - 1) / threads, 65535)); }
+
+int launch_view_impl(const TileDesc* tiles, unsigned char* blob, unsigned char* state, int precision, const int2* cv,
+                     const ViewArgs& va, double* view, int64_t n, void* stream) {
   if (n <= 0) return 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int threads = 256;
-  const int64_t blocks = std::min<int64_t>((n + threads - 1) / threads, 65535);
   if (precision == BC_PREC_F64)
-    view_kernel<double><<<int(blocks), threads, 0, st>>>(blob, state, off_hi, off_lo, view, n, write);
+    view_kernel<double><<<grid_for(n, threads), threads, 0, st>>>(tiles, blob, reinterpret_cast<double*>(state), cv, va,
+                                                                  view, n);
   else
-    view_kernel<float><<<int(blocks), threads, 0, st>>>(blob, state, off_hi, off_lo, view, n, write);
+    view_kernel<float><<<grid_for(n, threads), threads, 0, st>>>(tiles, blob, reinterpret_cast<float*>(state), cv, va,
+                                                                 view, n);
+  return int(cudaGetLastError());
+}
+
+int launch_pulse_amp_impl(PulseRec* pulses, const int32_t* src, const double* scale, const double* amp, int64_t n,
+                          void* stream) {
+  if (n <= 0) return 0;
+  pulse_amp_kernel<<<grid_for(n, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(pulses, src, scale, amp, n);
   return int(cudaGetLastError());
 }
 
 // Scratch of bc_state_download_noalloc, part of the module image (no allocation
-// call): three 8-byte arrays of BC_NOALLOC_MAX_CV entries, 256-byte aligned.
-static __device__ __align__(256) unsigned char g_noalloc_view_scratch[3 * 8 * size_t(BC_NOALLOC_MAX_CV)];
+// call): BC_NOALLOC_MAX_CV values.
+static __device__ __align__(256) unsigned char g_noalloc_view_scratch[8 * size_t(BC_NOALLOC_MAX_CV)];
 
 int noalloc_view_scratch_address(void** out) {
   return int(cudaGetSymbolAddress(out, g_noalloc_view_scratch));

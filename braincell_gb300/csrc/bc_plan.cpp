@@ -151,11 +151,18 @@ struct bc_plan {
   int n_smem_tiles = 0;
   size_t smem_bytes = 0;
   std::vector<int64_t> cell_ncv;
-  std::vector<int32_t> cv_tile, cv_node;
-  std::vector<uint64_t> cv_mech;  // region bits, extension channels' BC_X_* bits in the high word
+  // (tile, node) of every CV, and room for one view's values; a call holds the mutex until
+  // its values have left the device, as several threads may read one plan
+  int2* d_cv = nullptr;
+  double* d_view = nullptr;
+  std::mutex view_mu;
   std::vector<bc::PulseRec> pulses;
   std::vector<int64_t> pulse_src;   // spec pulse id of each record (records are in tile / node order)
   std::vector<double> pulse_scale;  // record amp per nA
+  std::vector<double> pulse_amp;    // bc_pulse_set_amp's last amplitudes (nA); the host records follow when next used
+  int32_t* d_pulse_src = nullptr;
+  double* d_pulse_scale = nullptr;
+  double* d_pulse_amp = nullptr;
   double pulses_dt = -1.0;
   std::vector<double> probe_vrest;
   // synapses and connections (host copies; device mirrors below)
@@ -243,6 +250,11 @@ static void free_plan(bc_plan* p) {
   cudaFree(p->d_state);
   cudaFree(p->d_tiles);
   cudaFree(p->d_pulses);
+  cudaFree(p->d_pulse_src);
+  cudaFree(p->d_pulse_scale);
+  cudaFree(p->d_pulse_amp);
+  cudaFree(p->d_cv);
+  cudaFree(p->d_view);
   cudaFree(p->d_vinit);
   cudaFree(p->d_vinit_off);
   cudaFree(p->d_traces);
@@ -499,7 +511,6 @@ struct TileOut {
   std::vector<PortRec> ports;         // stim_begin / stim_end relative to port_pulses
   std::vector<PulseRec> port_pulses;  // amp in nA
   std::vector<std::pair<int64_t, int32_t>> cv_local;  // (global cv id, local node)
-  std::vector<uint64_t> cv_mech;
   int64_t crit = 0;
 };
 
@@ -951,7 +962,6 @@ static bc_status build_tile(const BuildCtx& cx, const TileBuild& tb, int T, Tile
     for (int32_t k = 0; k < lc.n_cv; ++k) {
       const int32_t v = lc.cv_node[k];
       out.cv_local.push_back({base + k, node_tile[li][v]});
-      out.cv_mech.push_back(region_bits(s, c * R + lc.region[v]));
     }
   }
   // special records: pulses in node order, probe ids
@@ -1117,6 +1127,8 @@ static bc_status update_pulses(bc_plan* p, double dt, void* stream) {
     p->port_pulses_dt = dt;
   }
   if (p->pulses.empty() || p->pulses_dt == dt) return BC_OK;
+  if (!p->pulse_amp.empty())
+    for (size_t k = 0; k < p->pulses.size(); ++k) p->pulses[k].amp = p->pulse_amp[p->pulse_src[k]] * p->pulse_scale[k];
   for (auto& pr : p->pulses) {
     pr.on_step = first_step_at(pr.t_on, dt);
     pr.off_step = first_step_at(pr.t_off, dt);
@@ -1924,9 +1936,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   int64_t state_total = 0;
   std::vector<int64_t> vinit_off;
   p->tiles.clear();
-  p->cv_tile.assign(p->n_cv, -1);
-  p->cv_node.assign(p->n_cv, -1);
-  p->cv_mech.assign(p->n_cv, 0);
+  std::vector<int2> cv_map(p->n_cv);
   for (size_t k = 0; k < tord.size(); ++k) {
     TileOut& to = outs[tord[k]];
     TileDesc d = to.desc;
@@ -1956,9 +1966,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     vinit_off.push_back(int64_t(vinit_total));
     vinit_total += to.vinit.size();
     for (size_t q = 0; q < to.cv_local.size(); ++q) {
-      p->cv_tile[to.cv_local[q].first] = int32_t(k);
-      p->cv_node[to.cv_local[q].first] = to.cv_local[q].second;
-      p->cv_mech[to.cv_local[q].first] = to.cv_mech[q];
+      cv_map[to.cv_local[q].first] = make_int2(int(k), to.cv_local[q].second);
     }
     p->max_phases = std::max<int64_t>(p->max_phases, d.n_phases);
     p->max_chain_nodes = std::max<int64_t>(p->max_chain_nodes, to.crit);
@@ -2018,6 +2026,17 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   BC_TRY(dalloc(p, &p->d_timers, 4));
   BC_TRYC(cudaMemset(p->d_timers, 0, 4 * sizeof(unsigned long long)));
   BC_TRYC(cudaMemcpy(p->d_blob, blob.data(), blob_total, cudaMemcpyHostToDevice));
+  BC_TRY(dalloc(p, &p->d_cv, size_t(p->n_cv)));
+  BC_TRY(dalloc(p, &p->d_view, size_t(p->n_cv)));
+  BC_TRYC(cudaMemcpy(p->d_cv, cv_map.data(), cv_map.size() * sizeof(int2), cudaMemcpyHostToDevice));
+  if (!p->pulses.empty()) {
+    const std::vector<int32_t> src(p->pulse_src.begin(), p->pulse_src.end());
+    BC_TRY(dalloc(p, &p->d_pulse_src, src.size()));
+    BC_TRY(dalloc(p, &p->d_pulse_scale, src.size()));
+    BC_TRY(dalloc(p, &p->d_pulse_amp, size_t(p->n_pulses)));
+    BC_TRYC(cudaMemcpy(p->d_pulse_src, src.data(), src.size() * 4, cudaMemcpyHostToDevice));
+    BC_TRYC(cudaMemcpy(p->d_pulse_scale, p->pulse_scale.data(), src.size() * 8, cudaMemcpyHostToDevice));
+  }
   BC_TRYC(cudaMemcpy(p->d_tiles, p->tiles.data(), p->tiles.size() * sizeof(TileDesc), cudaMemcpyHostToDevice));
   BC_TRYC(cudaMemcpy(p->d_vinit, vinit.data(), vinit.size() * sizeof(double), cudaMemcpyHostToDevice));
   BC_TRYC(cudaMemcpy(p->d_vinit_off, vinit_off.data(), vinit_off.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
@@ -2340,73 +2359,56 @@ bc_status bc_run_timed(bc_plan_t p, int64_t n_steps, double dt, void* stream, do
   return bc_check(p, stream);
 }
 
-static bc_status view_offsets(bc_plan* p, int32_t which, std::vector<int64_t>& hi, std::vector<int64_t>& lo) {
+static bc_status view_args(int32_t which, int32_t mode, ViewArgs* va) {
   if (which < 0 || which >= BC_NSTATE_VIEW) return fail(BC_ERR_INVALID, "unknown state view");
-  hi.assign(p->n_cv, -1);
-  lo.assign(p->n_cv, -1);
-  const size_t rs = p->real_size;
-  for (int64_t k = 0; k < p->n_cv; ++k) {
-    const TileDesc& d = p->tiles[p->cv_tile[k]];
-    const int64_t j = p->cv_node[k];
-    const int64_t base = d.blob_offset;
-    if (which == BC_STATE_V) {
-      hi[k] = base + d.off_v + 2 * j * rs;
-      lo[k] = hi[k] + rs;
-      continue;
-    }
-    uint64_t bit = 0;
-    int slot = -1;
-    state_view(which, &bit, &slot);
-    if (which != BC_STATE_V_LAST && !(p->cv_mech[k] & bit)) slot = -1;
-    const bool has_lo = which == BC_STATE_CA_CI || which == BC_STATE_V_LAST;
-    if (slot < 0) continue;
-    // states live in the separate state array: offsets are tagged by +state_tag
-    const int lo_slot = which == BC_STATE_V_LAST ? kSlotVLastLo : kSlotCaLo;
-    hi[k] = kStateTag + (d.state_offset + int64_t(slot) * d.n_nodes + j) * int64_t(rs);
-    if (has_lo) lo[k] = kStateTag + (d.state_offset + int64_t(lo_slot) * d.n_nodes + j) * int64_t(rs);
+  *va = ViewArgs{mode, -1, -1, 0, 0.0};
+  if (which == BC_STATE_V) return BC_OK;
+  uint64_t bit = 0;
+  int slot = -1;
+  state_view(which, &bit, &slot);
+  va->slot = slot;
+  if (which == BC_STATE_V_LAST) {
+    va->slot_lo = kSlotVLastLo;
+  } else {
+    va->owner = bit;
+    if (which == BC_STATE_CA_CI) va->slot_lo = kSlotCaLo;
   }
   return BC_OK;
 }
 
-static bc_status view_io(bc_plan* p, int32_t which, double* host, bool write, void* stream) {
-  if (!p || !host) return fail(BC_ERR_INVALID, "null argument");
-  BC_NEED_DEVICE(p);
+static bc_status view_io(bc_plan* p, const ViewArgs& va, double* host, void* stream) {
   BC_CUDA(cudaSetDevice(p->device));
-  std::vector<int64_t> hi, lo;
-  bc_status st = view_offsets(p, which, hi, lo);
-  if (st != BC_OK) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const size_t n = size_t(p->n_cv);
-  int64_t *dhi = nullptr, *dlo = nullptr;
-  double* dv = nullptr;
-  BC_CUDA(cudaMalloc(reinterpret_cast<void**>(&dhi), n * 8));
-  BC_CUDA(cudaMalloc(reinterpret_cast<void**>(&dlo), n * 8));
-  BC_CUDA(cudaMalloc(reinterpret_cast<void**>(&dv), n * 8));
-  cudaError_t e = cudaMemcpyAsync(dhi, hi.data(), n * 8, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(dlo, lo.data(), n * 8, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess && write) e = cudaMemcpyAsync(dv, host, n * 8, cudaMemcpyHostToDevice, s);
+  const size_t bytes = size_t(p->n_cv) * 8;
+  std::lock_guard<std::mutex> lock(p->view_mu);
+  cudaError_t e = cudaSuccess;
+  if (va.mode == kViewWrite) e = cudaMemcpyAsync(p->d_view, host, bytes, cudaMemcpyHostToDevice, s);
   int ke = 0;
   if (e == cudaSuccess)
-    ke = launch_view_impl(p->d_blob, p->d_state, p->precision, dhi, dlo, dv, int64_t(n), write, stream);
-  if (e == cudaSuccess && !ke && !write) e = cudaMemcpyAsync(host, dv, n * 8, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  cudaFree(dhi);
-  cudaFree(dlo);
-  cudaFree(dv);
+    ke = launch_view_impl(p->d_tiles, p->d_blob, p->d_state, p->precision, p->d_cv, va, p->d_view, p->n_cv, stream);
+  if (e == cudaSuccess && !ke && va.mode != kViewWrite)
+    e = cudaMemcpyAsync(host, p->d_view, bytes, cudaMemcpyDeviceToHost, s);
+  const cudaError_t es = cudaStreamSynchronize(s);  // also after a failure: nothing of this call outlives the lock
   if (ke) return fail(BC_ERR_CUDA, std::string("view kernel: ") + cudaGetErrorString(cudaError_t(ke)));
+  if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return fail(BC_ERR_CUDA, std::string("state view: ") + cudaGetErrorString(e));
   return BC_OK;
 }
 
+static bc_status view_call(bc_plan* p, int32_t which, int32_t mode, double* host, void* stream) {
+  if (!p || !host) return fail(BC_ERR_INVALID, "null argument");
+  BC_NEED_DEVICE(p);
+  ViewArgs va;
+  const bc_status st = view_args(which, mode, &va);
+  return st == BC_OK ? view_io(p, va, host, stream) : st;
+}
+
 bc_status bc_state_download(bc_plan_t p, int32_t which, double* out, void* stream) {
-  return view_io(p, which, out, false, stream);
+  return view_call(p, which, kViewRead, out, stream);
 }
 
 bc_status bc_state_upload(bc_plan_t p, int32_t which, const double* in, void* stream) {
-  bc_status st = view_io(p, which, const_cast<double*>(in), true, stream);
-  // a new voltage starts a fresh history: no step has crossed anything since
-  if (st == BC_OK && which == BC_STATE_V) st = view_io(p, BC_STATE_V_LAST, const_cast<double*>(in), true, stream);
-  return st;
+  return view_call(p, which, kViewWrite, const_cast<double*>(in), stream);
 }
 
 bc_status bc_pulse_set_amp(bc_plan_t p, const double* amp_nA, void* stream) {
@@ -2416,29 +2418,23 @@ bc_status bc_pulse_set_amp(bc_plan_t p, const double* amp_nA, void* stream) {
   BC_CUDA(cudaSetDevice(p->device));
   for (int64_t q = 0; q < p->n_pulses; ++q)
     if (!std::isfinite(amp_nA[q])) return fail(BC_ERR_INVALID, "bc_pulse_set_amp: non-finite amplitude");
-  for (size_t k = 0; k < p->pulses.size(); ++k) p->pulses[k].amp = amp_nA[p->pulse_src[k]] * p->pulse_scale[k];
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // the records also carry the step bounds of the last dt; pageable source: wait
-  BC_CUDA(cudaMemcpyAsync(p->d_pulses, p->pulses.data(), p->pulses.size() * sizeof(PulseRec), cudaMemcpyHostToDevice,
-                          st));
+  p->pulse_amp.assign(amp_nA, amp_nA + p->n_pulses);
+  BC_CUDA(cudaMemcpyAsync(p->d_pulse_amp, p->pulse_amp.data(), p->pulse_amp.size() * 8, cudaMemcpyHostToDevice, st));
+  const int ke = launch_pulse_amp_impl(p->d_pulses, p->d_pulse_src, p->d_pulse_scale, p->d_pulse_amp,
+                                       int64_t(p->pulses.size()), stream);
+  if (ke) return fail(BC_ERR_CUDA, std::string("pulse amplitude kernel: ") + cudaGetErrorString(cudaError_t(ke)));
   BC_CUDA(cudaStreamSynchronize(st));
   return BC_OK;
 }
 
 bc_status bc_spike_state_download(bc_plan_t p, double v_th, double* out, void* stream) {
   if (!p || !out) return fail(BC_ERR_INVALID, "null argument");
-  std::vector<double> last(size_t(p->n_cv));
-  bc_status st = view_io(p, BC_STATE_V, out, false, stream);
-  if (st == BC_OK && p->n_cv > 0) st = view_io(p, BC_STATE_V_LAST, last.data(), false, stream);
-  if (st != BC_OK) return st;
-  for (int64_t k = 0; k < p->n_cv; ++k) out[k] = (last[size_t(k)] < v_th && out[k] >= v_th) ? 1.0 : 0.0;
-  return BC_OK;
+  BC_NEED_DEVICE(p);
+  return view_io(p, ViewArgs{kViewSpike, -1, -1, 0, v_th}, out, stream);
 }
 
 // ------------------------------------------------------------------ no-allocation download
-// Host staging of the offset tables, [hi | lo] with BC_NOALLOC_MAX_CV entries each
-// (zero-initialised static storage; nothing is allocated at run time).
-static int64_t g_noalloc_host_off[2 * size_t(BC_NOALLOC_MAX_CV)];
 constexpr int kNoAllocDevices = 64;
 static unsigned char* g_noalloc_scratch[kNoAllocDevices];
 static std::mutex g_noalloc_setup_mu;
@@ -2457,27 +2453,6 @@ static bc_status noalloc_scratch(int device, unsigned char** out) {
   }
   *out = g_noalloc_scratch[device];
   return BC_OK;
-}
-
-// Offsets of CV k in view `which`: the per-CV form of view_offsets.
-static void noalloc_offset(const bc_plan* p, int32_t which, int64_t k, int64_t* hi, int64_t* lo) {
-  const TileDesc& d = p->tiles[p->cv_tile[k]];
-  const int64_t j = p->cv_node[k];
-  const int64_t rs = int64_t(p->real_size);
-  *hi = -1;
-  *lo = -1;
-  if (which == BC_STATE_V) {
-    *hi = d.blob_offset + d.off_v + 2 * j * rs;
-    *lo = *hi + rs;
-    return;
-  }
-  uint64_t bit = 0;
-  int slot = -1;
-  state_view(which, &bit, &slot);
-  if (which != BC_STATE_V_LAST && !(p->cv_mech[k] & bit)) return;
-  *hi = kStateTag + (d.state_offset + int64_t(slot) * d.n_nodes + j) * rs;
-  if (which == BC_STATE_CA_CI) *lo = kStateTag + (d.state_offset + int64_t(kSlotCaLo) * d.n_nodes + j) * rs;
-  if (which == BC_STATE_V_LAST) *lo = kStateTag + (d.state_offset + int64_t(kSlotVLastLo) * d.n_nodes + j) * rs;
 }
 
 bc_status bc_state_download_noalloc(bc_plan_t p, int32_t which, double* out, void* stream) {
@@ -2502,15 +2477,11 @@ bc_status bc_state_download_noalloc(bc_plan_t p, int32_t which, double* out, voi
   if (st != BC_OK) return st;
   const int64_t n = p->n_cv;
   if (n == 0) return BC_OK;
-  int64_t* h_hi = g_noalloc_host_off;
-  int64_t* h_lo = g_noalloc_host_off + BC_NOALLOC_MAX_CV;
-  for (int64_t k = 0; k < n; ++k) noalloc_offset(p, which, k, &h_hi[k], &h_lo[k]);
-  // Entries [0, n) of all three arrays are written before they are read (offsets by
-  // the copies, values by the view kernel, which fills absent states with NaN), so
-  // nothing has to start at zero.
-  int64_t* d_hi = reinterpret_cast<int64_t*>(scratch);
-  int64_t* d_lo = d_hi + BC_NOALLOC_MAX_CV;
-  double* d_val = reinterpret_cast<double*>(d_lo + BC_NOALLOC_MAX_CV);
+  ViewArgs va;
+  st = view_args(which, kViewRead, &va);
+  if (st != BC_OK) return st;
+  // entries [0, n) are written by the view kernel (NaN for absent states) before they are read
+  double* d_val = reinterpret_cast<double*>(scratch);
   // Once something is enqueued, every return waits for the stream first, so that
   // no copy or kernel of this call still uses the shared scratch when the next,
   // serialised call (perhaps on another stream) writes it.
@@ -2518,13 +2489,9 @@ bc_status bc_state_download_noalloc(bc_plan_t p, int32_t which, double* out, voi
     (void)cudaStreamSynchronize(s);
     return fail(BC_ERR_CUDA, what + ": " + cudaGetErrorString(e));
   };
-  cudaError_t e = cudaMemcpyAsync(d_hi, h_hi, size_t(n) * 8, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return failed("offset upload", e);
-  e = cudaMemcpyAsync(d_lo, h_lo, size_t(n) * 8, cudaMemcpyHostToDevice, s);
-  if (e != cudaSuccess) return failed("offset upload", e);
-  const int ke = launch_view_impl(p->d_blob, p->d_state, p->precision, d_hi, d_lo, d_val, n, false, stream);
+  const int ke = launch_view_impl(p->d_tiles, p->d_blob, p->d_state, p->precision, p->d_cv, va, d_val, n, stream);
   if (ke) return failed("view kernel", cudaError_t(ke));
-  e = cudaMemcpyAsync(out, d_val, size_t(n) * 8, cudaMemcpyDeviceToHost, s);
+  cudaError_t e = cudaMemcpyAsync(out, d_val, size_t(n) * 8, cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return failed("value download", e);
   e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return fail(BC_ERR_CUDA, std::string("cudaStreamSynchronize: ") + cudaGetErrorString(e));
