@@ -91,25 +91,6 @@ __device__ __forceinline__ void xblock_frag(const float* xa, const float* xb, in
   a[3] = a[2];
 }
 
-// Pre-activations of N group jb (units 8 jb .. 8 jb + 7) for one M tile:
-// acc[0] r, acc[1] z, acc[2] hn, acc[3] nx.  ah: A fragments of h~ (4 k steps),
-// ax: the x block.  wext: BF16 pairs, row-major [4H][kGruK] (rows r, z, hn, nx).
-__device__ __forceinline__ void gru_preact(const uint32_t* __restrict__ wext, int jb, int g, int tq,
-                                           const uint32_t (*ah)[4], const uint32_t* ax, float (*acc)[4]) {
-  constexpr int kRow = kGruK / 2;  // uint32 per row
-#pragma unroll
-  for (int q = 0; q < 4; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0f;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const uint32_t* w = wext + size_t(q * kGruH + jb * 8 + g) * kRow;
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) mma_bf16_16816(acc[q], ah[kk], __ldg(w + kk * 8 + tq), __ldg(w + kk * 8 + 4 + tq));
-    mma_bf16_16816(acc[q], ax, __ldg(w + 32 + tq), __ldg(w + 36 + tq));
-  }
-  const uint32_t* w = wext + size_t(3 * kGruH + jb * 8 + g) * kRow;
-  mma_bf16_16816(acc[3], ax, __ldg(w + 32 + tq), __ldg(w + 36 + tq));
-}
-
 // Copy the row-major extended matrix into the fragment-major layout of a tile's
 // scratch (kGruFragPairs word pairs; see kGruFragSlots).
 __device__ __forceinline__ void gru_frag_fill(const uint32_t* __restrict__ wext, uint2* frag, int tid, int T) {
@@ -122,9 +103,10 @@ __device__ __forceinline__ void gru_frag_fill(const uint32_t* __restrict__ wext,
   }
 }
 
-// gru_preact with the B fragments of N group jb taken from the fragment-major
-// copy (frag = the tile's copy + jb * 16 slots * 32 lanes): the same products
-// in the same order, so the same results.
+// Pre-activations of N group jb (units 8 jb .. 8 jb + 7) for one M tile: acc[0] r,
+// acc[1] z, acc[2] hn, acc[3] nx.  ah: A fragments of h~ (4 k steps), ax: the x block,
+// frag: the tile's fragment-major copy + jb * 16 slots * 32 lanes.  Training runs the
+// same products in the same order.
 __device__ __forceinline__ void gru_preact_frag(const uint2* frag, int lane, const uint32_t (*ah)[4],
                                                 const uint32_t* ax, float (*acc)[4]) {
 #pragma unroll
