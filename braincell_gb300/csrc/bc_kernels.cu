@@ -742,7 +742,9 @@ __device__ __noinline__ void extra_channels(Real* st, int N, const Real* P, uint
 // are replaced by what the step needs (kDer), once per launch, in the records' shared-
 // memory copy or in a copy in the tile's scratch:
 //   PHI entries -> -dt phi;  CA_TAU -> c = 1 - exp(-dt / tau);  CA_D -> the shell's gain
-//   c tau 10 / (2 F d), so that the calcium step is Ci += max(gain ICa, 0) + c (C_rest - Ci).
+//   c tau 10 / (2 F d), so that the calcium step is Ci += max(gain ICa, 0) + c (C_rest - Ci);
+//   E_Ca of a dynamic ion, which nothing reads -> slope ln C_out, so that its Nernst
+//   potential is that minus slope ln Ci: no division beside the logarithm.
 template <typename Real>
 __device__ __forceinline__ Real launch_param(const Real* P, uint32_t m, int k, Real dt) {
   switch (k) {
@@ -759,6 +761,8 @@ __device__ __forceinline__ Real launch_param(const Real* P, uint32_t m, int k, R
       return (m & BC_M_CADET) ? -dexpm1(-dt / P[k]) : P[k];
     case BC_P_CA_D:
       return (m & BC_M_CADET) ? -dexpm1(-dt / P[BC_P_CA_TAU]) * P[BC_P_CA_TAU] * Real(kCaDrive) / P[k] : P[k];
+    case BC_P_ECA:
+      return (m & BC_M_CADET) ? Real(kNernstCa) * P[BC_P_CA_TEMP] * dlog(P[BC_P_CA_CO]) : P[k];
     default:
       return P[k];
   }
@@ -826,8 +830,8 @@ __device__ __forceinline__ void node_mechanisms(const NodeStates<Real, W>& s0, R
         const bool on = (m[j] & BC_M_CADET) != 0;
         cahi[j] = s0.cahi[j];
         calo[j] = s0.calo[j];
-        const Real co = P[j][BC_P_CA_CO], nernst = Real(kNernstCa) * P[j][BC_P_CA_TEMP];
-        Real c = cahi[j] + calo[j], E = nernst * dlog(adiv(co, c));
+        const Real slope = Real(kNernstCa) * P[j][BC_P_CA_TEMP], e_out = on ? k_of(j, BC_P_ECA) : Real(0);
+        Real c = cahi[j] + calo[j], E = fma_rn(-slope, ln_pos(c), e_out);
         if (kAdv) {
           Real ica = Real(0);
           if (mu & BC_M_CAL) {
@@ -845,7 +849,7 @@ __device__ __forceinline__ void node_mechanisms(const NodeStates<Real, W>& s0, R
           ff_add(cahi[j], calo[j],
                  (drive > Real(0) ? drive : Real(0)) + k_of(j, BC_P_CA_TAU) * (P[j][BC_P_CA_CREST] - c));
           c = cahi[j] + calo[j];
-          E = nernst * dlog(adiv(co, c));
+          E = fma_rn(-slope, ln_pos(c), e_out);
         }
         ci[j] = on ? c : ci[j];
         eca[j] = on ? E : eca[j];
@@ -896,7 +900,7 @@ __device__ __forceinline__ void node_mechanisms(const NodeStates<Real, W>& s0, R
             const Real n = P[j][BC_P_AHP_N];
             const Real a = P[j][BC_P_AHP_ALPHA] * (n == Real(2) || !on ? ci[j] * ci[j] : dpow(ci[j], n));
             const Real s = a + P[j][BC_P_AHP_BETA];
-            p[j] = p[j] - decay_em1(k_of(j, BC_P_AHP_PHI) * s) * (rdiv(a, s) - p[j]);
+            p[j] = p[j] - decay_em1(k_of(j, BC_P_AHP_PHI) * s) * (a * srcp(s) - p[j]);
           }
           add(j, BC_M_AHP, P[j][BC_P_AHP_G] * p[j] * p[j], P[j][BC_P_EK]);
         }
@@ -1895,7 +1899,7 @@ __global__ void __launch_bounds__(kVar >= 2 ? BC_PORT_MAX_THREADS : 1024, kVar >
       Real* L = rec + size_t(r) * tv.pstride;
       const uint32_t m = tv.mech[r];
       constexpr int keys[] = {BC_P_CA_D,    BC_P_CA_TAU,  BC_P_NA_PHI,  BC_P_KDR_PHI, BC_P_CAL_PHIP,
-                              BC_P_CAL_PHIQ, BC_P_CAT_PHIP, BC_P_CAT_PHIQ, BC_P_HCN_PHI, BC_P_AHP_PHI};
+                              BC_P_CAL_PHIQ, BC_P_CAT_PHIP, BC_P_CAT_PHIQ, BC_P_HCN_PHI, BC_P_AHP_PHI, BC_P_ECA};
 #pragma unroll
       for (int k : keys) L[k] = launch_param(P, m, k, dt);  // CA_D first: it reads CA_TAU
     }

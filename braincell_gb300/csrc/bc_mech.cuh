@@ -19,11 +19,12 @@
 //   Markov channels  channel/_base.py:677-1125 (template), quad/_backward_euler.py:31-64;
 //                    Nav1p6_MA2020_GoC sodium.py:727-940, Kca2p2_MA2020_GoC
 //                    potassium_calcium.py:613-790, Kca1p1_MA2020_GoC :1107-1353
-// CUDA's own exp / expm1 / log are called; nothing of the math library is
-// re-implemented here.
+// CUDA's own exp / expm1 / log / pow are called, but for the FP64 exponentials and
+// logarithms of the main mix, which have forms of their own (see exp2_256 and ln_pos).
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 
 #include "../../include/braincell_gb300.h"
 
@@ -66,53 +67,216 @@ __device__ __forceinline__ float adiv(float a, float b) {
 }
 __host__ __device__ __forceinline__ double adiv(double a, double b) { return a / b; }
 
-// 1 / x for the step's rate forms.  FP64: two Newton-Raphson steps from the hardware
-// estimate, r += r (1 - x r) (x normal and finite: the forms below see to it); on the
-// host, and where the estimate does not exist, the division.
+// 1 / x for the step's rate forms.  FP64: one third-order step from the hardware
+// estimate, e = 1 - x r, r += r (e + e^2) (x normal and finite: the forms below see to
+// it); on the host the division.
 __device__ __forceinline__ float srcp(float x) { return rcp_approx(x); }
 __host__ __device__ __forceinline__ double srcp(double x) {
 #ifdef __CUDA_ARCH__
   double r;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 #else
   return 1.0 / x;
 #endif
 }
 
-// exp(k v + c) with constant k and c.  FP32: one multiply-add into the base-2
+// ------------------------------------------------ FP64 exponential and logarithm
+// An SM retires two lanes of FP64 a clock, so an FP64 step takes as long as its FP64
+// instructions and nothing else: integer work, loads and branches are free beside them.
+// The main mix's exponentials and logarithms are therefore table-driven (P.T.P. Tang,
+// "Table-driven implementation of the exponential function", ACM TOMS 15, 1989, and "...
+// of the logarithm function", TOMS 16, 1990): 256 entries leave a polynomial of four
+// terms, and range checks and scaling are integer operations.  9 FP64 instructions for
+// exp(k v + c) with its linear argument and 8 for ln, where the library's functions with
+// the argument, the cap and the division before the logarithm take two to three times
+// that: 250 uneven cells of 50 to 2000 compartments, 200 FP64 steps, went from 50.2 to
+// 40.6 ms with these, the shorter decay series and the three-instruction reciprocal.
+// The tables come from the definitions, in double-double arithmetic at compile
+// time.
+struct TwoDouble {
+  double h, l;
+};
+constexpr TwoDouble dd_norm(double a, double b) {  // |a| >= |b|
+  const double s = a + b;
+  return {s, b - (s - a)};
+}
+constexpr double dd_upper(double a) {
+  const double t = 134217729.0 * a;
+  return t - (t - a);
+}
+constexpr TwoDouble dd_prod(double a, double b) {  // a b, exact (Dekker)
+  const double p = a * b, ah = dd_upper(a), bh = dd_upper(b), al = a - ah, bl = b - bh;
+  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr TwoDouble dd_mul(TwoDouble a, TwoDouble b) {
+  const TwoDouble p = dd_prod(a.h, b.h);
+  return dd_norm(p.h, p.l + (a.h * b.l + a.l * b.h));
+}
+constexpr TwoDouble dd_div(TwoDouble a, double b) {
+  const double q = a.h / b;
+  const TwoDouble p = dd_prod(q, b);
+  return dd_norm(q, ((a.h - p.h) - p.l + a.l) / b);
+}
+constexpr TwoDouble dd_add(TwoDouble a, TwoDouble b) {
+  const double s = a.h + b.h, t = s - a.h;
+  return dd_norm(s, ((a.h - (s - t)) + (b.h - t)) + (a.l + b.l));
+}
+constexpr TwoDouble kLn2{0.693147180559945309417, 2.31904681384629955842e-17};
+constexpr TwoDouble kLog2E2{1.44269504088896340736, 2.03552737409310331112e-17};
+
+constexpr int kExpTable = 256;
+struct ExpTable {
+  double t[kExpTable];  // 2^(j / 256)
+};
+constexpr ExpTable make_exp_table() {
+  const TwoDouble x = dd_div(kLn2, kExpTable);
+  TwoDouble step{1.0, 0.0}, term{1.0, 0.0};
+  for (int n = 1; n < 14; ++n) {
+    term = dd_div(dd_mul(term, x), double(n));
+    step = dd_add(step, term);
+  }
+  ExpTable e{};
+  TwoDouble v{1.0, 0.0};
+  for (int j = 0; j < kExpTable; ++j, v = dd_mul(v, step)) e.t[j] = v.h;
+  return e;
+}
+struct LnEntry {
+  double r, l;  // r close to 1 / (1 + (j + 1/2) / 256), l = -ln r
+};
+struct LnTable {
+  LnEntry t[256];
+};
+constexpr LnTable make_ln_table() {
+  LnTable e{};
+  for (int j = 0; j < 256; ++j) {
+    const double r = double(int(4096.0 / (1.0 + (j + 0.5) / 256) + 0.5)) / 4096;
+    const double z = (1.0 - r) / (1.0 + r), z2 = z * z;  // -ln r = 2 artanh z, z < 1/3
+    double s = 0.0;
+    for (int n = 35; n > 0; n -= 2) s = s * z2 + 1.0 / n;
+    e.t[j] = {r, 2.0 * z * s};
+  }
+  return e;
+}
+constexpr ExpTable kExp2Host = make_exp_table();
+constexpr LnTable kLnHost = make_ln_table();
+static __device__ const ExpTable kExp2Dev = make_exp_table();
+static __device__ const LnTable kLnDev = make_ln_table();
+
+__host__ __device__ __forceinline__ int hi_word(double x) {
+#ifdef __CUDA_ARCH__
+  return __double2hiint(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return int(u >> 32);
+#endif
+}
+__host__ __device__ __forceinline__ int lo_word(double x) {
+#ifdef __CUDA_ARCH__
+  return __double2loint(x);
+#else
+  uint64_t u;
+  memcpy(&u, &x, 8);
+  return int(uint32_t(u));
+#endif
+}
+__host__ __device__ __forceinline__ double from_words(int hi, int lo) {
+#ifdef __CUDA_ARCH__
+  return __hiloint2double(hi, lo);
+#else
+  const uint64_t u = uint64_t(uint32_t(hi)) << 32 | uint32_t(lo);
+  double x;
+  memcpy(&x, &u, 8);
+  return x;
+#endif
+}
+// 2^(y / 256).  |y| is capped at 258048 + (the exponent then stays normal: 2^-1008 to
+// 2^1008 stand for 0 and infinity); a NaN counts as the cap.
+__host__ __device__ __forceinline__ double exp2_256(double y) {
+  constexpr double kRound = 6755399441055744.0;  // 1.5 2^52: the sum's low word is y rounded
+  constexpr double c1 = dd_div(kLn2, 256.0).h, c2 = c1 * c1 / 2, c3 = c1 * c2 / 3, c4 = c1 * c3 / 4;
+  const int h = hi_word(y), mag = h & 0x7fffffff, cap = 0x410f8000;
+  y = from_words((h & int(0x80000000)) | (mag < cap ? mag : cap), lo_word(y));
+  const double t = y + kRound;
+  const int n = lo_word(t);
+  const double f = y - (t - kRound);
+  const double p = f * fma(f, fma(f, fma(f, c4, c3), c2), c1);  // e^(f ln2 / 256) - 1 to 3e-17
+#ifdef __CUDA_ARCH__
+  const double s = __ldg(&kExp2Dev.t[n & 255]);
+#else
+  const double s = kExp2Host.t[n & 255];
+#endif
+  const double r = fma(s, p, s);
+  return from_words(hi_word(r) + int(uint32_t(n & ~255) << 12), lo_word(r));
+}
+// ln x of a positive normal x, to the rounding of the result or of 1, whichever is
+// larger; log for any other x.
+__device__ __forceinline__ float ln_pos(float x) { return dlog(x); }
+__host__ __device__ __forceinline__ double ln_pos(double x) {
+  const int h = hi_word(x);
+  if (unsigned(h - 0x00100000) >= 0x7fe00000u) return dlog(x);
+  const double m = from_words((h & 0x000fffff) | 0x3ff00000, lo_word(x));
+#ifdef __CUDA_ARCH__
+  const double2 e = __ldg(reinterpret_cast<const double2*>(kLnDev.t) + (h >> 12 & 255));
+  const double er = e.x, el = e.y;
+#else
+  const double er = kLnHost.t[h >> 12 & 255].r, el = kLnHost.t[h >> 12 & 255].l;
+#endif
+  const double r = fma(m, er, -1.0);  // |r| < 2.2e-3: the series to r^5 leaves 2e-17
+  const int e2 = (h >> 20) - 1023;
+  const double n = from_words(0x43380000 + (e2 >> 31), e2) - 6755399441055744.0;
+  const double q = fma(r * r, fma(r, fma(r, fma(r, 1.0 / 5, -1.0 / 4), 1.0 / 3), -0.5), r);
+  return fma(n, kLn2.h, el) + q;
+}
+
+// exp((a v + b) / w) with constant a, b, w.  FP32: one multiply-add into the base-2
 // exponential, so the result may overflow to infinity (rcp makes it 0 again) but is
-// never wrong by a denormal's worth.  FP64: the exponent is capped at 700.
+// never wrong by a denormal's worth.  FP64: capped as exp2_256 is; the coefficients are
+// rounded once.
 constexpr double kLog2E = 1.4426950408889634;
+struct ExpLine {
+  float k32, c32;
+  double k, c;
+  constexpr ExpLine(double a, double b, double w)
+      : k32(float(a / w * kLog2E)), c32(float(b / w * kLog2E)),
+        k(256.0 * dd_mul(dd_div({a, 0.0}, w), kLog2E2).h), c(256.0 * dd_mul(dd_div({b, 0.0}, w), kLog2E2).h) {}
+};
 __device__ __forceinline__ float ex2_ftz(float x) {
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-__device__ __forceinline__ float lin_exp(float v, double k, double c) {
-  return ex2_ftz(fmaf(v, float(k * kLog2E), float(c * kLog2E)));
+__device__ __forceinline__ float lin_exp(float v, const ExpLine& e) { return ex2_ftz(fmaf(v, e.k32, e.c32)); }
+__host__ __device__ __forceinline__ double lin_exp(double v, const ExpLine& e) { return exp2_256(fma(v, e.k, e.c)); }
+// exp(a |x| / w), a < 0: at most 1, so squares and sums of it stay in range.  NaN stays NaN.
+__device__ __forceinline__ float exp_neg_abs(float x, const ExpLine& e) { return ex2_ftz(fabsf(x) * e.k32); }
+__host__ __device__ __forceinline__ double exp_neg_abs(double x, const ExpLine& e) {
+  const double y = fabs(x) * e.k;
+  return (hi_word(y) & 0x7fffffff) > 0x7ff00000 ? y : exp2_256(y);
 }
-__host__ __device__ __forceinline__ double lin_exp(double v, double k, double c) { return exp(fmin(fma(v, k, c), 700.0)); }
-// exp(-|x| k), k > 0: at most 1, so squares and sums of it stay in range.
-__device__ __forceinline__ float exp_neg_abs(float x, double k) { return ex2_ftz(fabsf(x) * float(-k * kLog2E)); }
-__host__ __device__ __forceinline__ double exp_neg_abs(double x, double k) { return exp(fabs(x) * -k); }
 
 // e^x - 1 for the exp-Euler decay of a gate (x = dt * lambda <= 0).  FP32: for
 // |x| < 1/4 the Taylor series of e^x - 1 to x^6 (truncation < 5e-8 relative, the
 // float rounding level); otherwise exp(x) - 1, which has no cancellation there.
-// FP64: the series to x^9 below 1/64 and to x^12 below 1/8 (truncation below 1e-18 of
-// the result), expm1 above.
+// FP64: the series to x^5 below 2^-10, to x^8 below 1/64 and to x^12 below 1/8
+// (truncation below 2e-18 of the result), expm1 above.
 __device__ __forceinline__ float decay_em1(float x) {
   const float p = x * (1.0f + x * (0.5f + x * (1.0f / 6.0f + x * (1.0f / 24.0f + x * (1.0f / 120.0f + x * (1.0f / 720.0f))))));
   return fabsf(x) < 0.25f ? p : ex2_ftz(x * float(kLog2E)) - 1.0f;
 }
 __host__ __device__ __forceinline__ double decay_em1(double x) {
-  if (!(fabs(x) < 0.125)) return expm1(x);
-  double s = 1.0 / 362880;
-  if (fabs(x) >= 0.015625) s += x * (1.0 / 3628800 + x * (1.0 / 39916800 + x * (1.0 / 479001600)));
-  return x * (1.0 + x * (1.0 / 2 + x * (1.0 / 6 + x * (1.0 / 24 + x * (1.0 / 120 + x * (1.0 / 720 +
-         x * (1.0 / 5040 + x * (1.0 / 40320 + x * s))))))));
+  const int mag = hi_word(x) & 0x7fffffff;
+  if (mag >= 0x3fc00000) return expm1(x);  // 1/8 and more, NaN
+  double s = 1.0 / 120;
+  if (mag >= 0x3f500000) {  // 2^-10
+    double t = 1.0 / 40320;
+    if (mag >= 0x3f900000)  // 1/64
+      t = fma(x, fma(x, fma(x, fma(x, 1.0 / 479001600, 1.0 / 39916800), 1.0 / 3628800), 1.0 / 362880), t);
+    s = fma(x, fma(x, fma(x, t, 1.0 / 5040), 1.0 / 720), s);
+  }
+  return x * fma(x, fma(x, fma(x, fma(x, s, 1.0 / 24), 1.0 / 6), 0.5), 1.0);
 }
 
 // exprel(x) = (e^x - 1) / x, exprel(0) = 1
@@ -225,35 +389,39 @@ struct GateStep {
   __host__ __device__ __forceinline__ Real step(Real g) const { return g - decay_em1(x) * (inf - g); }
 };
 template <typename Real>
-__host__ __device__ __forceinline__ Real bell_rate(Real k, Real y, double inv_width, double base, double height) {
-  const Real z = exp_neg_abs(y, inv_width);
+__host__ __device__ __forceinline__ Real bell_rate(Real k, Real y, const ExpLine& bell, double base, double height) {
+  const Real z = exp_neg_abs(y, bell);
   const Real w = Real(1) + z * z;  // tau = base + height z / w
   return k * w * srcp(Real(base) * w + Real(height) * z);
 }
 template <typename Real>
 __host__ __device__ __forceinline__ GateStep<Real> cal_p_step(Real vs, Real k) {
-  return {srcp(Real(1) + lin_exp(vs, -1.0 / 4, -10.0 / 4)), bell_rate(k, vs + Real(5), 1.0 / 15, 0.4, 0.7)};
+  constexpr ExpLine inf(-1.0, -10.0, 4.0), bell(-1.0, 0.0, 15.0);
+  return {srcp(Real(1) + lin_exp(vs, inf)), bell_rate(k, vs + Real(5), bell, 0.4, 0.7)};
 }
 template <typename Real>
 __host__ __device__ __forceinline__ GateStep<Real> cal_q_step(Real vs, Real k) {
-  return {srcp(Real(1) + lin_exp(vs, 1.0 / 2, 25.0 / 2)), bell_rate(k, vs + Real(40), 1.0 / 9.5, 300.0, 100.0)};
+  constexpr ExpLine inf(1.0, 25.0, 2.0), bell(-1.0, 0.0, 9.5);
+  return {srcp(Real(1) + lin_exp(vs, inf)), bell_rate(k, vs + Real(40), bell, 300.0, 100.0)};
 }
 template <typename Real>
 __host__ __device__ __forceinline__ GateStep<Real> cat_p_step(Real vs, Real k) {
   // tau = 1 / s + 0.612; s is capped where 1 / s no longer counts
-  Real s = lin_exp(vs, -1.0 / 16.7, -132.0 / 16.7) + lin_exp(vs, 1.0 / 18.2, 16.8 / 18.2);
+  constexpr ExpLine inf(-1.0, -59.0, 6.2), down(-1.0, -132.0, 16.7), up(1.0, 16.8, 18.2);
+  Real s = lin_exp(vs, down) + lin_exp(vs, up);
   s = s < Real(1e18) ? s : Real(1e18);
-  return {srcp(Real(1) + lin_exp(vs, -1.0 / 6.2, -59.0 / 6.2)), k * s * srcp(Real(1) + Real(0.612) * s)};
+  return {srcp(Real(1) + lin_exp(vs, inf)), k * s * srcp(Real(1) + Real(0.612) * s)};
 }
 template <typename Real>
 __host__ __device__ __forceinline__ GateStep<Real> cat_q_step(Real vs, Real k) {
-  const Real tau = vs >= Real(-80) ? lin_exp(vs, -1.0 / 10.5, -22.0 / 10.5) + Real(28) : lin_exp(vs, 1.0 / 66.6, 467.0 / 66.6);
-  return {srcp(Real(1) + lin_exp(vs, 1.0 / 4, 83.0 / 4)), k * srcp(tau)};
+  constexpr ExpLine inf(1.0, 83.0, 4.0), high(-1.0, -22.0, 10.5), low(1.0, 467.0, 66.6);
+  const Real tau = vs >= Real(-80) ? lin_exp(vs, high) + Real(28) : lin_exp(vs, low);
+  return {srcp(Real(1) + lin_exp(vs, inf)), k * srcp(tau)};
 }
 template <typename Real>
 __host__ __device__ __forceinline__ GateStep<Real> hcn_step(Real v, Real k) {
-  return {srcp(Real(1) + lin_exp(v, 1.0 / 5.5, 75.0 / 5.5)),
-          k * (lin_exp(v, -0.086, -14.59) + lin_exp(v, 0.0701, -1.87))};
+  constexpr ExpLine inf(1.0, 75.0, 5.5), down(-0.086, -14.59, 1.0), up(0.0701, -1.87, 1.0);
+  return {srcp(Real(1) + lin_exp(v, inf)), k * (lin_exp(v, down) + lin_exp(v, up))};
 }
 
 template <typename Real>
