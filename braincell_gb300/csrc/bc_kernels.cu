@@ -225,11 +225,12 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Reciprocal of a Hines pivot.  FP32: the hardware approximation (about 1 ulp;
-// pivots are >= 1 on membrane rows and O(dt * g / C) on boundary rows, far from
-// the denormal range); FP64: IEEE round-to-nearest.
-__device__ __forceinline__ float pivot_rcp(float d) { return rcp_approx(d); }
-__device__ __forceinline__ double pivot_rcp(double d) { return __drcp_rn(d); }
+// Reciprocal of a pivot, to about 1 ulp in both precisions (pivots are >= 1 on membrane
+// rows and O(dt * g / C) on boundary rows, far from the denormal range).
+template <typename Real>
+__device__ __forceinline__ Real pivot_rcp(Real d) {
+  return srcp(d);
+}
 
 // a * b and a + b rounded (never parts of a fused multiply-add), and a * b + c fused:
 // where the same sum stands in several copies of the code (the two nodes of a lane, the

@@ -1838,6 +1838,52 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   const size_t ctas_per_sm = std::max<size_t>(1, per_sm / (est + cta_reserve));
   const size_t packed_budget =
       std::min(smem_budget, std::max(est, per_sm / ctas_per_sm > cta_reserve ? per_sm / ctas_per_sm - cta_reserve : est));
+  // FP64 tiles that leave half of the SMs idle run as global-memory tiles, each on a cluster of CTAs: a step is bound
+  // by the FP64 pipes of the SMs in use, not by where the tile lives (63 tiles of 2500 nodes: 197 us a step on one CTA
+  // each, 159 on two; 20 cells of up to 2000: 154 on one, 103 on four).  FP32 tiles are bound by latency and stay.
+  // The cluster grows while that takes a fifth off the largest load of an SM, in nodes: the largest tile's share, or
+  // that of the CTAs an SM gets (clusters above two CTAs leave about an eighth of the SMs without one; the 63 tiles on
+  // four CTAs each: 177 us).  A CTA of 128 nodes already has a warp for each of its four FP64 pipes, so
+  // every CTA gets at least twice that.
+  std::vector<int> cls_was;
+  int want_cluster = 16;
+  if (p->precision == BC_PREC_F64 && s.n_ports == 0 && !p->use_graph) {
+    size_t n_tiles = 0;
+    int64_t largest = 0, total = 0;
+    for (size_t t = 0; t < builds.size(); ++t)
+      if (builds[t].cls != 3) {
+        ++n_tiles;
+        largest = std::max(largest, fill[t]);
+        total += fill[t];
+      }
+    const auto load = [&](int c) {
+      const int64_t ctas = int64_t(n_tiles) * c, sms = c > 2 ? n_sm * 7 / 8 : n_sm;
+      return std::max(double(largest) / c, double((ctas + sms - 1) / sms) * double(total) / double(ctas));
+    };
+    want_cluster = 1;
+    for (int c = 2; c <= 16 && n_tiles > 0 && largest >= 256 * c && load(c) < 0.8 * load(c / 2); c *= 2) want_cluster = c;
+    if (want_cluster > 1 && 2 * n_tiles <= size_t(n_sm))
+      for (TileBuild& tb : builds) {
+        cls_was.push_back(tb.cls);
+        if (tb.cls < 2) tb.cls = 2;
+      }
+  }
+  const auto global_cluster = [&]() {
+    int count = 0;
+    size_t bytes = 0;
+    for (size_t t = 0; t < builds.size(); ++t) {
+      if (builds[t].cls != 2) continue;
+      const TileDesc& d = outs[t].desc;
+      if (!d.sep_in_smem) return 1;
+      ++count;
+      bytes = std::max(bytes, size_t(d.sep_bytes) + size_t(d.off_rows - d.off_seps));
+    }
+    if (count == 0 || count > n_sm || s.n_ports > 0 || p->use_graph) return 1;
+    if (dry) return 2;
+    return tile_cluster(p->precision, p->extra ? BC_VARIANT_EXTRA : BC_VARIANT_LEAN, want_cluster, count, T_glob,
+                        bytes);
+  };
+build_again:
   for (size_t t = 0; t < builds.size(); ++t) {
     TileOut to;
     bc_status st = build_tile(cx, builds[t], class_threads[builds[t].cls], to);
@@ -1891,6 +1937,12 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     }
     outs.push_back(std::move(to));
   }
+  if (!cls_was.empty() && global_cluster() == 1) {  // no clusters after all: back to shared memory
+    for (size_t t = 0; t < builds.size(); ++t) builds[t].cls = cls_was[t];
+    cls_was.clear();
+    outs.clear();
+    goto build_again;
+  }
   // tiles ordered by class; one launch per class
   std::vector<size_t> tord;
   for (int cl = 0; cl < kMaxClasses; ++cl) {
@@ -1917,15 +1969,9 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
       });
     }
     lcz.count = int(tord.size()) - lcz.first;
-    if (cl == 2 && lcz.count > 0 && !dry && s.n_ports == 0 && !p->use_graph) {
-      // few global-memory tiles: on each the largest cluster of CTAs at which they all run at once (one cell of
-      // 18,700 nodes: 127 us a step on one CTA, 41 on 16; 16 cells on clusters of 16, more than fit: 81)
-      bool seps_fit = true;
-      for (size_t t = 0; t < builds.size(); ++t) seps_fit = seps_fit && (builds[t].cls != 2 || outs[t].desc.sep_in_smem);
-      if (seps_fit && 2 * lcz.count <= 2 * n_sm)
-        lcz.cluster = tile_cluster(p->precision, p->extra ? BC_VARIANT_EXTRA : BC_VARIANT_LEAN, 16, lcz.count, lcz.threads,
-                                   lcz.smem_bytes);
-    }
+    // few global-memory tiles: on each the largest cluster of CTAs at which they all run at once (one cell of 18,700
+    // nodes: 127 us a step on one CTA, 41 on 16; 16 cells on clusters of 16, more than fit: 81)
+    if (cl == 2) lcz.cluster = global_cluster();
     if (lcz.count > 0) p->classes.push_back(lcz);
   }
   p->n_smem_tiles = 0;
