@@ -1,7 +1,7 @@
 // sm_103a kernels of the multi-compartment Cell time step.
 //
 // One CTA owns one tile (one or more whole cells).  For shared-memory tiles the
-// tile's blob (voltages, axial coefficients, chain schedule, parameter records)
+// tile's blob (voltages, axial coefficients, segment schedule, parameter records)
 // is staged into shared memory with TMA bulk copies (cp.async.bulk + mbarrier),
 // stays resident for `n_steps` fused time steps, and only the voltages are
 // written back with a bulk store.  Mechanism states (gates, calcium) stream from

@@ -91,7 +91,7 @@ class Plan:
         self.n_probes = int(info.n_probes)
 
     def tile_stats(self) -> np.ndarray:
-        """``[n_tiles, 6]``: nodes, chain records, phases, critical path, class, shared bytes."""
+        """``[n_tiles, 6]``: nodes, segments, 1 + separator levels, critical path, class, shared bytes."""
         out = np.zeros((int(self.info["n_tiles"]), 6), dtype=np.int64)
         _abi.check(self._lib.bc_plan_tile_stats(self._h, out.ctypes.data_as(C.POINTER(C.c_int64))))
         return out

@@ -48,11 +48,11 @@ V_SCALE = 10.0       # mV
 # nodes each; 384 threads is the port kernel's register budget at two per SM.
 PORT_TILE_NODES = 1800
 PORT_THREADS = 384
-# Serial-walk length of the reduced tiles' warp slots: a GB300 sweep of the 10,000-cell
-# reduced run (1,000-step launches) gave 76.4 / 74.4 / 75.4 ms per 1,000 steps at 4 / 6 / 10.
+# Unbranched runs of the reduced cells above this many nodes may be cut.  The 10,000-cell reduced
+# run takes 53.3 / 52.9 / 52.9 ms per 1,000 steps at 4 / 6 / 10.
 PORT_LANE_NODES = 6
-# Reduced plans launch their longest tiles first (tile_order 1): 74.0-74.3 against
-# 74.7-74.9 ms per 1,000 steps in build order on the same GB300.
+# Reduced plans launch their longest tiles first (tile_order 1): 52.9 against 53.2 ms per 1,000
+# steps in build order on the same GB300.
 PORT_TILE_ORDER = 1
 # Fallback (full-morphology) plans run the kernel without ports in large tiles.
 FALLBACK_TILE_NODES = 2500

@@ -430,7 +430,7 @@ typedef struct bc_plan_info_t {
   int32_t threads_per_tile, tile_nodes, steps_per_launch, precision;
   int64_t smem_bytes_per_tile;   /* dynamic shared memory per CTA                    */
   int64_t device_bytes;          /* device memory held by the plan                   */
-  int64_t max_phases;            /* largest barrier-phase count of any tile          */
+  int64_t max_phases;            /* 1 + the most separator levels of any tile         */
   int64_t max_chain_nodes;       /* longest per-thread node walk (critical path)     */
   int32_t state_slots;           /* per-node mechanism state slots                   */
   int32_t n_smem_tiles;          /* tiles resident in shared memory                  */
@@ -475,7 +475,7 @@ bc_status bc_plan_destroy(bc_plan_t plan);
 bc_status bc_plan_info(bc_plan_t plan, bc_plan_info_t* info);
 
 /* Per-tile schedule statistics, 6 int64 per tile in launch order: real nodes,
- * chain records, barrier phases, critical-path estimate (node visits of the
+ * segments, 1 + separator levels, critical-path estimate (node visits of the
  * busiest thread summed over phases), launch class (0 packed shared-memory tile,
  * 1 single-cell shared-memory tile, 2 global-memory tile, 3 lane tile: one cell per
  * thread), shared bytes. */
