@@ -743,7 +743,8 @@ __device__ __noinline__ void extra_channels(Real* st, int N, const Real* P, uint
 // are replaced by what the step needs (kDer), once per launch, in the records' shared-
 // memory copy or in a copy in the tile's scratch:
 //   PHI entries -> -dt phi;  CA_TAU -> c = 1 - exp(-dt / tau);  CA_D -> the shell's gain
-//   c tau 10 / (2 F d), so that the calcium step is Ci += max(gain ICa, 0) + c (C_rest - Ci);
+//   c tau 10 / (2 F d) (c tau = dt where tau is infinite: shell_gain), so that the calcium
+//   step is Ci += max(gain ICa, 0) + c (C_rest - Ci);
 //   E_Ca of a dynamic ion, which nothing reads -> slope ln C_out, so that its Nernst
 //   potential is that minus slope ln Ci: no division beside the logarithm.
 template <typename Real>
@@ -761,7 +762,7 @@ __device__ __forceinline__ Real launch_param(const Real* P, uint32_t m, int k, R
     case BC_P_CA_TAU:
       return (m & BC_M_CADET) ? -dexpm1(-dt / P[k]) : P[k];
     case BC_P_CA_D:
-      return (m & BC_M_CADET) ? -dexpm1(-dt / P[BC_P_CA_TAU]) * P[BC_P_CA_TAU] * Real(kCaDrive) / P[k] : P[k];
+      return (m & BC_M_CADET) ? shell_gain(dt, P[BC_P_CA_TAU]) * Real(kCaDrive) / P[k] : P[k];
     case BC_P_ECA:
       return (m & BC_M_CADET) ? Real(kNernstCa) * P[BC_P_CA_TEMP] * dlog(P[BC_P_CA_CO]) : P[k];
     default:

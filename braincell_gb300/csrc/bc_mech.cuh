@@ -285,6 +285,15 @@ __host__ __device__ __forceinline__ Real exprel(Real x) {
   return x == Real(0) ? Real(1) : dexpm1(x) / x;
 }
 
+// What a step adds to the calcium of a shell per unit of its drive: dt exprel(-dt / tau) =
+// (1 - e^(-dt / tau)) tau, dt for a shell that does not decay (tau infinite, or so long that
+// the quotient has no bits left).
+template <typename Real>
+__host__ __device__ __forceinline__ Real shell_gain(Real dt, Real tau) {
+  const Real x = dt / tau;
+  return x < Real(1e-30) && x >= Real(0) ? dt : -dexpm1(-x) * tau;
+}
+
 // c / exprel(x) = c x / (e^x - 1), c at x = 0, with one division; FP32: x is capped at
 // 80, where the quotient is below 1e-32 of c.
 __device__ __forceinline__ float over_exprel(float c, float x) {
