@@ -351,6 +351,10 @@ struct LaunchArgs {
 // whose only optional feature is its ports).
 int launch_tiles(const LaunchArgs& a, int precision, bool smem, int threads, size_t smem_bytes, int variant,
                  void* stream);
+// Shared memory of a CTA that is not a tile's: the kernels' static variables, and slack.
+constexpr int kStaticSmem = 1024;
+// Raises the limits of the kernel that launch_tiles takes, on the current device, before the first launch.
+int prepare_tiles(int precision, bool smem, int variant);
 // Largest cluster, a power of two up to `want`, at which `count` global-memory tiles run at once.
 int tile_cluster(int precision, int variant, int want, int count, int threads, size_t smem_bytes);
 // Kernel-node parameters of the same launch for a CUDA graph (clusters of 1).  kernelParams

@@ -2379,16 +2379,46 @@ static void cluster_config(const LaunchArgs& a, int threads, size_t smem_bytes, 
   cfg.numAttrs = 1;
 }
 
+// Lets a tile kernel take as much dynamic shared memory as any plan may need, and clusters
+// of 16, once for each plan that runs it.  Both limits belong to the kernel, not to the
+// launch: set to each launch's own size, the first could be lowered by another thread's plan
+// just before the launch, which then failed.
+template <typename Kernel>
+static cudaError_t raise_limits(Kernel k, bool clusters) {
+  int device = 0, cap = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, cap - kStaticSmem);
+  if (e == cudaSuccess && clusters) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  return e;
+}
+
+template <int kVar>
+static int prepare_x(int precision, bool smem) {
+  if (precision == BC_PREC_F64)
+    return int(smem ? raise_limits(tile_step_kernel<double, true, kVar>, false)
+                    : raise_limits(tile_step_kernel<double, false, kVar>, kVar < 2));
+  return int(smem ? raise_limits(tile_step_kernel<float, true, kVar>, false)
+                  : raise_limits(tile_step_kernel<float, false, kVar>, kVar < 2));
+}
+
+int prepare_tiles(int precision, bool smem, int variant) {
+  switch (variant) {
+    case 0:
+      return prepare_x<0>(precision, smem);
+    case 1:
+      return prepare_x<1>(precision, smem);
+    case 2:
+      return prepare_x<2>(precision, smem);
+    default:
+      return prepare_x<3>(precision, smem);
+  }
+}
+
 template <typename Real, bool kSmem, int kVar>
 static int launch_impl(const LaunchArgs& a, int threads, size_t smem_bytes, cudaStream_t st) {
   auto k = tile_step_kernel<Real, kSmem, kVar>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
-  if (e != cudaSuccess) return int(e);
   if (!kSmem && a.cluster > 1) {
-    if (a.cluster > 8) {
-      e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return int(e);
-    }
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
     cluster_config(a, threads, smem_bytes, st, cfg, attr);
@@ -2402,8 +2432,7 @@ static int launch_impl(const LaunchArgs& a, int threads, size_t smem_bytes, cuda
 template <typename Real, int kVar>
 static int usable_cluster(int want, int count, int threads, size_t smem_bytes) {
   auto k = tile_step_kernel<Real, false, kVar>;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes)) != cudaSuccess) return 1;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) want = std::min(want, 8);
+  if (raise_limits(k, true) != cudaSuccess) return 1;
   for (int c = want; c > 1; c /= 2) {
     LaunchArgs a{};
     a.n_tiles = 1;
@@ -2458,10 +2487,7 @@ int launch_tiles(const LaunchArgs& a, int precision, bool smem, int threads, siz
 // that consumes the parameters.
 template <typename Real, bool kSmem, int kVar>
 static int node_impl(const LaunchArgs* a, int threads, size_t smem_bytes, cudaKernelNodeParams* np) {
-  auto k = tile_step_kernel<Real, kSmem, kVar>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_bytes));
-  if (e != cudaSuccess) return int(e);
-  np->func = reinterpret_cast<void*>(k);
+  np->func = reinterpret_cast<void*>(tile_step_kernel<Real, kSmem, kVar>);
   np->gridDim = dim3(a->n_tiles, 1, 1);
   np->blockDim = dim3(threads, 1, 1);
   np->sharedMemBytes = unsigned(smem_bytes);

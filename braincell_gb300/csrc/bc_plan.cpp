@@ -1728,8 +1728,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     delete p;
     return fail(BC_ERR_CUDA, "could not query the shared-memory limit of the device");
   }
-  const size_t static_smem = 1024;  // static shared memory of the kernel (mbarrier, status) + slack
-  const size_t smem_budget = smem_cap - static_smem;
+  const size_t smem_budget = smem_cap - kStaticSmem;
   // shared bytes per node, for packing: V, (alpha, beta) and row pairs, link and region / special indices, and
   // per 6.4 nodes a segment (record, inbox), per 16 a separator, a third of the nodes with a q entry
   const double bpn = 6.0 * double(rs) + 8.0 + (16.0 + 2.0 * double(rs)) / 6.4 + (20.0 + 9.0 * double(rs)) / 16.0 +
@@ -1832,7 +1831,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   // estimate); the shared-memory budget of one tile is then that SM's share, so
   // tiles fill up to tile_nodes without lowering the occupancy.
   const size_t per_sm = dry ? size_t(233472) : sm_smem(opts.device);
-  const size_t cta_reserve = 2 * static_smem;  // static shared memory + the system's per-CTA reserve
+  const size_t cta_reserve = 2 * kStaticSmem;  // static shared memory + the system's per-CTA reserve
   // a tile with ports also holds the weight fragments of the GRU
   const size_t est = size_t(double(tile_nodes) * bpn) + 2048 + (s.n_ports > 0 ? size_t(kGruSmemBytes) : 0);
   const size_t ctas_per_sm = std::max<size_t>(1, per_sm / (est + cta_reserve));
@@ -2058,6 +2057,8 @@ build_again:
   }
   p->blob_bytes = blob_total;
   p->scratch_bytes = scratch_total;
+  for (const LaunchClass& lcz : p->classes)
+    if (!lcz.lane) BC_TRYC(cudaError_t(prepare_tiles(p->precision, lcz.smem, kernel_variant(p))));
   BC_TRY(dalloc(p, &p->d_blob, blob_total));
   BC_TRY(dalloc(p, &p->d_scratch, scratch_total));
   p->state_bytes = size_t(state_total) * rs;
@@ -2134,7 +2135,7 @@ build_again:
     BC_TRY(dalloc(p, &p->d_gru, 1));
     BC_TRYC(cudaMemcpy(p->d_ports, p->ports.data(), p->ports.size() * sizeof(PortRec), cudaMemcpyHostToDevice));
   }
-  if (p->n_smem_tiles > 0 && p->smem_bytes + static_smem > smem_cap) {
+  if (p->n_smem_tiles > 0 && p->smem_bytes + kStaticSmem > smem_cap) {
     free_plan(p);
     return fail(BC_ERR_CAPACITY, "tile shared memory exceeds the device limit");
   }
