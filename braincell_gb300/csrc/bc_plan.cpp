@@ -1762,9 +1762,7 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     return fail(BC_ERR_INVALID, "plans with surrogate ports run at most " + std::to_string(BC_PORT_MAX_THREADS) +
                                     " threads per tile");
   }
-  const int class_threads[kMaxClasses] = {T_packed, T_big, T_glob, kLaneThreads};
-  p->threads = T_packed;
-  p->threads_global = T_glob;
+  int class_threads[kMaxClasses] = {T_packed, T_big, T_glob, kLaneThreads};
   std::vector<int64_t> order(s.n_cells);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(),
@@ -1861,11 +1859,15 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     };
     want_cluster = 1;
     for (int c = 2; c <= 16 && n_tiles > 0 && largest >= 256 * c && load(c) < 0.8 * load(c / 2); c *= 2) want_cluster = c;
-    if (want_cluster > 1 && 2 * n_tiles <= size_t(n_sm))
+    if (want_cluster > 1 && 2 * n_tiles <= size_t(n_sm)) {
+      int asked = 0;  // CTA size that the caller gave for the tiles that move
       for (TileBuild& tb : builds) {
         cls_was.push_back(tb.cls);
+        if (tb.cls < 2) asked = std::max(asked, tb.cls == 0 ? opts.threads_per_tile : opts.threads_big);
         if (tb.cls < 2) tb.cls = 2;
       }
+      if (opts.threads_global <= 0 && asked > 0) class_threads[2] = asked;
+    }
   }
   const auto global_cluster = [&]() {
     int count = 0;
@@ -1879,8 +1881,8 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
     }
     if (count == 0 || count > n_sm || s.n_ports > 0 || p->use_graph) return 1;
     if (dry) return 2;
-    return tile_cluster(p->precision, p->extra ? BC_VARIANT_EXTRA : BC_VARIANT_LEAN, want_cluster, count, T_glob,
-                        bytes);
+    return tile_cluster(p->precision, p->extra ? BC_VARIANT_EXTRA : BC_VARIANT_LEAN, want_cluster, count,
+                        class_threads[2], bytes);
   };
 build_again:
   for (size_t t = 0; t < builds.size(); ++t) {
@@ -1939,9 +1941,12 @@ build_again:
   if (!cls_was.empty() && global_cluster() == 1) {  // no clusters after all: back to shared memory
     for (size_t t = 0; t < builds.size(); ++t) builds[t].cls = cls_was[t];
     cls_was.clear();
+    class_threads[2] = T_glob;
     outs.clear();
     goto build_again;
   }
+  p->threads = cls_was.empty() ? T_packed : class_threads[2];
+  p->threads_global = class_threads[2];
   // tiles ordered by class; one launch per class
   std::vector<size_t> tord;
   for (int cl = 0; cl < kMaxClasses; ++cl) {

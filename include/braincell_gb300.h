@@ -406,7 +406,11 @@ typedef struct bc_plan_options {
   int32_t device;           /* CUDA device ordinal                                   */
   int32_t threads_big;      /* CTA size for tiles holding one cell larger than
                                tile_nodes; 0 = auto                                   */
-  int32_t threads_global;   /* CTA size for global-memory tiles; 0 = auto            */
+  int32_t threads_global;   /* CTA size for global-memory tiles; 0 = auto.  FP64 plans
+                               of few tiles run them as global-memory tiles, each on a
+                               cluster of CTAs of this size; where it is 0, of the size
+                               given for them by threads_per_tile or threads_big (the
+                               larger one when both kinds move), else 512            */
   int32_t narrow_lane_nodes; /* accepted and without effect: all runs of a tile are
                                eliminated in one pass, so there are no narrow phases */
   float reserved_b;         /* must be 0                                             */
@@ -427,7 +431,8 @@ typedef struct bc_plan* bc_plan_t;
 /* Plan statistics (host-side, filled by bc_plan_info). */
 typedef struct bc_plan_info_t {
   int64_t n_cells, n_cv, n_nodes, n_tiles, n_probes, n_pulses;
-  int32_t threads_per_tile, tile_nodes, steps_per_launch, precision;
+  int32_t threads_per_tile;      /* CTA size of the packed tiles (of the global-memory tiles they became) */
+  int32_t tile_nodes, steps_per_launch, precision;
   int64_t smem_bytes_per_tile;   /* dynamic shared memory per CTA                    */
   int64_t device_bytes;          /* device memory held by the plan                   */
   int64_t max_phases;            /* 1 + the most separator levels of any tile         */
