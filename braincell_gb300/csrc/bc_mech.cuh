@@ -290,8 +290,8 @@ __host__ __device__ __forceinline__ Real exprel(Real x) {
 // the quotient has no bits left).
 template <typename Real>
 __host__ __device__ __forceinline__ Real shell_gain(Real dt, Real tau) {
-  const Real x = dt / tau;
-  return x < Real(1e-30) && x >= Real(0) ? dt : -dexpm1(-x) * tau;
+  const Real x = -dt / tau, c = -dexpm1(x);  // c: the decay's own factor, formed once where both are
+  return fabs(x) < Real(1e-30) ? dt : c * tau;
 }
 
 // c / exprel(x) = c x / (e^x - 1), c at x = 0, with one division; FP32: x is capped at
