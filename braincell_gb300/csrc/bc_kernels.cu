@@ -234,7 +234,8 @@ __device__ __forceinline__ Real pivot_rcp(Real d) {
 
 // a * b and a + b rounded (never parts of a fused multiply-add), and a * b + c fused:
 // where the same sum stands in several copies of the code (the two nodes of a lane, the
-// forms of a warp), so that a node's result does not depend on which copy it met.
+// forms of a warp, tiles in shared and in global memory), so that a node's result does not
+// depend on which copy it met.
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
@@ -1200,13 +1201,14 @@ __device__ __forceinline__ void add_node_pulses(const TileView<Real>& tv, const 
 
 constexpr unsigned kFullMask = 0xffffffffu;
 
-// (alpha dt, beta dt) of node i: pre-scaled in shared-memory tiles, scaled here otherwise.
+// (alpha dt, beta dt) of node i: pre-scaled in shared-memory tiles, scaled here otherwise
+// (rounded as there).
 template <typename Real, bool kPre>
 __device__ __forceinline__ Pair<Real> coef(const TileView<Real>& tv, int i, Real dt) {
   Pair<Real> c = tv.ab[i];
   if (!kPre) {
-    c.x *= dt;
-    c.y *= dt;
+    c.x = mul_rn(c.x, dt);
+    c.y = mul_rn(c.y, dt);
   }
   return c;
 }
@@ -1242,7 +1244,7 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
     ds = vdelta<Real>(tv.v[ns], v0);
     as = cs.x;
     wE = wF = cs.y;
-    wR = cs.y * ds;
+    wR = mul_rn(cs.y, ds);
   }
   for (int k = 0; k < max_len; k += 4) {
     const int4 rn = rq[k / 4 + 1];
@@ -1261,16 +1263,16 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
       const bool act = len > k + j;
       const Real delta = vdelta<Real>(v[j], v[j + 1]);
       const Real E = row[j].x + wE;
-      const Real R = (row[j].y + wR) - c[j].x * delta;
+      const Real R = fma_rn(-c[j].x, delta, row[j].y + wR);
       const Real inv = pivot_rcp(E + c[j].x);
-      const Real g = c[j].y * inv;
-      if (act) tv.dr[id[j]] = make_pair(inv * R, c[j].x * inv);
+      const Real g = mul_rn(c[j].y, inv);
+      if (act) tv.dr[id[j]] = make_pair(mul_rn(inv, R), mul_rn(c[j].x, inv));
       if (kLower) {
-        if (act) tv.q[id[j]] = inv * wF;
-        wF = act ? g * wF : wF;
+        if (act) tv.q[id[j]] = mul_rn(inv, wF);
+        wF = act ? mul_rn(g, wF) : wF;
       }
-      wE = act ? (c[j].y * E) * inv : wE;
-      wR = act ? g * R + c[j].y * delta : wR;
+      wE = act ? mul_rn(mul_rn(c[j].y, E), inv) : wE;
+      wR = act ? fma_rn(g, R, mul_rn(c[j].y, delta)) : wR;
     }
     id0 = id[4];
     v0 = v[4];
@@ -1293,20 +1295,20 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
 #pragma unroll
     for (int j = 3; j >= 0; --j) {
       const bool act = len > k + j;
-      p = act ? d[j].x + d[j].y * p : p;
-      u = act ? d[j].y * u : u;
+      p = act ? fma_rn(d[j].y, p, d[j].x) : p;
+      u = act ? mul_rn(d[j].y, u) : u;
       if (act) tv.dr[id[j]] = make_pair(p, u);
       if (kLower) {
-        q = act ? f[j] + d[j].y * q : q;
+        q = act ? fma_rn(d[j].y, q, f[j]) : q;
         if (act) tv.q[id[j]] = q;
       }
     }
   }
   if (kLower && valid) {
     SepRow<Real> o;
-    o.e = row_s.x + as * (Real(1) - q - u);
-    o.r = row_s.y + as * (p - ds);
-    o.a = as * u;
+    o.e = fma_rn(as, Real(1) - q - u, row_s.x);
+    o.r = fma_rn(as, p - ds, row_s.y);
+    o.a = mul_rn(as, u);
     o.b = wF;
     tv.srow[sg.s] = o;
     tv.own[sg.s] = make_pair(wE - wF, wR);
@@ -1423,10 +1425,10 @@ __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int w
         }
       }
       const Real inv = pivot_rcp(E + it.row.a);
-      const Real w = it.row.b * inv;
+      const Real w = mul_rn(it.row.b, inv);
       const bool valid = b + lane < e;
-      if (valid) tv.inbox[it.rec.inbox] = make_pair(it.own.x + w * E, it.own.y + w * R);
-      if (valid) *reinterpret_cast<Pair<Real>*>(tv.srow + b + lane) = make_pair(it.row.a * inv, R * inv);
+      if (valid) tv.inbox[it.rec.inbox] = make_pair(fma_rn(w, E, it.own.x), fma_rn(w, R, it.own.y));
+      if (valid) *reinterpret_cast<Pair<Real>*>(tv.srow + b + lane) = make_pair(mul_rn(it.row.a, inv), mul_rn(R, inv));
       __syncwarp();
       b = e;
       cb = ce;
@@ -1444,7 +1446,7 @@ __device__ __forceinline__ void sweep_separators(const TileView<Real>& tv, int w
       const int j1 = min(b1 + lane, j_last);
       const uint32_t t1 = tv.seps[j1].t;
       const Pair<Real> d1 = *reinterpret_cast<const Pair<Real>*>(tv.srow + j1);
-      const Real x = d.y + d.x * tv.xsep[t];
+      const Real x = fma_rn(d.x, tv.xsep[t], d.y);
       if (b + lane < e) tv.xsep[b + lane] = x;
       __syncwarp();
       e = b;
