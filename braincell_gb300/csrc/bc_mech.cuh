@@ -57,13 +57,16 @@ __device__ __forceinline__ float rcp_approx(float x) {
 __device__ __forceinline__ float rdiv(float a, float b) { return a * rcp_approx(b); }
 __host__ __device__ __forceinline__ double rdiv(double a, double b) { return a / b; }
 
-// a / b to about half an ulp, for finite non-zero b: one Newton correction of
-// a * rcp(b) (the IEEE division takes about three times the instructions and a
-// branch to a subroutine).
+// a / b to half an ulp and 2^-44: the residual a - b q of the approximate quotient, exact by
+// the fused multiply-add, corrects it (P. Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  b is not zero, denormal
+// or minus infinity: the callers' sums of rates and e^x - 1 are neither.  Over an infinite
+// sum of rates a finite rate gives 0 (the cap keeps the residual finite).  The IEEE division
+// takes about three times the instructions and a branch to a subroutine.
 __device__ __forceinline__ float adiv(float a, float b) {
   const float r = rcp_approx(b);
   const float q = a * r;
-  return fmaf(fmaf(-b, q, a), r, q);
+  return fmaf(fmaf(-fminf(b, 3.4e38f), q, a), r, q);
 }
 __host__ __device__ __forceinline__ double adiv(double a, double b) { return a / b; }
 
