@@ -43,8 +43,9 @@ __host__ __device__ __forceinline__ double dpow(double x, double y) { return pow
 // build of this header can check the FP64 rates against the oracle on a CPU; the
 // FP32 forms stay device-only.
 // Rate-function arithmetic: FP32 uses the hardware approximations (__expf, and
-// a * rcp.approx(b) for a / b: a few ulp, far below what the rates need); FP64
-// stays exact so the FP64 build remains an oracle-grade run of the same kernels.
+// a * rcp.approx(b) for a / b: a few ulp, far below what the rates need); FP64 forms
+// are good to an ulp or two, so that the FP64 build is an oracle-grade run of the same
+// kernels.
 __device__ __forceinline__ float rexp(float x) { return __expf(x); }
 __device__ __forceinline__ float aexp(float x) { return expf(x); }
 __host__ __device__ __forceinline__ double aexp(double x) { return exp(x); }
@@ -70,14 +71,23 @@ __device__ __forceinline__ float adiv(float a, float b) {
 }
 __host__ __device__ __forceinline__ double adiv(double a, double b) { return a / b; }
 
-// 1 / x for the step's rate forms.  FP64: one third-order step from the hardware
-// estimate, e = 1 - x r, r += r (e + e^2) (x normal and finite: the forms below see to
-// it); on the host the division.
+// 1 / x of the pivots and the step's rate forms.  FP64, for finite |x| in 2^-1021 .. 2^1020:
+// an estimate r from the FP32 reciprocal of x's leading 24 bits, put together with integer
+// operations (free beside FP64), then 1 / x = r / (1 - e) = r (1 + e + e^2 + ..) with e = 1 - x r
+// (the cubic form of Schulz's iteration; M. Altman, "An optimum cubically convergent iterative
+// method of inverting a linear bounded operator in Hilbert space", Pacific J. Math. 10, 1960).
+// The leading bits and the estimate of their reciprocal are each off by 2^-23 at most, so
+// |e| <= 2^-22 and e^3 is 2^-66: the result is off by its last rounding and 2^-13 of that, for
+// three FP64 instructions.  NaN stays NaN.  On the host the division.
 __device__ __forceinline__ float srcp(float x) { return rcp_approx(x); }
 __host__ __device__ __forceinline__ double srcp(double x) {
 #ifdef __CUDA_ARCH__
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int m = (__funnelshift_l(lo, hi, 3) & 0x007fffff) | 0x3f800000;  // 1 <= m < 2: exponent 127 in FP32
+  const int f = __float_as_int(rcp_approx(__int_as_float(m)));
+  // FP64 exponent fields: f's is its own + 896; dividing by 2^k, k = x's field - 1023, takes k off
+  const int h = ((f >> 3) + ((896 + 1023) << 20) - (hi & 0x7ff00000)) | (hi & int(0x80000000));
+  const double r = __hiloint2double(h, f << 29);
   const double e = fma(-x, r, 1.0);
   return fma(r, fma(e, e, e), r);
 #else

@@ -7,8 +7,9 @@ FP32, u = 2^-24 (half an ulp, relative):
 - ``over_1pexp(c, x)`` = c / (1 + e^x): CUDA's expf 2 ulp = 4 u, the sum 1 u, the division 1 u.
 
 FP64, u = 2^-53 (``ln_pos`` and ``exp2_256`` against exact values, as the host test has them):
-- ``srcp(x)``: the hardware estimate takes 20 bits of x and gives 20 bits, so |e| = |1 - x r| < 2^-18.5; the series
-  r (1 + e + e^2) leaves e^3 < 2^-55.5 = 0.18 u, and the last rounding 1 u.
+- ``srcp(x)``: the estimate takes 24 bits of x (off by 2^-23 at most) and is CUDA's FP32 approximation of their
+  reciprocal (1 ulp, 2^-23), so |e| = |1 - x r| <= 2^-22; the series r (1 + e + e^2) leaves e^3 = 2^-66 and the last
+  rounding, 1 u.  CUDA's 1.0 / x is the correctly rounded one.
 """
 
 import ctypes as C
@@ -85,3 +86,59 @@ def test_fp32_rate_forms(lib):
     for fn in (OVER_EXPREL, OVER_1PEXP):
         c, _, got = _f32(lib, fn, 4.0, far)
         assert (got >= 0).all() and (got <= 1e-31).all()
+
+
+def _relative_error(got, want):
+    with decimal.localcontext() as ctx:
+        ctx.prec = 50
+        return max(abs(float(D(float(g)) / w - 1)) for g, w in zip(got, want))
+
+
+def test_fp64_reciprocal(lib):
+    rng = np.random.default_rng(2)
+    ends = [1.0, np.nextafter(1.0, 2.0), np.nextafter(2.0, 1.0), np.nextafter(1.0, 0.0), 1.5, 4.0 / 3.0, 1.0 + 2.0**-23,
+            1.0 + 2.0**-20, 2.0 - 2.0**-20, 1.0 - 2.0**-24]
+    # mantissas of every leading pattern's ends, exponents over the whole range, 2^+-1008 among them
+    x = np.concatenate([np.ldexp(rng.uniform(1.0, 2.0, 400_000), rng.integers(-1021, 1020, 400_000)),
+                        np.outer(np.exp2(np.r_[-1008:1009:96, 0]), ends).ravel(), 1.0 + np.arange(4096) / 4096,
+                        np.nextafter(1.0 + np.arange(4096) / 4096, 0.0)])
+    x = np.concatenate([x, -x])
+    got, want = _f64(lib, RCP, x), 1.0 / x
+    near = np.abs(got - want) <= np.spacing(np.abs(want))
+    assert near.all()
+    # the correctly rounded value but where 1 / x lies within 2^-13 u of the middle of two numbers
+    off = np.nonzero(got != want)[0]
+    assert off.size <= 2.0**-11 * x.size
+    for k in off:
+        assert abs(Fraction(float(got[k])) * Fraction(float(x[k])) - 1) <= Fraction(U64) * (1 + Fraction(1, 4096))
+
+
+def test_fp64_reciprocal_of_nan(lib):
+    assert np.isnan(_f64(lib, RCP, [np.nan, -np.nan])).all()
+
+
+def test_fp64_exponential(lib):
+    rng = np.random.default_rng(3)
+    y = np.concatenate([np.arange(-300, 300), np.arange(-300, 300) + np.nextafter(0.5, 0),
+                        rng.uniform(-2e4, 2e4, 1500), rng.uniform(-2.56e5, 2.56e5, 500)])
+    with decimal.localcontext() as ctx:
+        ctx.prec = 50
+        want = [(D(float(t)) / 256 * D(2).ln()).exp() for t in y]
+    assert _relative_error(_f64(lib, EXP2_256, y), want) < 2.4 * U64
+    far = _f64(lib, EXP2_256, [3e5, 1e300, np.inf, -3e5, -1e300, -np.inf])
+    assert np.isfinite(far).all() and (far[:3] > 1e303).all() and (far[3:] < 1e-303).all() and (far > 0).all()
+
+
+def test_fp64_logarithm(lib):
+    rng = np.random.default_rng(4)
+    j = 1.0 + np.arange(256) / 256
+    x = np.concatenate([j, np.nextafter(j, 0), j * 2.0**-13, np.exp(rng.uniform(-20, 10, 1500)),
+                        np.exp(rng.uniform(-700, 700, 300)), [2.0**-1022, 1.7e308]])
+    with decimal.localcontext() as ctx:
+        ctx.prec = 50
+        want = [D(float(t)).ln() for t in x]
+    for g, w in zip(_f64(lib, LN, x), want):
+        assert abs(D(float(g)) - w) < D(3 * U64) + D(3 * U64) * abs(w)
+    with np.errstate(all="ignore"):
+        x = np.array([0.0, -0.0, -1.0, 1e-310, np.inf, np.nan])
+        np.testing.assert_allclose(_f64(lib, LN, x), np.log(x), rtol=4 * U64, equal_nan=True)
