@@ -942,7 +942,7 @@ __device__ __forceinline__ void node_mechanisms(const NodeStates<Real, W>& s0, R
         if (kAdv) {
           const KdrRates<Real> r(v[j], P[j][BC_P_KDR_VSH]);
           const Real s = r.a + r.b;
-          p = p - dexpm1(k_of(j, BC_P_KDR_PHI) * s) * (adiv(r.a, s) - p);
+          p = p - dexpm1(k_of(j, BC_P_KDR_PHI) * s) * (adiv_sum(r.a, s) - p);
           st[kSlotKdrP * N + j] = p;
         }
         const Real p2 = p * p;

@@ -60,15 +60,22 @@ __host__ __device__ __forceinline__ double rdiv(double a, double b) { return a /
 
 // a / b to half an ulp and 2^-44: the residual a - b q of the approximate quotient, exact by
 // the fused multiply-add, corrects it (P. Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  b is not zero, denormal
-// or minus infinity: the callers' sums of rates and e^x - 1 are neither.  Over an infinite
-// sum of rates a finite rate gives 0 (the cap keeps the residual finite).  The IEEE division
-// takes about three times the instructions and a branch to a subroutine.
+// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990).  b is finite and neither
+// zero nor denormal, as the callers' sums of rates and e^x - 1 are.  The IEEE division takes
+// about three times the instructions and a branch to a subroutine.
 __device__ __forceinline__ float adiv(float a, float b) {
+  const float r = rcp_approx(b);
+  const float q = a * r;
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+// The same for a sum b of rates that may overflow: a finite rate's share of it is 0 then, as
+// the IEEE quotient is (the cap keeps the residual finite).
+__device__ __forceinline__ float adiv_sum(float a, float b) {
   const float r = rcp_approx(b);
   const float q = a * r;
   return fmaf(fmaf(-fminf(b, 3.4e38f), q, a), r, q);
 }
+__host__ __device__ __forceinline__ double adiv_sum(double a, double b) { return a / b; }
 __host__ __device__ __forceinline__ double adiv(double a, double b) { return a / b; }
 
 // 1 / x of the pivots and the step's rate forms.  FP64, for finite |x| in 2^-1021 .. 2^1020:
@@ -327,7 +334,7 @@ __host__ __device__ __forceinline__ double over_1pexp(double c, double x) { retu
 template <typename Real, bool kExact = false>
 __device__ __forceinline__ Real gate_ab(Real x, Real a, Real b, Real phi, Real dt) {
   const Real s = a + b;
-  if (kExact) return x - dexpm1(-dt * phi * s) * (adiv(a, s) - x);
+  if (kExact) return x - dexpm1(-dt * phi * s) * (adiv_sum(a, s) - x);
   const Real xinf = rdiv(a, s);
   return x - decay_em1(-dt * phi * s) * (xinf - x);
 }

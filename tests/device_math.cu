@@ -3,7 +3,7 @@
 #include "../braincell_gb300/csrc/bc_mech.cuh"
 
 namespace {
-enum { kRcp = 0, kExp2_256, kLn, kDiv, kOverExprel, kOver1pExp };
+enum { kRcp = 0, kExp2_256, kLn, kDiv, kOverExprel, kOver1pExp, kDivSum };
 
 __global__ void apply_f64(int fn, const double* x, int n, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -13,7 +13,12 @@ __global__ void apply_f64(int fn, const double* x, int n, double* out) {
 __global__ void apply_f32(int fn, const float* a, const float* b, int n, float* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  out[i] = fn == kDiv ? bc::adiv(a[i], b[i]) : fn == kOverExprel ? bc::over_exprel(a[i], b[i]) : bc::over_1pexp(a[i], b[i]);
+  switch (fn) {
+    case kDiv: out[i] = bc::adiv(a[i], b[i]); break;
+    case kDivSum: out[i] = bc::adiv_sum(a[i], b[i]); break;
+    case kOverExprel: out[i] = bc::over_exprel(a[i], b[i]); break;
+    default: out[i] = bc::over_1pexp(a[i], b[i]);
+  }
 }
 
 template <typename T>

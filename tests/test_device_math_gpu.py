@@ -1,7 +1,7 @@
 """The device forms of the library's own arithmetic (``bc_mech.cuh``), compiled for sm_103a.
 
 FP32, u = 2^-24 (half an ulp, relative):
-- ``adiv(a, b)``: the quotient's residual is exact but for its own rounding, and the correction is 2^-22 of the
+- ``adiv(a, b)``, ``adiv_sum(a, b)``: the quotient's residual is exact but for its own rounding, and the correction is 2^-22 of the
   quotient, so what is left is the last rounding, 1 u, and 2^-44;
 - ``over_exprel(c, x)`` = c x / (e^x - 1): the product 1 u, CUDA's expm1f 1 ulp = 2 u, the division 1 u;
 - ``over_1pexp(c, x)`` = c / (1 + e^x): CUDA's expf 2 ulp = 4 u, the sum 1 u, the division 1 u.
@@ -25,7 +25,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-RCP, EXP2_256, LN, DIV, OVER_EXPREL, OVER_1PEXP = range(6)
+RCP, EXP2_256, LN, DIV, OVER_EXPREL, OVER_1PEXP, DIV_SUM = range(7)
 U32, U64 = 2.0**-24, 2.0**-53
 D = decimal.Decimal
 
@@ -61,14 +61,15 @@ def test_fp32_division(lib):
     n = 200_000
     a = rng.choice([-1.0, 1.0], n) * np.exp2(rng.uniform(-60, 60, n))
     b = rng.choice([-1.0, 1.0], n) * np.exp2(rng.uniform(-60, 60, n))
-    a, b, q = _f32(lib, DIV, a, b)
-    assert np.max(np.abs(q / (a / b) - 1.0)) <= U32 * (1 + 2.0**-18)
+    for fn in (DIV, DIV_SUM):
+        x, y, q = _f32(lib, fn, a, b)
+        assert np.max(np.abs(q / (x / y) - 1.0)) <= U32 * (1 + 2.0**-18)
 
 
 def test_fp32_division_at_the_ends(lib):
     # rates of a gate far outside its range: a finite rate over an infinite sum is 0, as the IEEE quotient
     inf, nan = np.inf, np.nan
-    a, b, q = _f32(lib, DIV, [0.0, 1.0, 1e30, 0.0, 1e-30, inf, nan, 1.0], [inf, inf, inf, 1e30, 1e38, inf, 1.0, nan])
+    a, b, q = _f32(lib, DIV_SUM, [0.0, 1.0, 1e30, 0.0, 1e-30, inf, nan, 1.0], [inf, inf, inf, 1e30, 1e38, inf, 1.0, nan])
     np.testing.assert_array_equal(q[:4], 0.0)
     assert abs(q[4]) <= 1.2e-38  # below the normal numbers
     assert np.isnan(q[5:]).all()
