@@ -685,10 +685,9 @@ def run_ours(a):
         plan.reset(stream=sid)
     e2e_s = reduce_max(float(np.median(e2e_t)))
     e2e_value = n_cv * a.sim_steps * world / e2e_s
-    # bytes the API moves: upload = values + hi/lo offset tables (24 B/CV); download = its
-    # offset tables up (16 B/CV) and values down (8 B/CV); spike counts down (4 B/probe)
-    h2d_total = 24 * n_cv + 16 * n_cv
-    d2h = 8 * n_cv + 4 * int(counts.size)
+    # bytes the API moves: the voltages up, the voltages and the spike counts down
+    h2d_total = v_host.nbytes
+    d2h = v_out.nbytes + counts.nbytes
 
     peak, peak_kind = _peaks()
     achieved_gbs = nbytes * n_cv * a.sim_steps / (kernel_ms * 1e-3) / 1e9
