@@ -2518,7 +2518,7 @@ bc_status bc_state_download_noalloc(bc_plan_t p, int32_t which, double* out, voi
   BC_NEED_DEVICE(p);
   BC_CUDA(cudaSetDevice(p->device));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // The call copies from pageable host memory and synchronises the stream, and
+  // The call copies to pageable host memory and synchronises the stream, and
   // neither is allowed while the stream is being captured into a graph.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   BC_CUDA(cudaStreamIsCapturing(s, &cap));

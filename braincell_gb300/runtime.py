@@ -173,7 +173,7 @@ class Plan:
         """Like :meth:`state`, into a caller-held float64 array, with no device allocation.
 
         Goes through ``bc_state_download_noalloc``: fixed library scratch instead of
-        per-call buffers, for plans of at most ``BC_NOALLOC_MAX_CV`` CVs.  Calls from
+        the plan's locked value buffer, for plans of at most ``BC_NOALLOC_MAX_CV`` CVs.  Calls from
         several threads at once race on that scratch and must be serialised.
         """
         if out.dtype != np.float64 or out.shape != (self.n_cv,) or not out.flags.c_contiguous:

@@ -694,14 +694,15 @@ bc_status bc_state_upload(bc_plan_t plan, int32_t which, const double* in /* [n_
  * (a monitor, a closed-loop controller) and cannot afford cudaMalloc/cudaFree,
  * which synchronise the whole device and so stall every queued launch; and a
  * process whose device memory is already held by a caching allocator, where a
- * fresh cudaMalloc may fail.  bc_state_download allocates its offset tables and
- * value buffer per call; this variant uses one fixed scratch array in the
- * library's device image plus a host staging array of the same capacity, both
- * sized for BC_NOALLOC_MAX_CV compartments (24 bytes each on the device: 6 MiB).
+ * fresh cudaMalloc may fail.  (bc_state_download allocates nothing per call either:
+ * the plan holds the compartment map and a buffer for one view's values, under a
+ * lock, so that several threads may read one plan.)  This variant takes the values
+ * through one fixed scratch array in the library's device image, sized for
+ * BC_NOALLOC_MAX_CV compartments (8 bytes each: 2 MiB), and no lock.
  * Plans with more CVs are rejected with BC_ERR_INVALID (use bc_state_download).
  * The first call on each device looks up the scratch address (cudaGetSymbolAddress)
  * and caches it.  Never call it on a stream that is being captured into a CUDA
- * graph: it copies from pageable host memory and synchronises the stream, so it
+ * graph: it copies to pageable host memory and synchronises the stream, so it
  * returns BC_ERR_INVALID there.  The scratch is shared by every plan of the
  * process: calls that overlap in time (from several host threads) race on it, so
  * the caller must serialise them.  Returns once `out` holds the values (the stream
