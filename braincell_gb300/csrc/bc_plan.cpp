@@ -1746,6 +1746,10 @@ bc_status bc_plan_create(const bc_batch_spec* spec, const bc_plan_options* opts_
   if (tile_nodes <= 0) tile_nodes = 900;
   tile_nodes = std::max(tile_nodes, 16);
   p->tile_nodes = tile_nodes;
+  // A tile is never packed with more nodes than the arrays of (V), (alpha, beta) and row pairs and of indices leave
+  // room for in shared memory: it would only be split again, and before that it might hold more separators than 16
+  // bits count, or go to one cluster as a whole.
+  tile_nodes = int(std::min<size_t>(tile_nodes, smem_budget / (6 * rs + 8)));
   // Launch classes: 0 = packed shared-memory tiles (cells <= tile_nodes), 1 = one big
   // cell per shared-memory tile, 2 = global-memory tiles (too big for shared memory).
   // (a thread for every pair of nodes and a warp for the heavy ones, up to 512: two such tiles fill an SM's registers)
