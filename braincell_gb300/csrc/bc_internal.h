@@ -84,8 +84,10 @@ struct alignas(16) SlotRec {
   int32_t kind;      // kSlotLeaf, kSlotLower: segments without / with a lower separator; kSlotCell: whole cells
 };
 constexpr int32_t kSlotLeaf = 0, kSlotLower = 1, kSlotCell = 2;
-// On the GB300, 1,000 network cells of 9 nodes x 400 steps: 7.19 ms cut into segments, 6.77 ms whole; 20,000 cells of
-// 8 to 100 nodes x 401 steps: 8.79 ms with all of them cut, 9.14 / 9.64 ms with those of up to 10 / 16 nodes whole.
+// When only the solve was new, 1,000 network cells of 9 nodes x 400 steps took 7.19 ms cut into segments, 6.77 ms whole.
+// With the update pass and the chunked sweep it is the other way round: 2.48 ms cut, 3.04 ms whole (20,000 cells of
+// 9.7 nodes: 8.7 / 10.6 us a step in FP32, 112 / 110 in FP64), and cut cells are nearer to 64 bits.  The line stays
+// where it is because results would move with it, V by 1e-5 of itself.
 constexpr int kCellLaneNodes = 10;
 // A separator's inbox holds an entry per segment below it, padded to pairs, two or more.
 struct alignas(16) SepRec {

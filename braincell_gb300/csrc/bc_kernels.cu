@@ -1185,7 +1185,8 @@ __device__ __forceinline__ void add_node_pulses(const TileView<Real>& tv, const 
 //      (wE, wF) = b_k inv_k (E_k, F_k),  wR = b_k (inv_k R_k + Delta_k),
 //    starting from wE = wF = b_s, wR = b_s Delta_s (0 at a leaf), then walks back down
 //    to leave x_k = p_k + q_k x_s + u_k x_t in every node and to hand both separators
-//    their rows' share.  The excess form has no subtraction in the pivots.
+//    their rows' share.  The excess form has no subtraction in a segment's pivots (the
+//    separators' own excess, a_s (1 - q - u), has: it cancels where a_s is large).
 // 2. Separators (sweep_separators): the same elimination on the tree of separators,
 //    one warp per group of cells, level by level, then back down to x.
 // 3. Every other node's x is one or two multiply-adds on its separators' x, taken by
@@ -1317,9 +1318,8 @@ __device__ __forceinline__ void eliminate_slot(const TileView<Real>& tv, const S
 
 // One slot of whole cells: lane l eliminates and back-substitutes its cell, in the
 // diagonal form.  A parent with one child is the next row and takes its child's terms
-// from registers; other parents collect them in their rows, child by child.  For cells
-// this small the separators are as many as the segments, and their sweep, inboxes and
-// records cost more than the walk.
+// from registers; other parents collect them in their rows, child by child.  (See
+// kCellLaneNodes for which cells, and both sides measured.)
 template <typename Real, bool kPre>
 __device__ __forceinline__ void solve_cells(const TileView<Real>& tv, const SlotRec& sr, int lane, Real dt) {
   const int32_t* rows = tv.rows + sr.rows0;

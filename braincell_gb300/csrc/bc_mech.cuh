@@ -113,8 +113,8 @@ __host__ __device__ __forceinline__ double srcp(double x) {
 // the argument, the cap and the division before the logarithm take two to three times
 // that: 250 uneven cells of 50 to 2000 compartments, 200 FP64 steps, went from 50.2 to
 // 40.6 ms with these, the shorter decay series and the three-instruction reciprocal.
-// The tables come from the definitions, in double-double arithmetic at compile
-// time.
+// The tables come from the definitions at compile time: the powers in double-double
+// arithmetic, the logarithms by the artanh series in double.
 struct TwoDouble {
   double h, l;
 };
@@ -329,8 +329,8 @@ __host__ __device__ __forceinline__ double over_1pexp(double c, double x) { retu
 
 // One exp-Euler step y += dt * exprel(dt * lam) * f of a gate whose right-hand
 // side is affine in the gate: with lam = -phi (a + b) and f = -lam (x_inf - x) the
-// step is x - expm1(dt * lam) * (x_inf - x).  kExact selects IEEE division and
-// expm1 (the spike-generating Na / K gates) over the fast forms.
+// step is x - expm1(dt * lam) * (x_inf - x).  kExact selects the corrected
+// quotient and expm1 (the spike-generating Na / K gates) over the fast forms.
 template <typename Real, bool kExact = false>
 __device__ __forceinline__ Real gate_ab(Real x, Real a, Real b, Real phi, Real dt) {
   const Real s = a + b;
